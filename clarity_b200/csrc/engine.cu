@@ -765,8 +765,22 @@ static Status make_otf(Context& ctx, const PlanEntry& pe, const float* ker,
   pro.scale = scale;
   pro.xmode = pe.P.xmode;
   CL_TRY(xy_forward(ctx, pe, pro, H));
-  CL_TRY(z_pass(ctx, pe, ModForward{}, H, H));
+  // the kernel's planes wrap around plane 0; those between are zero
+  ModForward m;
+  m.zn = kd.z - kd.z / 2;
+  m.zh = wd.z - kd.z / 2;
+  CL_TRY(z_pass(ctx, pe, m, H, H));
   return Status::Ok();
+}
+
+// The spectral product of a convolution whose input is zero in planes z >= zn
+// and of whose result only planes z < zout are wanted.
+static ModOTF otf_between(const float2* H, float scale, int zn, int zout,
+                          const float* scale2 = nullptr) {
+  ModOTF m{H, scale, scale2};
+  m.zn = zn;
+  m.zout = zout;
+  return m;
 }
 
 static Status setup(Context& ctx, Dims id, Dims kd, const PlanEntry** pe,
@@ -826,7 +840,6 @@ Status Context::tune(const Dims& wd, std::unique_ptr<PlanEntry>* out) {
     CL_CHECK(cudaEventCreate(&e0));
     CL_CHECK(cudaEventCreate(&e1));
     const ImageSrc g{u, wd.x, wd.y, wd.z};
-    const WorkVol wv{wd.x, wd.y, wd.z};
     for (int c = 0; c < nc; ++c) {
       std::unique_ptr<PlanEntry> pe;
       CL_TRY(build_entry(cand[c], &pe));
@@ -836,8 +849,9 @@ Status Context::tune(const Dims& wd, std::unique_ptr<PlanEntry>* out) {
         CL_TRY(xy_inv_fwd(*this, *pe, MidRLRatio{g, xm}, S));
         CL_TRY(z_pass(*this, *pe, ModOTF{S, 1.f}, S, S));
         EpiRLProduct epi{};
-        epi.cur = u; epi.g = g; epi.scale = nullptr; epi.unew = u; epi.partial = partial;
-        epi.w = wv; epi.xmode = xm; epi.acc = 0.0; epi.nblocks = nullptr;
+        epi.cur = u; epi.X = wd.x; epi.Y = wd.y; epi.Z = wd.z;
+        epi.scale = nullptr; epi.unew = u; epi.partial = partial;
+        epi.xmode = xm; epi.acc = 0.0; epi.nblocks = nullptr;
         CL_TRY(xy_inv_fwd(*this, *pe, epi, S));
         return Status::Ok();
       };
@@ -883,7 +897,7 @@ Status run_convolve(Context& ctx, const float* img, Dims id, const float* ker,
   CL_TRY(make_otf(ctx, *pe, ker, kd, wd, ws->H, nullptr));
   ProImage pro{image_src(img, id), P.xmode};
   CL_TRY(xy_forward(ctx, *pe, pro, ws->S));
-  CL_TRY(z_pass(ctx, *pe, ModOTF{ws->H, inv_volume(wd)}, ws->S, ws->S));
+  CL_TRY(z_pass(ctx, *pe, otf_between(ws->H, inv_volume(wd), id.z, id.z), ws->S, ws->S));
   EpiClip epi{out, id.x, id.y, id.z, nullptr, P.xmode};
   CL_TRY(xy_inverse(ctx, *pe, epi, ws->S));
   return Status::Ok();
@@ -906,7 +920,7 @@ Status run_correlate(Context& ctx, const float* img, Dims id, const float* ker, 
   CL_CHECK(cudaGetLastError());
   ProImage pro{image_src(img, id), P.xmode};
   CL_TRY(xy_forward(ctx, *pe, pro, ws->S));
-  CL_TRY(z_pass(ctx, *pe, ModOTF{ws->HG, inv_volume(wd)}, ws->S, ws->S));
+  CL_TRY(z_pass(ctx, *pe, otf_between(ws->HG, inv_volume(wd), id.z, id.z), ws->S, ws->S));
   EpiClip epi{out, id.x, id.y, id.z, nullptr, P.xmode};
   CL_TRY(xy_inverse(ctx, *pe, epi, ws->S));
   return Status::Ok();
@@ -922,7 +936,9 @@ Status run_wiener(Context& ctx, const float* img, Dims id, const float* ker,
   CL_TRY(make_otf(ctx, *pe, ker, kd, wd, ws->H, nullptr));
   ProImage pro{image_src(img, id), P.xmode};
   CL_TRY(xy_forward(ctx, *pe, pro, ws->S));
-  CL_TRY(z_pass(ctx, *pe, ModWiener{ws->H, eps, inv_volume(wd)}, ws->S, ws->S));
+  ModWiener m{ws->H, eps, inv_volume(wd)};
+  m.zn = m.zout = id.z;
+  CL_TRY(z_pass(ctx, *pe, m, ws->S, ws->S));
   EpiClip epi{out, id.x, id.y, id.z, nullptr, P.xmode};
   CL_TRY(xy_inverse(ctx, *pe, epi, ws->S));
   return Status::Ok();
@@ -1006,7 +1022,6 @@ static Status rl_core(Context& ctx, const PlanEntry& pe, Workspace& ws,
   const ImageSrc u0 = start ? image_src(start, sd) : g;
   const float2* H = roles.otf ? roles.otf : ws.H;
   const float2* H2 = roles.otf2 ? roles.otf2 : H;
-  const WorkVol wv{wd.x, wd.y, wd.z};
   const float scale_n = inv_volume(wd);
   float* sdev = ws.fscal;  // deferred flux scale
   if (rescale) {
@@ -1021,11 +1036,10 @@ static Status rl_core(Context& ctx, const PlanEntry& pe, Workspace& ws,
   CL_TRY(xy_forward(ctx, pe, ProImage{u0, P.xmode}, ws.S));
   for (int k = 0; k < iters; ++k) {
     const float* sk = (k == 0 || !rescale) ? nullptr : sdev;
-    // P3 reads only planes z < Z (the image is zero beyond): the rest of this
-    // pass's output is neither inverse-transformed along y0 nor stored
-    ModOTF m2{H, scale_n, sk};
-    m2.zout = id.z;
-    CL_TRY(z_pass(ctx, pe, m2, ws.S, ws.S));
+    // the estimate is zero in planes z >= its extent, and P3 reads only planes
+    // z < Z (the image is zero beyond): no other plane is read, or
+    // inverse-transformed along y0, or stored
+    CL_TRY(z_pass(ctx, pe, otf_between(H, scale_n, sd.z, id.z, sk), ws.S, ws.S));
     MidRLRatio ratio{g, P.xmode};
     if (idiv) {
       ratio.idiv_partial = ws.partial;
@@ -1039,17 +1053,17 @@ static Status rl_core(Context& ctx, const PlanEntry& pe, Workspace& ws,
       CL_CHECK(cudaGetLastError());
     }
     // the ratio is zero in planes z >= Z (the image is zero there): P3 does
-    // not write them and this pass reads them as zeros
-    ModOTF m4{H2, scale_n};
-    m4.zn = id.z;
-    CL_TRY(z_pass(ctx, pe, m4, ws.S, ws.S));
+    // not write them and this pass reads them as zeros; P5 wants the
+    // estimate's planes only
+    CL_TRY(z_pass(ctx, pe, otf_between(H2, scale_n, id.z, sd.z), ws.S, ws.S));
     EpiRLProduct epi;
-    epi.cur = (k == 0) ? nullptr : ws.u;
-    epi.g = u0;
+    epi.cur = (k == 0) ? u0.src : ws.u;
+    epi.X = sd.x;
+    epi.Y = sd.y;
+    epi.Z = sd.z;
     epi.scale = sk;
     epi.unew = ws.u;
     epi.partial = ws.partial;
-    epi.w = wv;
     epi.xmode = P.xmode;
     epi.acc = 0.0;
     epi.nblocks = ws.iscal;  // the partials' count, as launched
@@ -1070,8 +1084,9 @@ static Status rl_core(Context& ctx, const PlanEntry& pe, Workspace& ws,
   if (idiv && iters > 0) {
     // idiv[iters]: the result's own I-divergence (h * s u', one more forward
     // transform, z pass and xy inverse that only accumulates)
-    CL_TRY(xy_forward(ctx, pe, ProWork{ws.u, rescale ? sdev : nullptr, wv, P.xmode}, ws.S));
-    CL_TRY(z_pass(ctx, pe, ModOTF{H, scale_n}, ws.S, ws.S));
+    CL_TRY(xy_forward(ctx, pe, ProImage{image_src(ws.u, sd), P.xmode, rescale ? sdev : nullptr},
+                      ws.S));
+    CL_TRY(z_pass(ctx, pe, otf_between(H, scale_n, sd.z, id.z), ws.S, ws.S));
     MidRLRatio tr{g, P.xmode};
     tr.idiv_partial = ws.partial;
     tr.nblocks = ws.iscal + 1;
@@ -1115,7 +1130,7 @@ static Status rl_solve(Context& ctx, const PlanEntry& pe, Workspace& ws, const f
       const VolPlan& P = pe.P;
       CL_TRY(make_otf(ctx, pe, ker, kd, wd, ws.H, nullptr));
       CL_TRY(xy_forward(ctx, pe, ProImage{image_src(est, id), P.xmode}, ws.S));
-      CL_TRY(z_pass(ctx, pe, ModOTF{ws.H, inv_volume(wd)}, ws.S, ws.S));
+      CL_TRY(z_pass(ctx, pe, otf_between(ws.H, inv_volume(wd), id.z, id.z), ws.S, ws.S));
       MidRLRatio tr{image_src(img, id), P.xmode};
       tr.idiv_partial = ws.partial;
       tr.nblocks = ws.iscal + 1;
@@ -1134,8 +1149,7 @@ static Status rl_solve(Context& ctx, const PlanEntry& pe, Workspace& ws, const f
   }
   CL_TRY(rl_core(ctx, pe, ws, img, id, wd, iters, true, start, idiv, roles));
   count_small();
-  CLARITY_LAUNCH(k_clip, kReduceBlocks, 256, 0, st)(ws.u, wd.x, wd.y, out, id.x, id.y, id.z,
-                                                    ws.fscal);
+  CLARITY_LAUNCH(k_scale_copy, kReduceBlocks, 256, 0, st)(ws.u, ws.fscal, out, id.n());
   CL_CHECK(cudaGetLastError());
   return Status::Ok();
 }
@@ -1204,7 +1218,7 @@ Status run_rl_accel(Context& ctx, const float* img, Dims id, const float* ker, D
     return Status::Ok();
   }
   const VolPlan& P = pe->P;
-  const long long n = wd.n();
+  const long long n = id.n();  // the estimates are zero outside the image
   CL_TRY(ensure_volumes(ws->accel, &ws->accel_cap, n));
   // partials: one per XY block for the flux sum, two per reduce block for
   // the extrapolation sums
@@ -1215,7 +1229,6 @@ Status run_rl_accel(Context& ctx, const float* img, Dims id, const float* ker, D
   }
   CL_TRY(make_otf(ctx, *pe, ker, kd, wd, ws->H, nullptr));
   const ImageSrc g = image_src(img, id);
-  const WorkVol wv{wd.x, wd.y, wd.z};
   const float scale_n = inv_volume(wd);
   float* B[3] = {ws->accel[0], ws->accel[1], ws->accel[2]};
   float* Y = ws->accel[3];
@@ -1225,14 +1238,12 @@ Status run_rl_accel(Context& ctx, const float* img, Dims id, const float* ker, D
   int xi = 0, pi = 0, ui = 1;  // x, x_prev, x_next buffers (x_prev = x at first)
   CL_TRY(reduce_sum_into(ctx, img, id.n(), ws->partial, ws->dscal + 0));
   count_small();
-  CLARITY_LAUNCH(k_pad_image, kReduceBlocks, 256, 0, st)(start ? image_src(start, id) : g, wv,
-                                                         B[0]);
+  CLARITY_LAUNCH(k_copy, kReduceBlocks, 256, 0, st)(start ? start : img, B[0], n);
   CL_CHECK(cudaMemsetAsync(alpha, 0, sizeof(float), st));
   for (int k = 0; k < iters; ++k) {
-    CL_TRY(xy_forward(ctx, *pe, ProAccel{B[xi], B[pi], alpha, Y, wv, P.xmode}, ws->S));
-    ModOTF m2{ws->H, scale_n};
-    m2.zout = id.z;  // the ratio pass reads planes z < Z only
-    CL_TRY(z_pass(ctx, *pe, m2, ws->S, ws->S));
+    CL_TRY(xy_forward(ctx, *pe, ProAccel{B[xi], B[pi], alpha, Y, id.x, id.y, id.z, P.xmode},
+                      ws->S));
+    CL_TRY(z_pass(ctx, *pe, otf_between(ws->H, scale_n, id.z, id.z), ws->S, ws->S));
     MidRLRatio ratio{g, P.xmode};
     if (idiv) {
       ratio.idiv_partial = ws->partial;
@@ -1244,16 +1255,15 @@ Status run_rl_accel(Context& ctx, const float* img, Dims id, const float* ker, D
       CLARITY_LAUNCH(k_finish_sum_np, 1, 256, 0, st)(ws->partial, ws->iscal + 1, idiv + k);
       CL_CHECK(cudaGetLastError());
     }
-    ModOTF m4{ws->H, scale_n};
-    m4.zn = id.z;
-    CL_TRY(z_pass(ctx, *pe, m4, ws->S, ws->S));
+    CL_TRY(z_pass(ctx, *pe, otf_between(ws->H, scale_n, id.z, id.z), ws->S, ws->S));
     EpiRLProduct epi;
     epi.cur = Y;
-    epi.g = g;
+    epi.X = id.x;
+    epi.Y = id.y;
+    epi.Z = id.z;
     epi.scale = nullptr;
     epi.unew = B[ui];
     epi.partial = ws->partial;
-    epi.w = wv;
     epi.xmode = P.xmode;
     epi.acc = 0.0;
     epi.nblocks = ws->iscal;
@@ -1276,8 +1286,8 @@ Status run_rl_accel(Context& ctx, const float* img, Dims id, const float* ker, D
     ui = 3 - pi - xi;
   }
   if (idiv) {
-    CL_TRY(xy_forward(ctx, *pe, ProWork{B[xi], nullptr, wv, P.xmode}, ws->S));
-    CL_TRY(z_pass(ctx, *pe, ModOTF{ws->H, scale_n}, ws->S, ws->S));
+    CL_TRY(xy_forward(ctx, *pe, ProImage{image_src(B[xi], id), P.xmode}, ws->S));
+    CL_TRY(z_pass(ctx, *pe, otf_between(ws->H, scale_n, id.z, id.z), ws->S, ws->S));
     MidRLRatio tr{g, P.xmode};
     tr.idiv_partial = ws->partial;
     tr.nblocks = ws->iscal + 1;
@@ -1287,8 +1297,7 @@ Status run_rl_accel(Context& ctx, const float* img, Dims id, const float* ker, D
     CL_CHECK(cudaGetLastError());
   }
   count_small();
-  CLARITY_LAUNCH(k_clip, kReduceBlocks, 256, 0, st)(B[xi], wd.x, wd.y, out, id.x, id.y, id.z,
-                                                    nullptr);
+  CLARITY_LAUNCH(k_copy, kReduceBlocks, 256, 0, st)(B[xi], out, n);
   CL_CHECK(cudaGetLastError());
   return Status::Ok();
 }
@@ -1409,9 +1418,8 @@ Status run_rl_batch(Context& ctx, int n, const float* const* imgs, const Dims* i
                                qbuf, origin));
         for (int i = 0; i < n; ++i) {
           count_small();
-          CLARITY_LAUNCH(k_clip, kReduceBlocks, 256, 0, origin)(
-              wss[i]->u, wds[i].x, wds[i].y, outs[i], ids[i].x, ids[i].y, ids[i].z,
-              wss[i]->fscal);
+          CLARITY_LAUNCH(k_scale_copy, kReduceBlocks, 256, 0, origin)(wss[i]->u, wss[i]->fscal,
+                                                                       outs[i], ids[i].n());
           CL_CHECK(cudaGetLastError());
         }
       }
@@ -1470,8 +1478,7 @@ Status run_blind(Context& ctx, const float* img, Dims id, const float* ker,
   CL_TRY(make_otf(ctx, *pe, ker, kd, wd, ws->H, ws->fscal + 2));
   CL_TRY(rl_core(ctx, *pe, *ws, img, id, wd, iters, false));
   count_small();
-  CLARITY_LAUNCH(k_clip, kReduceBlocks, 256, 0, st)(ws->u, wd.x, wd.y, out, id.x, id.y, id.z,
-                                        nullptr);
+  CLARITY_LAUNCH(k_copy, kReduceBlocks, 256, 0, st)(ws->u, out, id.n());
   CL_CHECK(cudaGetLastError());
   return Status::Ok();
 }
@@ -1879,7 +1886,8 @@ Status run_jvc(Context& ctx, const float* img, Dims id, const float* ker,
   for (int k = 0; k < total; ++k) {
     const bool last = k + 1 == total;
     const bool smooth_now = smooth && (k + 1) % smooth_interval == 0;
-    CL_TRY(z_pass(ctx, *pe, ModOTF{ws->H, scale_n}, ws->S, ws->S));
+    // the first update transforms the image, zero in planes z >= Z
+    CL_TRY(z_pass(ctx, *pe, otf_between(ws->H, scale_n, k == 0 ? id.z : wd.z, wd.z), ws->S, ws->S));
     EpiJVC epi{k == 0 ? nullptr : ws->u, g, ws->u, hc[0], hc[1], wv, P.xmode};
     if (!last || smooth_now)
       CL_TRY(xy_inv_fwd(ctx, *pe, epi, ws->S));

@@ -80,7 +80,6 @@ struct Vol {
   float* fscal;   // [0] deferred flux scale
   int* iscal;     // [0] partials the product pass wrote
   ImageSrc g;
-  WorkVol w;
   float scale_n;
   int tiles[kKinds];
 };
@@ -129,9 +128,10 @@ __device__ __forceinline__ void run_item(float2* sm, const VolPlan& P, const Vol
   const float* sk = k == 0 ? nullptr : V.fscal;  // deferred flux scale
   switch (kind) {
     case kZ2: {
-      // the ratio pass reads only planes z < Z: the rest are not stored
+      // the estimate is zero in planes z >= Z and the ratio pass reads only
+      // planes z < Z
       ModOTF m{V.H, V.scale_n, sk};
-      m.zout = V.g.Z;
+      m.zn = m.zout = V.g.Z;
       z_body(sm, P, m, V.S, V.S, V.tw, tile);
       break;
     }
@@ -141,20 +141,21 @@ __device__ __forceinline__ void run_item(float2* sm, const VolPlan& P, const Vol
       break;
     }
     case kZ4: {
-      // the ratio is zero in planes z >= Z: read as zeros
+      // the ratio is zero in planes z >= Z and the product wants no others
       ModOTF m{V.H, V.scale_n};
-      m.zn = V.g.Z;
+      m.zn = m.zout = V.g.Z;
       z_body(sm, P, m, V.S, V.S, V.tw, tile);
       break;
     }
     case kProduct: {
       EpiRLProduct e;
-      e.cur = k == 0 ? nullptr : V.u;
-      e.g = V.g;
+      e.cur = k == 0 ? V.g.src : V.u;
+      e.X = V.g.X;
+      e.Y = V.g.Y;
+      e.Z = V.g.Z;
       e.scale = sk;
       e.unew = V.u;
       e.partial = V.partial;
-      e.w = V.w;
       e.xmode = P.xmode;
       e.acc = 0.0;
       e.nblocks = V.iscal;
@@ -335,13 +336,12 @@ Status launch_rl_batch(Context& ctx, int n, const PlanEntry* const* pes, Workspa
     V.fscal = wss[i]->fscal;
     V.iscal = wss[i]->iscal;
     V.g = ImageSrc{imgs[i], ids[i].x, ids[i].y, ids[i].z};
-    V.w = WorkVol{wds[i].x, wds[i].y, wds[i].z};
     V.scale_n = (float)(1.0 / ((double)wds[i].x * wds[i].y * wds[i].z));
     const int ngroups = P.By / P.G;
     V.tiles[batchk::kZ2] = P.z_blocks;
     V.tiles[batchk::kRatio] = std::min(ids[i].z, P.nz) * ngroups;  // planes z < Z only
     V.tiles[batchk::kZ4] = P.z_blocks;
-    V.tiles[batchk::kProduct] = P.xy_blocks;
+    V.tiles[batchk::kProduct] = V.tiles[batchk::kRatio];
     V.tiles[batchk::kFinish] = 1;
     if (P.xy_threads != 256 || P.z_threads != 256) {
       Status s;

@@ -28,6 +28,14 @@ bool static_xy_inverse(const PlanEntry&, cudaStream_t, const F&, const float2*, 
   } while (0)
 #endif
 
+// Blocks of an XY pass over the planes its functor wants (all by default).
+template <class F>
+inline int xy_grid(const VolPlan& P, const F& f) {
+  int nz = P.nz;
+  if constexpr (requires { f.live_planes(nz); }) nz = f.live_planes(nz);
+  return nz * (P.By / P.G);
+}
+
 template <class K>
 static cudaError_t prep_kernel(K kernel, int smem) {
   // Opt in to the dynamic shared memory this launch needs (once per kernel).
@@ -44,7 +52,7 @@ Status xy_forward(Context& ctx, const PlanEntry& pe, const Pro& pro,
   auto k = k_xy_forward<Pro>;
   CL_CHECK(prep_kernel(k, P.xy_smem));
   note_launch_begin(KK_XY_FORWARD, ctx.exec_stream());
-  CLARITY_LAUNCH(k, P.xy_blocks, P.xy_threads, P.xy_smem, ctx.exec_stream())(P, pro, S, pe.tw,
+  CLARITY_LAUNCH(k, xy_grid(P, pro), P.xy_threads, P.xy_smem, ctx.exec_stream())(P, pro, S, pe.tw,
                                                                  pe.xrev);
   note_launch_end(KK_XY_FORWARD, ctx.exec_stream());
   CL_CHECK(cudaGetLastError());
@@ -61,7 +69,7 @@ Status xy_inverse(Context& ctx, const PlanEntry& pe, const Epi& epi,
   auto k = k_xy_inverse<Epi>;
   CL_CHECK(prep_kernel(k, P.xy_smem));
   note_launch_begin(KK_XY_INVERSE, ctx.exec_stream());
-  CLARITY_LAUNCH(k, P.xy_blocks, P.xy_threads, P.xy_smem, ctx.exec_stream())(P, epi, S, pe.tw,
+  CLARITY_LAUNCH(k, xy_grid(P, epi), P.xy_threads, P.xy_smem, ctx.exec_stream())(P, epi, S, pe.tw,
                                                                  pe.xrev);
   note_launch_end(KK_XY_INVERSE, ctx.exec_stream());
   CL_CHECK(cudaGetLastError());
@@ -78,7 +86,7 @@ Status xy_inv_fwd(Context& ctx, const PlanEntry& pe, const Mid& mid,
   auto k = k_xy_inv_fwd<Mid>;
   CL_CHECK(prep_kernel(k, P.xy_smem));
   note_launch_begin(family_of<Mid, KK_XY_INV_FWD>(), ctx.exec_stream());
-  CLARITY_LAUNCH(k, P.xy_blocks, P.xy_threads, P.xy_smem, ctx.exec_stream())(P, mid, S, pe.tw,
+  CLARITY_LAUNCH(k, xy_grid(P, mid), P.xy_threads, P.xy_smem, ctx.exec_stream())(P, mid, S, pe.tw,
                                                                  pe.xrev);
   note_launch_end(family_of<Mid, KK_XY_INV_FWD>(), ctx.exec_stream());
   CL_CHECK(cudaGetLastError());

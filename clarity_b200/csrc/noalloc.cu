@@ -154,7 +154,14 @@ extern "C" CLARITY_API ClarityResult_t clarityx_convolve_noalloc(
   pk.nx = nx; pk.ny = ny; pk.nz = nz;
   const ProPadded pro_k{pk, nullptr, P.xmode};
   const ProImage pro_i{ImageSrc{image, imageDim.x, imageDim.y, imageDim.z}, P.xmode};
-  const ModOTF mod{H, 1.0f / ((float)wd.z * wd.y * wd.x)};
+  // planes outside the kernel's and the image's extents are neither
+  // transformed nor read (as make_otf and run_convolve)
+  ModForward fwd;
+  fwd.zn = kernelDim.z - kernelDim.z / 2;
+  fwd.zh = nz - kernelDim.z / 2;
+  ModOTF mod{H, 1.0f / ((float)wd.z * wd.y * wd.x)};
+  mod.zn = mod.zout = imageDim.z;
+  const int groups = P.By / P.G;
   const EpiClip epi{out, imageDim.x, imageDim.y, imageDim.z, nullptr, P.xmode};
 
   auto kf = k_xy_forward<ProPadded>;
@@ -169,11 +176,11 @@ extern "C" CLARITY_API ClarityResult_t clarityx_convolve_noalloc(
       (e = allow_smem(ki, P.xy_smem)) != cudaSuccess)
     return fail(CLARITY_INVALID_OPERATION, cudaGetErrorString(e));
   // OTF of the shifted kernel, then R2C(image) * OTF / N, then C2R + clip
-  CLARITY_LAUNCH(kf, P.xy_blocks, P.xy_threads, P.xy_smem, st)(P, pro_k, H, tw, xrev);
-  CLARITY_LAUNCH(kzf, P.z_blocks, P.z_threads, P.z_smem, st)(P, ModForward{}, H, H, tw);
-  CLARITY_LAUNCH(kfi, P.xy_blocks, P.xy_threads, P.xy_smem, st)(P, pro_i, S, tw, xrev);
+  CLARITY_LAUNCH(kf, kernelDim.z * groups, P.xy_threads, P.xy_smem, st)(P, pro_k, H, tw, xrev);
+  CLARITY_LAUNCH(kzf, P.z_blocks, P.z_threads, P.z_smem, st)(P, fwd, H, H, tw);
+  CLARITY_LAUNCH(kfi, imageDim.z * groups, P.xy_threads, P.xy_smem, st)(P, pro_i, S, tw, xrev);
   CLARITY_LAUNCH(kzm, P.z_blocks, P.z_threads, P.z_smem, st)(P, mod, S, S, tw);
-  CLARITY_LAUNCH(ki, P.xy_blocks, P.xy_threads, P.xy_smem, st)(P, epi, S, tw, xrev);
+  CLARITY_LAUNCH(ki, imageDim.z * groups, P.xy_threads, P.xy_smem, st)(P, epi, S, tw, xrev);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(CLARITY_INVALID_OPERATION, cudaGetErrorString(e));
   return CLARITY_SUCCESS;

@@ -2,6 +2,10 @@
 //
 // Prologues (XY forward): load_c(m, y, z) returns complex row element m of
 //   row (y, z): (v[2m], v[2m+1]) for even nx, (v[m], 0) for odd nx.
+//   live_planes(nz) planes can be nonzero, plane(p) is the p-th of them and
+//   live_rows the leading rows of a line group inside the volume: the pass
+//   transforms and writes nothing else (Mod::zn, Mod::zh say the same to the
+//   z pass that reads its output).
 // Epilogues (XY inverse): apply_c(m, y, z, c) receives the same pair of
 //   real-space values after the inverse transform; the returned pair feeds
 //   the forward transform when the epilogue is fused into k_xy_inv_fwd.
@@ -94,36 +98,54 @@ struct ProWork {
     const float a = CLARITY_LDG(&v[w.idx(m, y, z)]);
     return make_float2(scale ? s * a : a, 0.f);
   }
+  int live_planes(int nz) const { return nz; }
+  __device__ __forceinline__ int plane(int p) const { return p; }
+  static constexpr bool has_zero_rows = false;
+  __device__ __forceinline__ int live_rows(int, int, int ay) const { return ay; }
   __device__ __forceinline__ void finish() const {}
 };
+
+// Rows y0base + by*j of a line group that lie below Y (j < the result).
+__device__ __forceinline__ int rows_below(int Y, int y0base, int by, int ay) {
+  const int l = (Y - y0base + by - 1) / by;
+  return l < 0 ? 0 : (l > ay ? ay : l);
+}
 
 // Extrapolated estimate of accelerated RL (Biggs-Andrews): y = max(0,
 // x + alpha (x - xp)), one fused multiply-add, stored to yout on the way into
 // the forward transform (the product step reads it back as the estimate).
+// The estimates are volumes of the image's extent (X, Y, Z): they are zero in
+// the padding (see EpiRLProduct).
 struct ProAccel {
   const float* CLARITY_RESTRICT x;
   const float* CLARITY_RESTRICT xp;
   const float* CLARITY_RESTRICT alpha;
   float* CLARITY_RESTRICT yout;
-  WorkVol w;
+  int X, Y, Z;
   int xmode;
   __device__ __forceinline__ static float extrap(float a, float x, float xp) {
     return fmaxf(0.f, fmaf(a, x - xp, x));
   }
+  __device__ __forceinline__ float one(float a, int i, int y, int z) const {
+    if (i >= X || y >= Y || z >= Z) return 0.f;
+    const unsigned o = ((unsigned)z * Y + y) * X + i;
+    const float r = extrap(a, CLARITY_LDG(x + o), CLARITY_LDG(xp + o));
+    yout[o] = r;
+    return r;
+  }
   __device__ __forceinline__ float2 load_c(int m, int y, int z) const {
     const float a = CLARITY_LDG(alpha);
     if (xmode == 0) {
-      const unsigned i = w.idx(2 * m, y, z);
-      const float2 xv = CLARITY_LDG(reinterpret_cast<const float2*>(x + i));
-      const float2 pv = CLARITY_LDG(reinterpret_cast<const float2*>(xp + i));
-      const float2 r = make_float2(extrap(a, xv.x, pv.x), extrap(a, xv.y, pv.y));
-      *reinterpret_cast<float2*>(yout + i) = r;
-      return r;
+      const float lo = one(a, 2 * m, y, z);
+      return make_float2(lo, one(a, 2 * m + 1, y, z));
     }
-    const unsigned i = w.idx(m, y, z);
-    const float r = extrap(a, CLARITY_LDG(x + i), CLARITY_LDG(xp + i));
-    yout[i] = r;
-    return make_float2(r, 0.f);
+    return make_float2(one(a, m, y, z), 0.f);
+  }
+  int live_planes(int nz) const { return Z < nz ? Z : nz; }
+  __device__ __forceinline__ int plane(int p) const { return p; }
+  static constexpr bool has_zero_rows = true;
+  __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
+    return rows_below(Y, y0base, by, ay);
   }
   __device__ __forceinline__ void finish() const {}
 };
@@ -144,16 +166,36 @@ struct ProPadded {
     if (scale) a = s * a;
     return make_float2(a, 0.f);
   }
+  // With the shift by -Z/2 the source's planes wrap around plane 0: its upper
+  // Z - Z/2 planes land on planes 0.., the others on the last Z/2.
+  int live_planes(int) const { return p.Z; }
+  __device__ __forceinline__ int plane(int q) const {
+    return q < p.Z + p.sz ? q : q + (p.nz - p.Z);
+  }
+  static constexpr bool has_zero_rows = false;
+  __device__ __forceinline__ int live_rows(int, int, int ay) const { return ay; }
   __device__ __forceinline__ void finish() const {}
 };
 
-// The padded image (zero shift) as a prologue.
+// The padded image (zero shift) as a prologue, times an optional scale.
 struct ProImage {
   ImageSrc p;
   int xmode;
+  const float* CLARITY_RESTRICT scale = nullptr;
   __device__ __forceinline__ float2 load_c(int m, int y, int z) const {
-    if (xmode == 0) return make_float2(p.at(2 * m, y, z), p.at(2 * m + 1, y, z));
-    return make_float2(p.at(m, y, z), 0.f);
+    float2 v = xmode == 0 ? make_float2(p.at(2 * m, y, z), p.at(2 * m + 1, y, z))
+                          : make_float2(p.at(m, y, z), 0.f);
+    if (scale) {
+      const float s = *scale;
+      v = make_float2(s * v.x, s * v.y);
+    }
+    return v;
+  }
+  int live_planes(int nz) const { return p.Z < nz ? p.Z : nz; }
+  __device__ __forceinline__ int plane(int q) const { return q; }
+  static constexpr bool has_zero_rows = true;
+  __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
+    return rows_below(p.Y, y0base, by, ay);
   }
   __device__ __forceinline__ void finish() const {}
 };
@@ -223,7 +265,7 @@ struct EpiWork {
 // Store only the image region (crop from the origin, src/ImageClip.cxx:41-46)
 // into an unpadded (X, Y, Z) volume, times an optional device scale.
 struct EpiClip {
-  static constexpr bool has_zero_rows = false;
+  static constexpr bool has_zero_rows = true;
   float* CLARITY_RESTRICT out;
   int X, Y, Z;
   const float* CLARITY_RESTRICT scale;
@@ -243,80 +285,86 @@ struct EpiClip {
     }
     return c;
   }
-    // padding rows / z planes where the result is known to be zero
-  __device__ __forceinline__ bool zero_row(int, int) const { return false; }
-  __device__ __forceinline__ bool zero_plane(int) const { return false; }
-  // rows y0base + BY*j, j < live_rows, can be nonzero (all here)
-  __device__ __forceinline__ int live_rows(int, int, int ay) const { return ay; }
+  // rows and planes outside the image are not asked for: not transformed
+  __device__ __forceinline__ bool zero_row(int y, int z) const { return y >= Y || z >= Z; }
+  __device__ __forceinline__ bool zero_plane(int z) const { return z >= Z; }
+  int live_planes(int nz) const { return Z < nz ? Z : nz; }
+  __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
+    return rows_below(Y, y0base, by, ay);
+  }
   __device__ __forceinline__ void prefetch_row(int, int) const {}
   __device__ __forceinline__ void finish() {}
 };
 
 // RL step 4 (src/MaximumLikelihoodDeconvolve.cxx:69-70) with the flux sum of
-// step 5 (:73-74): u_new = cur * c, cur = scale * u (or the padded image on
-// the first iteration), partial sums of u_new in FP64.
+// step 5 (:73-74): u_new = cur * c, cur = scale * u, partial sums of u_new in
+// FP64.  The first estimate is zero outside its extent (X, Y, Z) -- the image's,
+// or the whole work box where a caller starts from a work-box volume -- and a
+// product keeps it zero there, so cur and u_new are volumes of that extent and
+// the pass transforms only its rows and planes.  At the 512x512x128 box with a
+// 256x256x64 image that is an eighth of the work-box volume and a quarter of
+// its rows: the pass went from 176 to 112 us.
 struct EpiRLProduct {
-  static constexpr bool has_zero_rows = false;
+  static constexpr bool has_zero_rows = true;
   static constexpr int kFamily = KK_XY_PRODUCT;
-  const float* CLARITY_RESTRICT cur;     // work-box estimate, or nullptr
-  ImageSrc g;                        // used when cur == nullptr
-  const float* CLARITY_RESTRICT scale;   // deferred flux scale for cur
+  const float* CLARITY_RESTRICT cur;     // the estimate (X, Y, Z)
+  int X, Y, Z;
+  const float* CLARITY_RESTRICT scale;   // deferred flux scale for cur, or nullptr
   float* CLARITY_RESTRICT unew;
   double* CLARITY_RESTRICT partial;
-  WorkVol w;
   int xmode;
   double acc;
   int* nblocks = nullptr;  // receives the grid size (the number of partials), or nullptr
-  __device__ __forceinline__ float cur_at(int x, int y, int z) const {
-    if (cur) {
-      const float u = CLARITY_LDG(&cur[w.idx(x, y, z)]);
-      return scale ? *scale * u : u;
-    }
-    return g.at(x, y, z);
+  __device__ __forceinline__ unsigned at(int x, int y, int z) const {
+    return ((unsigned)z * Y + y) * X + x;
+  }
+  __device__ __forceinline__ float one(int x, int y, int z, float c) {
+    if (x >= X || y >= Y || z >= Z) return 0.f;
+    float u = CLARITY_LDG(&cur[at(x, y, z)]);
+    if (scale) u = *scale * u;
+    const float a = u * c;
+    unew[at(x, y, z)] = a;
+    acc += (double)a;
+    return a;
   }
   __device__ __forceinline__ float2 apply_c(int m, int y, int z, float2 c) {
     if (xmode == 0) {
-      const float a = cur_at(2 * m, y, z) * c.x;
-      const float b = cur_at(2 * m + 1, y, z) * c.y;
-      *reinterpret_cast<float2*>(unew + w.idx(2 * m, y, z)) = make_float2(a, b);
-      acc += (double)a;
-      acc += (double)b;
-      return make_float2(a, b);
+      const float a = one(2 * m, y, z, c.x);
+      return make_float2(a, one(2 * m + 1, y, z, c.y));
     }
-    const float a = cur_at(m, y, z) * c.x;
-    unew[w.idx(m, y, z)] = a;
-    acc += (double)a;
-    return make_float2(a, 0.f);
+    return make_float2(one(m, y, z, c.x), 0.f);
   }
-    // padding rows / z planes where the result is known to be zero
-  __device__ __forceinline__ bool zero_row(int, int) const { return false; }
-  __device__ __forceinline__ bool zero_plane(int) const { return false; }
-  // rows y0base + BY*j, j < live_rows, can be nonzero (all here)
-  __device__ __forceinline__ int live_rows(int, int, int ay) const { return ay; }
+  __device__ __forceinline__ bool zero_row(int y, int z) const { return y >= Y || z >= Z; }
+  __device__ __forceinline__ bool zero_plane(int z) const { return z >= Z; }
+  int live_planes(int nz) const { return Z < nz ? Z : nz; }
+  __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
+    return rows_below(Y, y0base, by, ay);
+  }
   // the estimate row this block's epilogue will read, into L2
   __device__ __forceinline__ void prefetch_row(int y, int z) const {
-    if (cur) prefetch_l2_range(cur + w.idx(0, y, z), sizeof(float) * (size_t)w.nx);
+    if (y < Y && z < Z) prefetch_l2_range(cur + at(0, y, z), sizeof(float) * (size_t)X);
   }
-  // Staged form (passes_xy_tma.cuh): row (y, z) of cur (or of the image on
-  // the first iteration) arrives in shared memory; u' overwrites it there and
-  // leaves by a bulk store to unew.
+  // Staged form (passes_xy_tma.cuh): row (y, z) of cur arrives in shared
+  // memory; u' overwrites it there and leaves for unew as whole rows.
   static constexpr bool kStaged = true;
   static constexpr bool kStoreRows = true;
   __device__ __forceinline__ st::RowRef in_row(int y, int z) const {
-    if (cur) return {cur + w.idx(0, y, z), w.nx};
-    if (y < g.Y && z < g.Z) return {g.src + ((unsigned)z * g.Y + y) * g.X, g.X};
+    if (y < Y && z < Z) return {cur + at(0, y, z), X};
     return {nullptr, 0};
   }
-  __device__ __forceinline__ float* out_row(int y, int z) const { return unew + w.idx(0, y, z); }
+  __device__ __forceinline__ float* out_row(int y, int z) const {
+    return y < Y && z < Z ? unew + at(0, y, z) : nullptr;
+  }
   __device__ __forceinline__ float2 apply_s(int m, int, int, float2 c, float* sr, int n) {
     const int x = 2 * m;
     float u0 = x < n ? sr[x] : 0.f, u1 = x + 1 < n ? sr[x + 1] : 0.f;
-    if (cur && scale) {
+    if (scale) {
       const float s = CLARITY_LDG(scale);
       u0 = s * u0;
       u1 = s * u1;
     }
-    const float a = u0 * c.x, b = u1 * c.y;
+    // outside the estimate the product is zero whatever c is there
+    const float a = x < n ? u0 * c.x : 0.f, b = x + 1 < n ? u1 * c.y : 0.f;
     sr[x] = a;
     sr[x + 1] = b;
     acc += (double)a;
@@ -326,6 +374,13 @@ struct EpiRLProduct {
   __device__ __forceinline__ void finish() {
     block_sum_store(acc, partial);
     if (nblocks && CLARITY_BLOCK_ID() == 0 && threadIdx.x == 0) *nblocks = (int)CLARITY_GRID_DIM();
+  }
+  // a block whose plane lies outside the estimate contributes zero
+  __device__ __forceinline__ void finish_skipped() {
+    if (threadIdx.x == 0) {
+      partial[CLARITY_BLOCK_ID()] = 0.0;
+      if (nblocks && CLARITY_BLOCK_ID() == 0) *nblocks = (int)CLARITY_GRID_DIM();
+    }
   }
 };
 
@@ -376,8 +431,7 @@ struct MidRLRatio {
   int live_planes(int nz) const { return g.Z < nz ? g.Z : nz; }
   // rows y0base + by*j with j < live_rows lie inside the image (y < Y)
   __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
-    const int l = (g.Y - y0base + by - 1) / by;
-    return l < 0 ? 0 : (l > ay ? ay : l);
+    return rows_below(g.Y, y0base, by, ay);
   }
   __device__ __forceinline__ void prefetch_row(int y, int z) const {
     if (y < g.Y && z < g.Z)
@@ -475,9 +529,11 @@ struct ModOTF {
   const float2* CLARITY_RESTRICT H;
   float scale;
   const float* CLARITY_RESTRICT scale2 = nullptr;
-  // only the first zn z planes of the input spectrum are nonzero (the rest
-  // were never written and are read as zeros)
+  // only the z planes z < zn and z >= zh of the input spectrum are nonzero
+  // (the rest were never written and are read as zeros); no plane lies at or
+  // beyond the default zh
   int zn = 1 << 30;
+  int zh = 1 << 30;
   // only the first zout z planes of the output are read by the next pass:
   // the rest are neither inverse-transformed along y0 nor stored
   int zout = 1 << 30;
@@ -512,6 +568,7 @@ struct ModWiener {
   const float2* CLARITY_RESTRICT H;
   float eps, scale;
   int zn = 1 << 30;
+  int zh = 1 << 30;
   int zout = 1 << 30;
   __device__ __forceinline__ void prefetch_tile(unsigned base, int tile, int p, int np) const {
     const size_t chunk = ((size_t)tile * 8 / np + 15) & ~size_t(15);
@@ -533,6 +590,7 @@ struct ModWiener {
 struct ModForward {
   static constexpr bool forward_only = true;
   int zn = 1 << 30;
+  int zh = 1 << 30;
   int zout = 1 << 30;
   __device__ __forceinline__ void prefetch_tile(unsigned, int, int, int) const {}
   __device__ __forceinline__ float2 apply(long long, float2 v) const { return v; }

@@ -523,8 +523,9 @@ __device__ __forceinline__ void xy_forward_body(float2* sm, const VolPlan& P, co
                                                 const float2* CLARITY_RESTRICT tw,
                                                 const int* CLARITY_RESTRICT xrev, int bid) {
   const int ngroups = P.By / P.G;
-  const int z = bid / ngroups;
-  const int y0base = (bid - z * ngroups) * P.G;
+  const int p = bid / ngroups;
+  const int z = pro.plane(p);
+  const int y0base = (bid - p * ngroups) * P.G;
   const float2* twx = tw + P.ax.tw_off;
   x_first_pass_rt(sm, P, pro, z, y0base, twx);
   __syncthreads();
@@ -589,17 +590,18 @@ __device__ __forceinline__ void z_body(float2* sm, const VolPlan& P, const Mod& 
   const long long base = (long long)bid * tile;
   // load (16-byte vectors when the tile size is even, which keeps every
   // tile base 16-byte aligned)
-  // planes z >= zn of the input are zero (not read)
+  // planes zn <= z < zh of the input are zero (not read)
   const long long live = (long long)(mod.zn < P.nz ? mod.zn : P.nz) * P.By * P.W;
-  if ((tile & 1) == 0 && (live & 1) == 0) {
+  const long long high = (long long)(mod.zh < P.nz ? mod.zh : P.nz) * P.By * P.W;
+  if ((tile & 1) == 0 && (live & 1) == 0 && (high & 1) == 0) {
     const float4* src = reinterpret_cast<const float4*>(Sin + base);
     float4* dst = reinterpret_cast<float4*>(sm);
-    const int n4 = (int)(tile / 2), live4 = (int)(live / 2);
+    const int n4 = (int)(tile / 2), live4 = (int)(live / 2), high4 = (int)(high / 2);
     for (int t = threadIdx.x; t < n4; t += blockDim.x)
-      dst[t] = t < live4 ? CLARITY_LDG(&src[t]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      dst[t] = t < live4 || t >= high4 ? CLARITY_LDG(&src[t]) : make_float4(0.f, 0.f, 0.f, 0.f);
   } else {
     for (int t = threadIdx.x; t < tile; t += blockDim.x)
-      sm[t] = t < live ? Sin[base + t] : make_float2(0.f, 0.f);
+      sm[t] = t < live || t >= high ? Sin[base + t] : make_float2(0.f, 0.f);
   }
   __syncthreads();
   const int BW = P.By * P.W;

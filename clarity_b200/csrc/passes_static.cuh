@@ -146,7 +146,7 @@ __device__ __forceinline__ int visit_rows(int L) {
 }
 template <class SH, bool COMPACT>
 __device__ __forceinline__ int visit_row(int rv, int L) {
-  if constexpr (!COMPACT) return rv;
+  if constexpr (!COMPACT || SH::G == 1) return rv;
   const int g = rv / L;
   return g * SH::AY + (rv - g * L);
 }
@@ -211,16 +211,30 @@ __device__ __forceinline__ void x_inverse_down_to(float2* sm, const float2* tw,
   }
 }
 
-// First x pass straight from HBM through the prologue.
+// Rows j >= L of every line group set to zero.
+template <class SH>
+__device__ __forceinline__ void zero_dead_rows(float2* sm, int L) {
+  const int dead = SH::G * (SH::AY - L) * SH::ROWSTRIDE;
+  for (int t = threadIdx.x; t < dead; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
+    const int rd = t / SH::ROWSTRIDE, e = t - rd * SH::ROWSTRIDE;
+    const int g = rd / (SH::AY - L), j = L + (rd - g * (SH::AY - L));
+    sm[g * SH::GSTRIDE + j * SH::ROWSTRIDE + e] = make_float2(0.f, 0.f);
+  }
+}
+
+// First x pass straight from HBM through the prologue (rows j < L of each
+// group; the others are zero).
 template <class SH, class Pro>
 __device__ __forceinline__ void x_first(float2* sm, const Pro& pro, int z, int y0base,
-                                        const float2* __restrict__ tw) {
+                                        const float2* __restrict__ tw, int L) {
   using X = typename SH::X;
-  constexpr int R = X::radix(0), span = X::span(0), total = SH::ROWS * span;
+  constexpr int R = X::radix(0), span = X::span(0);
+  const int total = visit_rows<SH, Pro::has_zero_rows>(L) * span;
 #pragma unroll 1
   for (int f = threadIdx.x; f < total; f += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
-    const int r = f / span;
-    const int i = f - r * span;
+    const int rv = f / span;
+    const int r = visit_row<SH, Pro::has_zero_rows>(rv, L);
+    const int i = f - rv * span;
     const int g = r / SH::AY, j = r - g * SH::AY;
     const int y = y0base + g + SH::BY * j;
     float2 v[R];
@@ -555,11 +569,14 @@ template <class SH, class Pro>
 __global__ void __launch_bounds__(SH::THREADS, SH::XY_MINB)
     ks_xy_forward(const Pro pro, float2* __restrict__ S, const Tables T) {
   CLARITY_DYN_SMEM(float2, sm);
-  const int z = blockIdx.x / SH::NGROUPS;
-  const int y0base = (blockIdx.x - z * SH::NGROUPS) * SH::G;
-  x_first<SH>(sm, pro, z, y0base, T.twx);
+  const int p = blockIdx.x / SH::NGROUPS;
+  const int y0base = (blockIdx.x - p * SH::NGROUPS) * SH::G;
+  const int z = pro.plane(p);
+  const int L = pro.live_rows(y0base, SH::BY, SH::AY);
+  x_first<SH>(sm, pro, z, y0base, T.twx, L);
+  if constexpr (Pro::has_zero_rows) zero_dead_rows<SH>(sm, L);
   __syncthreads();
-  x_forward_from<SH, 1>(sm, T.twx);
+  x_forward_from<SH, 1, NoSkip, Pro::has_zero_rows>(sm, T.twx, NoSkip{}, L);
   cols_forward<SH>(sm, S, z, y0base, T.twr, T.twny);
   pro.finish();
 }
@@ -584,8 +601,10 @@ __global__ void __launch_bounds__(SH::THREADS, SH::XY_MINB)
   prefetch_tile_rows<SH>(epi, z, y0base);
   cols_inverse<SH>(sm, S, z, y0base, T.twr, T.twny);
   __syncthreads();
-  x_inverse_down_to<SH, 1>(sm, T.twx);
-  x_last<SH, Epi, false>(sm, epi, z, y0base, T.twx);
+  constexpr bool CP = Epi::has_zero_rows;  // rows j < L are all the epilogue wants
+  const int L = epi.live_rows(y0base, SH::BY, SH::AY);
+  x_inverse_down_to<SH, 1, NoSkip, CP>(sm, T.twx, NoSkip{}, L);
+  x_last<SH, Epi, false, NoSkip, CP>(sm, epi, z, y0base, T.twx, NoSkip{}, L);
   epi.finish();
 }
 
@@ -610,12 +629,7 @@ __global__ void __launch_bounds__(SH::THREADS, SH::XY_MINB)
     const int L = mid.live_rows(y0base, SH::BY, SH::AY);
     x_inverse_down_to<SH, 1, RowSkip<SH, Mid>, true>(sm, T.twx, skip, L);
     x_last<SH, Mid, true, RowSkip<SH, Mid>, true>(sm, mid, z, y0base, T.twx, skip, L);
-    const int dead = SH::G * (SH::AY - L) * SH::ROWSTRIDE;
-    for (int t = threadIdx.x; t < dead; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
-      const int rd = t / SH::ROWSTRIDE, e = t - rd * SH::ROWSTRIDE;
-      const int g = rd / (SH::AY - L), j = L + (rd - g * (SH::AY - L));
-      sm[g * SH::GSTRIDE + j * SH::ROWSTRIDE + e] = make_float2(0.f, 0.f);
-    }
+    zero_dead_rows<SH>(sm, L);
     __syncthreads();
     x_forward_from<SH, 1, RowSkip<SH, Mid>, true>(sm, T.twx, skip, L);
   } else {
@@ -657,15 +671,16 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
   if (threadIdx.x < 16) mod.prefetch_tile((unsigned)base, tile, threadIdx.x, 16);
   static_assert(tile % 2 == 0, "tile must be even");
   {
-    // planes z >= zn are zero; BW is even so a float4 never spans two planes
+    // planes zn <= z < zh are zero; BW is even so a float4 never spans two planes
     static_assert(SH::BW % 2 == 0, "tile rows must hold whole float4s");
     const int zn = mod.zn < SH::NZ ? mod.zn : SH::NZ;
-    const int live4 = zn * SH::BW / 2;
+    const int zh = mod.zh < SH::NZ ? mod.zh : SH::NZ;
+    const int live4 = zn * SH::BW / 2, high4 = zh * SH::BW / 2;
     const float4* src = reinterpret_cast<const float4*>(Sin + base);
     float4* dst = reinterpret_cast<float4*>(sm);
 #pragma unroll 4
     for (int t = threadIdx.x; t < tile / 2; t += CLARITY_BLOCK_STRIDE(SH::THREADS))
-      dst[t] = t < live4 ? __ldg(&src[t]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      dst[t] = t < live4 || t >= high4 ? __ldg(&src[t]) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
   tile_forward_from<SH, typename SH::Y, 0, false>(sm, T.twy);
@@ -791,7 +806,9 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
   constexpr bool BULK = (BW * 8) % 16 == 0 && (ZS * 8) % 16 == 0;
   using A = typename SH::Z;
   const unsigned gbase = blockIdx.x * (unsigned)SH::TILE;
-  const int zn = mod.zn < NZ ? mod.zn : NZ;  // planes z >= zn are zero
+  // planes zn <= z < zh are zero: the q-th live plane is q, or q + gap
+  const int zn = mod.zn < NZ ? mod.zn : NZ;
+  const int gap = (mod.zh < NZ ? mod.zh : NZ) - zn;
   if (threadIdx.x < 16) mod.prefetch_tile(gbase, SH::TILE, threadIdx.x, 16);
   // z twiddles in shared memory: a z-pass task's twiddle is the same for all
   // lanes of a warp (a broadcast), where the table in global memory cost an
@@ -809,10 +826,12 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
     if ((int)threadIdx.x < CLARITY_ISSUE_LANES) {
-      if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, (uint32_t)(zn * BW * 8));
+      if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, (uint32_t)((NZ - gap) * BW * 8));
       __syncwarp();
-      for (int z = threadIdx.x; z < zn; z += CLARITY_ISSUE_LANES)
+      for (int q = threadIdx.x; q < NZ - gap; q += CLARITY_ISSUE_LANES) {
+        const int z = q < zn ? q : q + gap;
         bulk_load(sm + z * ZS, Sin + gbase + z * BW, BW * 8, &bar);
+      }
     }
     if (!mbar_wait(&bar, 0, T.err)) {
       mbar_wait(&bar, 0, nullptr);  // give copies in flight a last chance
@@ -825,7 +844,7 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
     const int ki = l % W, z = l / W;
     float2 v[BY];
     float2* d = sm + z * ZS + ki;
-    if (z >= zn) {  // known-zero plane: its transform is zero
+    if (z >= zn && z < zn + gap) {  // known-zero plane: its transform is zero
 #pragma unroll
       for (int k = 0; k < BY; ++k) d[k * W] = make_float2(0.f, 0.f);
       continue;

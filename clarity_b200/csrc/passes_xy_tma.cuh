@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(256, 3)
   float* stg = reinterpret_cast<float*>(buf + X::BUF_F2);
   __shared__ alignas(8) uint64_t bars[2];
   __shared__ int nf[X::NROWS];
-  __shared__ int bulk_ok;
+  __shared__ int bulk_ok, bulk_out;
   constexpr int NB = SH::BY / X::TG;
   const int z = blockIdx.x / NB;
   const int y0base = (blockIdx.x - z * NB) * X::TG;
@@ -361,14 +361,20 @@ __global__ void __launch_bounds__(256, 3)
     return;
   }
   if (threadIdx.x == 0) {
-    int ok = 1;
+    int ok = 1, out_ok = 1;
     for (int r = 0; r < X::NROWS; ++r) {
       const int g = r / X::AY, j = r - g * X::AY;
       const RowRef rr = epi.in_row(y0base + g + SH::BY * j, z);
       nf[r] = rr.nf;
       if (rr.nf > 0 && (((uintptr_t)rr.p & 15u) != 0 || (rr.nf & 3) != 0)) ok = 0;
+      if constexpr (Epi::kStoreRows) {
+        // the output rows have the input rows' extent
+        const float* o = epi.out_row(y0base + g + SH::BY * j, z);
+        if (o && (((uintptr_t)o & 15u) != 0 || (rr.nf & 3) != 0)) out_ok = 0;
+      }
     }
     bulk_ok = ok;
+    bulk_out = out_ok;
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
   }
@@ -436,28 +442,27 @@ __global__ void __launch_bounds__(256, 3)
     // bulk stores while the forward transform runs
     fence_smem_to_async();
     __syncthreads();
+    const bool rows_bulk = bulk_out != 0;
     if (threadIdx.x < 32) {
       for (int r = threadIdx.x; r < X::NROWS; r += CLARITY_ISSUE_LANES) {
         const int g = r / X::AY, j = r - g * X::AY;
         float* dst = epi.out_row(y0base + g + SH::BY * j, z);
-        if (((uintptr_t)dst & 15u) == 0) {
-          bulk_store(dst, stg + r * X::NX, 4u * X::NX);
-        } else {
-          for (int x = 0; x < X::NX; ++x) dst[x] = stg[r * X::NX + x];
-        }
+        if (dst && rows_bulk) bulk_store(dst, stg + r * X::NX, 4u * (uint32_t)nf[r]);
       }
       bulk_commit();
+    }
+    if (!rows_bulk) {  // rows that are not 16-byte runs: plain stores
+      for (int t = threadIdx.x; t < X::STG_F; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
+        const int r = t / X::NX, x = t - r * X::NX;
+        const int g = r / X::AY, j = r - g * X::AY;
+        float* dst = epi.out_row(y0base + g + SH::BY * j, z);
+        if (dst && x < nf[r]) dst[x] = stg[t];
+      }
     }
   }
   if constexpr (FUSE) {
     if constexpr (CP) {
-      // rows j >= L of each group are zero
-      const int dead = X::TG * (SH::AY - L) * TS::ROWSTRIDE;
-      for (int t = threadIdx.x; t < dead; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
-        const int rd = t / TS::ROWSTRIDE, e = t - rd * TS::ROWSTRIDE;
-        const int g = rd / (SH::AY - L), j = L + (rd - g * (SH::AY - L));
-        buf[g * TS::GSTRIDE + j * TS::ROWSTRIDE + e] = make_float2(0.f, 0.f);
-      }
+      zero_dead_rows<TS>(buf, L);
     }
     __syncthreads();
     x_forward_from<TS, 1, RowSkip<TS, Epi>, CP>(buf, twx, skip, L);

@@ -46,6 +46,14 @@ inline st::Tables tables_of(const PlanEntry& pe) {
                     pe.tw + P.tw_r2c_off, pe.tw + P.tw_ny_off, pe.err};
 }
 
+// Planes a launch covers: all of them, or those a functor says can be nonzero
+// (or are wanted).
+template <class F>
+inline int launch_planes(const F& f, int nz) {
+  if constexpr (requires { f.live_planes(nz); }) return f.live_planes(nz);
+  else return nz;
+}
+
 template <class K>
 inline cudaError_t allow_smem_st(K kernel, int smem) {
   return smem_opt_in(reinterpret_cast<const void*>(kernel), smem);
@@ -95,10 +103,7 @@ inline bool try_xy_tma(const PlanEntry& pe, cudaStream_t st, const F& fn, const 
     *err = allow_smem_st(k, X::SMEM);
     if (*err != cudaSuccess) return true;
     const st::Tables T = tables_of(pe);
-    // planes known to be zero need no block at all
-    int nz = SH::NZ;
-    if constexpr (requires { fn.live_planes(1); }) nz = fn.live_planes(SH::NZ);
-    const int blocks = nz * (SH::BY / X::TG);
+    const int blocks = launch_planes(fn, SH::NZ) * (SH::BY / X::TG);
     if (blocks <= 0) return true;
     note_launch_begin(family, st);
     CLARITY_LAUNCH_PDL(k, blocks, SH::THREADS, X::SMEM, st, pdl_enabled())(fn, tm, T);
@@ -128,7 +133,8 @@ inline bool try_static(const PlanEntry& pe, cudaStream_t st, const F& fn, float2
     *err = allow_smem_st(k, SH::XY_SMEM);
     if (*err != cudaSuccess) return true;
     note_launch_begin(KK_XY_FORWARD, st);
-    CLARITY_LAUNCH(k, pe.P.xy_blocks, SH::THREADS, SH::XY_SMEM, st)(fn, Sa, T);
+    CLARITY_LAUNCH(k, launch_planes(fn, SH::NZ) * SH::NGROUPS, SH::THREADS, SH::XY_SMEM, st)
+    (fn, Sa, T);
     note_launch_end(KK_XY_FORWARD, st);
   } else if constexpr (KIND == 1) {
     if constexpr (SH::Y_PER_LINE) {
@@ -161,7 +167,8 @@ inline bool try_static(const PlanEntry& pe, cudaStream_t st, const F& fn, float2
     *err = allow_smem_st(k, SH::XY_SMEM);
     if (*err != cudaSuccess) return true;
     note_launch_begin(family_of<F, KK_XY_INV_FWD>(), st);
-    CLARITY_LAUNCH(k, pe.P.xy_blocks, SH::THREADS, SH::XY_SMEM, st)(fn, Sa, T);
+    CLARITY_LAUNCH(k, launch_planes(fn, SH::NZ) * SH::NGROUPS, SH::THREADS, SH::XY_SMEM, st)
+    (fn, Sa, T);
     note_launch_end(family_of<F, KK_XY_INV_FWD>(), st);
   } else {
     if (try_xy_tma<SH, false>(pe, st, fn, Sb, KK_XY_INVERSE, err)) return true;
@@ -169,7 +176,8 @@ inline bool try_static(const PlanEntry& pe, cudaStream_t st, const F& fn, float2
     *err = allow_smem_st(k, SH::XY_SMEM);
     if (*err != cudaSuccess) return true;
     note_launch_begin(KK_XY_INVERSE, st);
-    CLARITY_LAUNCH(k, pe.P.xy_blocks, SH::THREADS, SH::XY_SMEM, st)(fn, Sb, T);
+    CLARITY_LAUNCH(k, launch_planes(fn, SH::NZ) * SH::NGROUPS, SH::THREADS, SH::XY_SMEM, st)
+    (fn, Sb, T);
     note_launch_end(KK_XY_INVERSE, st);
   }
   *err = cudaGetLastError();

@@ -247,3 +247,21 @@ def test_emulated_idiv_restoration_zero_iterations_returns_the_image(emu, tmp_pa
     out = run_emu(emu, tmp_path, "idiv", img, d["psf"], 0)
     assert out.min() >= 0
     assert rel_l2(out, np.maximum(img, 0)) <= 1e-6
+
+
+@pytest.mark.parametrize("ishape,kshape", [((20, 30, 40), (12, 34, 24)),   # even PSF depth
+                                           ((25, 29, 41), (7, 35, 23)),    # odd, rows not 16-byte
+                                           ((31, 63, 63), (1, 1, 1)),      # one PSF plane
+                                           ((10, 20, 30), (1, 10, 6))])    # runtime-planned box
+def test_emulated_single_pass_filters_with_uneven_split(emu, tmp_path, ishape, kshape, oracle_lib):
+    # the first passes transform the image's and the PSF's planes only (the
+    # PSF's wrap around plane 0) and the last one the image's; the z pass
+    # reads and writes no others
+    r = syn.rng(7 + sum(kshape))
+    img = (r.random(ishape) * 100).astype(np.float32)
+    psf = syn.gaussian_psf(kshape, 1.5, 2.0).astype(np.float32)
+    want = oracle_lib.convolve(img, psf)
+    assert rel_l2(run_emu(emu, tmp_path, "convolve", img, psf, 0), want) <= 1e-6
+    assert rel_l2(run_emu(emu, tmp_path, "convolve_noalloc", img, psf, 0), want) <= 1e-6
+    assert rel_l2(run_emu(emu, tmp_path, "wiener", img, psf, 1e-2),
+                  oracle_lib.wiener(img, psf, 1e-2)) <= 2e-6
