@@ -361,13 +361,15 @@ __global__ void k_copy(const float* __restrict__ a, float* __restrict__ b,
 static constexpr int kReduceBlocks = 592;  // 4 x 148 SMs
 
 // hc = conj(h) over a spectrum: the OTF of the reflected kernel h(-x), whose
-// product is a correlation with h.
+// product is a correlation with h.  pair: the column-pair layout (the real
+// parts of two columns, then the imaginary parts), where n counts its float2.
 __global__ void k_conj_spectrum(const float2* __restrict__ h, float2* __restrict__ hc,
-                                long long n) {
+                                long long n, int pair) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     const float2 v = h[i];
-    hc[i] = make_float2(v.x, -v.y);
+    if (pair) hc[i] = (i & 1) ? make_float2(-v.x, -v.y) : v;
+    else hc[i] = make_float2(v.x, -v.y);
   }
 }
 
@@ -466,14 +468,20 @@ Status Context::init() {
   return Status::Ok();
 }
 
+static void free_entry(PlanEntry& pe) {
+  cudaFree(pe.tw);
+  cudaFree(pe.xrev);
+  cudaFree(pe.pair_tw);
+  cudaFree(pe.pair_slots);
+}
+
 Context::~Context() {
   cudaSetDevice(device_);
   release_workspaces();
   for (cudaStream_t b : bstreams_) cudaStreamDestroy(b);
   bstreams_.clear();
   for (auto& kv : plans_) {
-    cudaFree(kv.second->tw);
-    cudaFree(kv.second->xrev);
+    free_entry(*kv.second);
   }
   plans_.clear();
   if (stream_) cudaStreamDestroy(stream_);
@@ -557,34 +565,42 @@ void Context::add_graph(std::vector<unsigned long long> key, cudaGraphExec_t g) 
   graphs_.push_back(GraphEntry{std::move(key), g});
 }
 
-Status Context::build_entry(const VolPlan& P0, std::unique_ptr<PlanEntry>* out) {
-  auto pe = std::make_unique<PlanEntry>();
-  pe->P = P0;
-  const VolPlan& P = pe->P;
-  CL_CHECK(dev_alloc((void**)&pe->tw, sizeof(float2) * P.twiddle_count));
-  CL_CHECK(dev_alloc((void**)&pe->xrev, sizeof(int) * std::max(P.xrev_count, 1)));
-  pe->err = err_dev_;
-  std::vector<int> rev;
-  std::vector<TwTable> tabs;
-  plan_tables(P, &rev, &tabs);
+// Twiddle tables and slot table of one plan, on the device.
+static Status upload_tables(const std::vector<int>& slots, const std::vector<TwTable>& tabs,
+                            int twiddles, cudaStream_t st, float2** tw, int** dslots) {
+  CL_CHECK(dev_alloc((void**)tw, sizeof(float2) * (size_t)twiddles));
+  CL_CHECK(dev_alloc((void**)dslots, sizeof(int) * std::max<size_t>(slots.size(), 1)));
   TwTable* dtabs = nullptr;
   CL_CHECK(dev_alloc((void**)&dtabs, sizeof(TwTable) * tabs.size()));
-  cudaStream_t st = exec_stream();
-  CL_CHECK(cudaMemcpyAsync(pe->xrev, rev.data(), sizeof(int) * rev.size(),
+  CL_CHECK(cudaMemcpyAsync(*dslots, slots.data(), sizeof(int) * slots.size(),
                            cudaMemcpyHostToDevice, st));
   CL_CHECK(cudaMemcpyAsync(dtabs, tabs.data(), sizeof(TwTable) * tabs.size(),
                            cudaMemcpyHostToDevice, st));
-  CLARITY_LAUNCH(k_gen_twiddles, 64, 256, 0, st)(pe->tw, dtabs, (int)tabs.size());
+  CLARITY_LAUNCH(k_gen_twiddles, 64, 256, 0, st)(*tw, dtabs, (int)tabs.size());
   CL_CHECK(cudaGetLastError());
   CL_CHECK(cudaStreamSynchronize(st));
   cudaFree(dtabs);
-  *out = std::move(pe);
   return Status::Ok();
 }
 
-static void free_entry(PlanEntry& pe) {
-  cudaFree(pe.tw);
-  cudaFree(pe.xrev);
+// pair: plan the column-pair passes too, for boxes without compile-time
+// kernels.
+Status Context::build_entry(const VolPlan& P0, bool pair, std::unique_ptr<PlanEntry>* out) {
+  auto pe = std::make_unique<PlanEntry>();
+  pe->P = P0;
+  pe->err = err_dev_;
+  cudaStream_t st = exec_stream();
+  std::vector<int> slots;
+  std::vector<TwTable> tabs;
+  plan_tables(P0, &slots, &tabs);
+  CL_TRY(upload_tables(slots, tabs, P0.twiddle_count, st, &pe->tw, &pe->xrev));
+  if (pair && static_family_mask() == 0xF && !has_static_shape(P0) &&
+      make_pair_plan(P0.nx, P0.ny, P0.nz, &pe->pair)) {
+    pair_tables(pe->pair, &slots, &tabs);
+    CL_TRY(upload_tables(slots, tabs, pe->pair.twiddle_count, st, &pe->pair_tw, &pe->pair_slots));
+  }
+  *out = std::move(pe);
+  return Status::Ok();
 }
 
 Status Context::plan(const Dims& wd, const PlanEntry** out) {
@@ -610,7 +626,7 @@ Status Context::plan(const Dims& wd, const PlanEntry** out) {
               std::to_string(wd.y) + "x" + std::to_string(wd.z) + ": " + why;
       return s;
     }
-    CL_TRY(build_entry(P, &pe));
+    CL_TRY(build_entry(P, true, &pe));
   }
   *out = pe.get();
   plans_[key] = std::move(pe);
@@ -696,17 +712,16 @@ Status Context::workspace_slot(int slot, const PlanEntry& pe, const Dims& img, c
 static Status fill_workspace(Workspace& w, const PlanEntry& pe, const Dims& img,
                              const Dims& ker) {
   const VolPlan& P = pe.P;
-  long long sc = w.spec_cap;
+  const long long spec = pe.spec_elems();
   Status s;
-  if (w.spec_cap < P.spec_elems || !w.S || !w.H) {
+  if (w.spec_cap < spec || !w.S || !w.H) {
     cudaFree(w.S); cudaFree(w.H); cudaFree(w.HG);
     w.S = w.H = w.HG = nullptr;
     w.spec_cap = 0;
-    CL_CHECK(dev_alloc((void**)&w.S, sizeof(float2) * (size_t)P.spec_elems));
-    CL_CHECK(dev_alloc((void**)&w.H, sizeof(float2) * (size_t)P.spec_elems));
-    w.spec_cap = P.spec_elems;
+    CL_CHECK(dev_alloc((void**)&w.S, sizeof(float2) * (size_t)spec));
+    CL_CHECK(dev_alloc((void**)&w.H, sizeof(float2) * (size_t)spec));
+    w.spec_cap = spec;
   }
-  (void)sc;
   s = ensure(&w.u, &w.work_cap, P.n_real());
   if (!s.ok()) return s;
   long long ic = (long long)w.img_cap, kc = (long long)w.ker_cap;
@@ -720,6 +735,7 @@ static Status fill_workspace(Workspace& w, const PlanEntry& pe, const Dims& img,
   // one partial per XY block: at most one block per (z, y0) line
   s = ensure(&w.partial, &pc,
              std::max<long long>({(long long)P.xy_blocks, (long long)P.nz * P.By,
+                                  (long long)P.nz * pe.pair.By,
                                   (long long)kReduceBlocks, 1}));
   if (!s.ok()) return s;
   w.partial_cap = (int)pc;
@@ -816,8 +832,16 @@ Status Context::tune(const Dims& wd, std::unique_ptr<PlanEntry>* out) {
             "x" + std::to_string(wd.z) + ": " + why;
     return s;
   }
-  if (nc == 1) return build_entry(cand[0], out);
-  long long spec = 0, parts = kReduceBlocks;
+  // the default plan with the column-pair passes where they serve the box
+  // (candidate -1), then the planner's tilings of the other passes
+  std::unique_ptr<PlanEntry> first;
+  CL_TRY(build_entry(cand[0], true, &first));
+  if (nc == 1 && !first->pair.ok) {
+    *out = std::move(first);
+    return Status::Ok();
+  }
+  long long spec = first->spec_elems();
+  long long parts = std::max<long long>(kReduceBlocks, (long long)wd.z * first->pair.By);
   for (int c = 0; c < nc; ++c) {
     spec = std::max(spec, cand[c].spec_elems);
     parts = std::max<long long>({parts, (long long)cand[c].xy_blocks,
@@ -840,9 +864,10 @@ Status Context::tune(const Dims& wd, std::unique_ptr<PlanEntry>* out) {
     CL_CHECK(cudaEventCreate(&e0));
     CL_CHECK(cudaEventCreate(&e1));
     const ImageSrc g{u, wd.x, wd.y, wd.z};
-    for (int c = 0; c < nc; ++c) {
+    for (int c = first->pair.ok ? -1 : 0; c < nc; ++c) {
       std::unique_ptr<PlanEntry> pe;
-      CL_TRY(build_entry(cand[c], &pe));
+      if (c <= 0 && first) pe = std::move(first);
+      else CL_TRY(build_entry(cand[c], false, &pe));
       const int xm = pe->P.xmode;
       auto iteration = [&]() -> Status {
         CL_TRY(z_pass(*this, *pe, ModOTF{S, 1.f}, S, S));
@@ -881,6 +906,7 @@ Status Context::tune(const Dims& wd, std::unique_ptr<PlanEntry>* out) {
   if (e1) cudaEventDestroy(e1);
   if (!st.ok()) {
     if (best) free_entry(*best);
+    if (first) free_entry(*first);
     return st;
   }
   *out = std::move(best);
@@ -903,6 +929,17 @@ Status run_convolve(Context& ctx, const float* img, Dims id, const float* ker,
   return Status::Ok();
 }
 
+// The conjugated OTF (ws.HG) from ws.H.
+static Status conj_otf(Context& ctx, const PlanEntry& pe, Workspace& ws) {
+  if (!ws.HG) CL_CHECK(dev_alloc((void**)&ws.HG, sizeof(float2) * (size_t)ws.spec_cap));
+  const long long n = pe.pair.ok ? pe.pair.spec_elems : pe.P.spec_elems;
+  count_small();
+  CLARITY_LAUNCH(k_conj_spectrum, kReduceBlocks, 256, 0, ctx.exec_stream())(ws.H, ws.HG, n,
+                                                                            pe.pair.ok);
+  CL_CHECK(cudaGetLastError());
+  return Status::Ok();
+}
+
 // Circular correlation: Clarity_Convolve's passes with the conjugated OTF
 // applied in the z pass.
 Status run_correlate(Context& ctx, const float* img, Dims id, const float* ker, Dims kd,
@@ -913,11 +950,7 @@ Status run_correlate(Context& ctx, const float* img, Dims id, const float* ker, 
   CL_TRY(setup(ctx, id, kd, &pe, &ws, &wd));
   const VolPlan& P = pe->P;
   CL_TRY(make_otf(ctx, *pe, ker, kd, wd, ws->H, nullptr));
-  if (!ws->HG) CL_CHECK(dev_alloc((void**)&ws->HG, sizeof(float2) * (size_t)ws->spec_cap));
-  count_small();
-  CLARITY_LAUNCH(k_conj_spectrum, kReduceBlocks, 256, 0, ctx.exec_stream())(ws->H, ws->HG,
-                                                                            P.spec_elems);
-  CL_CHECK(cudaGetLastError());
+  CL_TRY(conj_otf(ctx, *pe, *ws));
   ProImage pro{image_src(img, id), P.xmode};
   CL_TRY(xy_forward(ctx, *pe, pro, ws->S));
   CL_TRY(z_pass(ctx, *pe, otf_between(ws->HG, inv_volume(wd), id.z, id.z), ws->S, ws->S));
@@ -1095,16 +1128,6 @@ static Status rl_core(Context& ctx, const PlanEntry& pe, Workspace& ws,
     CLARITY_LAUNCH(k_finish_sum_np, 1, 256, 0, st)(ws.partial, ws.iscal + 1, idiv + iters);
     CL_CHECK(cudaGetLastError());
   }
-  return Status::Ok();
-}
-
-// The conjugated OTF (ws.HG) from ws.H, for the correlation opt-ins.
-static Status conj_otf(Context& ctx, const PlanEntry& pe, Workspace& ws) {
-  if (!ws.HG) CL_CHECK(dev_alloc((void**)&ws.HG, sizeof(float2) * (size_t)ws.spec_cap));
-  count_small();
-  CLARITY_LAUNCH(k_conj_spectrum, kReduceBlocks, 256, 0, ctx.exec_stream())(ws.H, ws.HG,
-                                                                            pe.P.spec_elems);
-  CL_CHECK(cudaGetLastError());
   return Status::Ok();
 }
 
@@ -1403,7 +1426,7 @@ Status run_rl_batch(Context& ctx, int n, const float* const* imgs, const Dims* i
       for (int i = 0; i < n; ++i) {
         StreamScope scope(ctx, bs[i % ns]);
         if (persistent)
-          CL_TRY(rl_prologue(ctx, *pes[i], *wss[i], imgs[i], ids[i], kers[i], kds[i], wds[i]));
+          CL_TRY(rl_prologue(ctx, pes[i]->classic(), *wss[i], imgs[i], ids[i], kers[i], kds[i], wds[i]));
         else
           CL_TRY(rl_solve(ctx, *pes[i], *wss[i], imgs[i], ids[i], kers[i], kds[i], wds[i],
                           outs[i], iters));
@@ -1678,11 +1701,8 @@ Status run_idiv_cg(Context& ctx, const float* img, Dims id, const float* ker, Di
     CL_TRY(ensure(&ws->partial, &pc, 2 * (long long)kReduceBlocks));
     ws->partial_cap = (int)pc;
   }
-  if (!ws->HG) CL_CHECK(dev_alloc((void**)&ws->HG, sizeof(float2) * (size_t)ws->spec_cap));
   CL_TRY(make_otf(ctx, *pe, ker, kd, wd, ws->H, nullptr));
-  count_small();
-  CLARITY_LAUNCH(k_conj_spectrum, kReduceBlocks, 256, 0, st)(ws->H, ws->HG, pe->P.spec_elems);
-  CL_CHECK(cudaGetLastError());
+  CL_TRY(conj_otf(ctx, *pe, *ws));
   const ImageSrc g = image_src(img, id);
   const WorkVol wv{wd.x, wd.y, wd.z};
   float* a = ws->accel[0];

@@ -39,7 +39,24 @@ struct PlanEntry {
   float2* tw = nullptr;  // twiddle tables (FP64-generated, rounded)
   int* xrev = nullptr;   // natural x frequency -> smem slot after x passes
   int* err = nullptr;    // the context's error word (device alias; not owned)
+  // The column-pair passes (pair.ok): they serve every pass of the box, with a
+  // spectrum layout of their own.
+  PairPlan pair = {};
+  float2* pair_tw = nullptr;
+  int* pair_slots = nullptr;
+  // The same box on the passes of P (the persistent batched launch, whose
+  // tiles run those bodies).
+  PlanEntry classic() const {
+    PlanEntry c = *this;
+    c.pair.ok = 0;
+    return c;
+  }
+  long long spec_elems() const {
+    return pair.spec_elems > P.spec_elems ? pair.spec_elems : P.spec_elems;
+  }
 };
+// Whether compile-time kernels exist for the plan's box (kern_static_z.cu).
+bool has_static_shape(const VolPlan& P);
 
 
 // Device allocation that honours the host-side fault injector.
@@ -128,7 +145,7 @@ class Context {
   size_t bq_cap_ = 0;
   cudaStream_t user_stream_ = nullptr;
   bool has_user_stream_ = false;
-  Status build_entry(const VolPlan& P, std::unique_ptr<PlanEntry>* out);
+  Status build_entry(const VolPlan& P, bool pair, std::unique_ptr<PlanEntry>* out);
   Status tune(const Dims& wd, std::unique_ptr<PlanEntry>* out);
   // keyed by the work box and whether the autotuner chose the plan
   std::map<std::tuple<int, int, int, int>, std::unique_ptr<PlanEntry>> plans_;

@@ -5,6 +5,11 @@
 #include "static_dispatch.cuh"
 
 namespace clarity {
+template <class... SHs>
+static bool any_shape(ShapeList<SHs...>, const VolPlan& P) {
+  return (st::matches<SHs>(P) || ...);
+}
+bool has_static_shape(const VolPlan& P) { return any_shape(StaticShapes{}, P); }
 template bool static_z<ModOTF>(const PlanEntry&, cudaStream_t, const ModOTF&, const float2*, float2*, cudaError_t*);
 template bool static_z<ModWiener>(const PlanEntry&, cudaStream_t, const ModWiener&, const float2*, float2*, cudaError_t*);
 template bool static_z<ModForward>(const PlanEntry&, cudaStream_t, const ModForward&, const float2*, float2*, cudaError_t*);

@@ -20,6 +20,14 @@ bool static_xy_inv_fwd(const PlanEntry&, cudaStream_t, const F&, float2*, cudaEr
 template <class F>
 bool static_xy_inverse(const PlanEntry&, cudaStream_t, const F&, const float2*, cudaError_t*);
 
+// Column-pair launches (pair_dispatch.cuh, instantiated in kern_pair_*.cu).
+template <class F>
+bool pair_xy_forward(const PlanEntry&, cudaStream_t, const F&, float2*, cudaError_t*);
+template <class F, bool FUSE>
+bool pair_xy_inverse(const PlanEntry&, cudaStream_t, const F&, float2*, cudaError_t*);
+template <class F>
+bool pair_z(const PlanEntry&, cudaStream_t, const F&, const float2*, float2*, cudaError_t*);
+
 #ifndef CL_CHECK
 #define CL_CHECK(call)                                         \
   do {                                                         \
@@ -47,7 +55,8 @@ Status xy_forward(Context& ctx, const PlanEntry& pe, const Pro& pro,
                          float2* S) {
   const VolPlan& P = pe.P;
   cudaError_t se = cudaSuccess;
-  if (static_xy_forward(pe, ctx.exec_stream(), pro, S, &se))
+  if (pair_xy_forward(pe, ctx.exec_stream(), pro, S, &se) ||
+      static_xy_forward(pe, ctx.exec_stream(), pro, S, &se))
     return status_from_cuda(se, "xy forward");
   auto k = k_xy_forward<Pro>;
   CL_CHECK(prep_kernel(k, P.xy_smem));
@@ -64,7 +73,8 @@ Status xy_inverse(Context& ctx, const PlanEntry& pe, const Epi& epi,
                          const float2* S) {
   const VolPlan& P = pe.P;
   cudaError_t se = cudaSuccess;
-  if (static_xy_inverse(pe, ctx.exec_stream(), epi, S, &se))
+  if (pair_xy_inverse<Epi, false>(pe, ctx.exec_stream(), epi, const_cast<float2*>(S), &se) ||
+      static_xy_inverse(pe, ctx.exec_stream(), epi, S, &se))
     return status_from_cuda(se, "xy inverse");
   auto k = k_xy_inverse<Epi>;
   CL_CHECK(prep_kernel(k, P.xy_smem));
@@ -81,7 +91,8 @@ Status xy_inv_fwd(Context& ctx, const PlanEntry& pe, const Mid& mid,
                          float2* S) {
   const VolPlan& P = pe.P;
   cudaError_t se = cudaSuccess;
-  if (static_xy_inv_fwd(pe, ctx.exec_stream(), mid, S, &se))
+  if (pair_xy_inverse<Mid, true>(pe, ctx.exec_stream(), mid, S, &se) ||
+      static_xy_inv_fwd(pe, ctx.exec_stream(), mid, S, &se))
     return status_from_cuda(se, "xy inverse+forward");
   auto k = k_xy_inv_fwd<Mid>;
   CL_CHECK(prep_kernel(k, P.xy_smem));
@@ -98,7 +109,8 @@ Status z_pass(Context& ctx, const PlanEntry& pe, const Mod& mod,
                      const float2* Sin, float2* Sout) {
   const VolPlan& P = pe.P;
   cudaError_t se = cudaSuccess;
-  if (static_z(pe, ctx.exec_stream(), mod, Sin, Sout, &se))
+  if (pair_z(pe, ctx.exec_stream(), mod, Sin, Sout, &se) ||
+      static_z(pe, ctx.exec_stream(), mod, Sin, Sout, &se))
     return status_from_cuda(se, "z pass");
   auto k = k_z<Mod>;
   CL_CHECK(prep_kernel(k, P.z_smem));

@@ -11,10 +11,17 @@
 //   the forward transform when the epilogue is fused into k_xy_inv_fwd.
 // Spectral operations (Z pass): apply(idx, v) with idx the element's offset
 //   in the S layout (the OTF shares that layout).
+// The column-pair passes (passes_pair.cuh) work on real rows instead: row(y, z)
+// describes one (a default Row is a dead one, zero or unwanted), a prologue's
+// Row::load(x) is its value at x, an epilogue's pre(row, x) loads what it needs
+// there (ahead of the result) and put(row, x, v, pre) takes the result and
+// returns what the forward transform sees; a spectral operation's pair(h, v)
+// takes two columns at once.
 #pragma once
 #include "launch_macro.cuh"
 
 #include "dft_codelets.cuh"
+#include "dft_pair.cuh"
 #include "plan.hpp"
 #include "tma.cuh"
 
@@ -34,6 +41,15 @@ struct RowRef {
 // below 1e-5).
 __device__ __forceinline__ float rl_ratio(float g, float b) {
   return (fabsf(b) <= 1e-5f) ? 0.f : g / b;
+}
+
+// The ratio inside the image, 0 outside it (where g is zero).  A zero dividend
+// would send the whole warp through the division's out-of-line path -- half
+// the elements of a row whose image ends at its middle -- so dead elements
+// divide 1 by 1.
+__device__ __forceinline__ float live_ratio(bool live, float g, float b) {
+  const float q = rl_ratio(live ? g : 1.f, live ? b : 1.f);
+  return live ? q : 0.f;
 }
 
 // Real volume on the padded work box, x fastest.  The planner rejects boxes
@@ -81,6 +97,19 @@ struct PaddedSrc {
   }
 };
 
+// A real row read by a prologue: n floats at p seen from x = -off on an axis
+// of length `wrap` (the pad/shift map), zero elsewhere, times s.
+struct SrcRow {
+  const float* CLARITY_RESTRICT p = nullptr;
+  int n = 0, off = 0, wrap = 1 << 30;
+  float s = 1.f;
+  __device__ __forceinline__ float load(int x) const {
+    int i = x + off;
+    if (i >= wrap) i -= wrap;
+    return i < n ? s * ld_l2(p + i) : 0.f;
+  }
+};
+
 // ---------------------------------------------------------------- prologues
 // Plain work-box volume, optionally multiplied by a device-resident scale
 // (the deferred RL flux rescale).
@@ -97,6 +126,10 @@ struct ProWork {
     }
     const float a = CLARITY_LDG(&v[w.idx(m, y, z)]);
     return make_float2(scale ? s * a : a, 0.f);
+  }
+  using Row = SrcRow;
+  __device__ __forceinline__ Row row(int y, int z) const {
+    return Row{v + w.idx(0, y, z), w.nx, 0, 1 << 30, scale ? ld_l2(scale) : 1.f};
   }
   int live_planes(int nz) const { return nz; }
   __device__ __forceinline__ int plane(int p) const { return p; }
@@ -141,6 +174,23 @@ struct ProAccel {
     }
     return make_float2(one(a, m, y, z), 0.f);
   }
+  struct Row {
+    const float *CLARITY_RESTRICT x = nullptr, *CLARITY_RESTRICT xp = nullptr;
+    float* CLARITY_RESTRICT y = nullptr;
+    int n = 0;
+    float a = 0.f;
+    __device__ __forceinline__ float load(int i) const {
+      if (i >= n) return 0.f;
+      const float r = extrap(a, ld_l2(x + i), ld_l2(xp + i));
+      y[i] = r;
+      return r;
+    }
+  };
+  __device__ __forceinline__ Row row(int yy, int z) const {
+    if (yy >= Y || z >= Z) return Row{};
+    const unsigned o = ((unsigned)z * Y + yy) * X;
+    return Row{x + o, xp + o, yout + o, X, ld_l2(alpha)};
+  }
   int live_planes(int nz) const { return Z < nz ? Z : nz; }
   __device__ __forceinline__ int plane(int p) const { return p; }
   static constexpr bool has_zero_rows = true;
@@ -168,6 +218,13 @@ struct ProPadded {
   }
   // With the shift by -Z/2 the source's planes wrap around plane 0: its upper
   // Z - Z/2 planes land on planes 0.., the others on the last Z/2.
+  using Row = SrcRow;
+  __device__ __forceinline__ Row row(int y, int z) const {
+    const int k = PaddedSrc::wrap(z, p.sz, p.nz), j = PaddedSrc::wrap(y, p.sy, p.ny);
+    if (j >= p.Y || k >= p.Z) return Row{};
+    return Row{p.src + ((long long)k * p.Y + j) * p.X, p.X, -p.sx, p.nx,
+               scale ? ld_l2(scale) : 1.f};
+  }
   int live_planes(int) const { return p.Z; }
   __device__ __forceinline__ int plane(int q) const {
     return q < p.Z + p.sz ? q : q + (p.nz - p.Z);
@@ -190,6 +247,12 @@ struct ProImage {
       v = make_float2(s * v.x, s * v.y);
     }
     return v;
+  }
+  using Row = SrcRow;
+  __device__ __forceinline__ Row row(int y, int z) const {
+    if (y >= p.Y || z >= p.Z) return Row{};
+    return Row{p.src + ((unsigned)z * p.Y + y) * p.X, p.X, 0, 1 << 30,
+               scale ? ld_l2(scale) : 1.f};
   }
   int live_planes(int nz) const { return p.Z < nz ? p.Z : nz; }
   __device__ __forceinline__ int plane(int q) const { return q; }
@@ -253,6 +316,17 @@ struct EpiWork {
       out[w.idx(m, y, z)] = c.x;
     return c;
   }
+  struct Row {
+    float* o = nullptr;
+  };
+  __device__ __forceinline__ Row row(int y, int z) const { return Row{out + w.idx(0, y, z)}; }
+  struct Pre {};
+  __device__ __forceinline__ Pre pre(const Row&, int) const { return Pre{}; }
+  __device__ __forceinline__ float put(const Row& r, int x, float v, Pre) {
+    if (!r.o) return 0.f;
+    r.o[x] = v;
+    return v;
+  }
     // padding rows / z planes where the result is known to be zero
   __device__ __forceinline__ bool zero_row(int, int) const { return false; }
   __device__ __forceinline__ bool zero_plane(int) const { return false; }
@@ -284,6 +358,20 @@ struct EpiClip {
       put(m, y, z, c.x);
     }
     return c;
+  }
+  struct Row {
+    float* o = nullptr;
+    float s = 1.f;
+  };
+  __device__ __forceinline__ Row row(int y, int z) const {
+    if (y >= Y || z >= Z) return Row{};
+    return Row{out + ((long long)z * Y + y) * X, scale ? ld_l2(scale) : 1.f};
+  }
+  struct Pre {};
+  __device__ __forceinline__ Pre pre(const Row&, int) const { return Pre{}; }
+  __device__ __forceinline__ float put(const Row& r, int x, float v, Pre) {
+    if (r.o && x < X) r.o[x] = r.s * v;
+    return v;
   }
   // rows and planes outside the image are not asked for: not transformed
   __device__ __forceinline__ bool zero_row(int y, int z) const { return y >= Y || z >= Z; }
@@ -333,6 +421,25 @@ struct EpiRLProduct {
       return make_float2(a, one(2 * m + 1, y, z, c.y));
     }
     return make_float2(one(m, y, z, c.x), 0.f);
+  }
+  struct Row {
+    unsigned o = 0;  // offset of the row in cur and unew
+    int n = 0;       // its live extent
+    float s = 1.f;
+  };
+  __device__ __forceinline__ Row row(int y, int z) const {
+    if (y >= Y || z >= Z) return Row{};
+    return Row{at(0, y, z), X, scale ? ld_l2(scale) : 1.f};
+  }
+  using Pre = float;
+  __device__ __forceinline__ Pre pre(const Row& r, int x) const {
+    return x < r.n ? ld_l2(cur + (r.o + x)) : 0.f;
+  }
+  __device__ __forceinline__ float put(const Row& r, int x, float c, Pre u) {
+    const float a = x < r.n ? (r.s * u) * c : 0.f;
+    if (x < r.n) unew[r.o + x] = a;
+    acc += (double)a;
+    return a;
   }
   __device__ __forceinline__ bool zero_row(int y, int z) const { return y >= Y || z >= Z; }
   __device__ __forceinline__ bool zero_plane(int z) const { return z >= Z; }
@@ -422,6 +529,22 @@ struct MidRLRatio {
                          rl_ratio(g.at(2 * m + 1, y, z), b.y));
     return make_float2(rl_ratio(g.at(m, y, z), b.x), 0.f);
   }
+  struct Row {
+    unsigned o = 0;  // offset of the row in the image
+    int n = 0;       // its live extent
+  };
+  __device__ __forceinline__ Row row(int y, int z) const {
+    if (y >= g.Y || z >= g.Z) return Row{};
+    return Row{((unsigned)z * g.Y + y) * g.X, g.X};
+  }
+  using Pre = float;
+  __device__ __forceinline__ Pre pre(const Row& r, int x) const {
+    return x < r.n ? ld_l2(g.src + (r.o + x)) : 0.f;
+  }
+  __device__ __forceinline__ float put(const Row& r, int x, float b, Pre a) {
+    if (idiv_partial && x < r.n) idiv_add(a, b);
+    return live_ratio(x < r.n, a, b);
+  }
     // g is zero outside the image, so the ratio is exactly zero there
   // (0/b, or the 1e-5 guard): rows with y >= Y and planes with z >= Z need no
   // transform at all
@@ -452,7 +575,7 @@ struct MidRLRatio {
       if (x < n) idiv_add(a0, b.x);
       if (x + 1 < n) idiv_add(a1, b.y);
     }
-    return make_float2(rl_ratio(a0, b.x), rl_ratio(a1, b.y));
+    return make_float2(live_ratio(x < n, a0, b.x), live_ratio(x + 1 < n, a1, b.y));
   }
   __device__ __forceinline__ void finish() {
     if (idiv_partial) {
@@ -504,6 +627,27 @@ struct EpiJVC {
     inext[w.idx(m, y, z)] = r;
     return make_float2(r, 0.f);
   }
+  struct Row {
+    const float *CLARITY_RESTRICT i = nullptr, *CLARITY_RESTRICT g = nullptr;
+    float* CLARITY_RESTRICT o = nullptr;
+  };
+  __device__ __forceinline__ Row row(int y, int z) const {
+    const unsigned k = w.idx(0, y, z);
+    const bool in = y < g.Y && z < g.Z;
+    return Row{cur ? cur + k : nullptr, in ? g.src + ((unsigned)z * g.Y + y) * g.X : nullptr,
+               inext + k};
+  }
+  using Pre = float2;  // image, estimate
+  __device__ __forceinline__ Pre pre(const Row& r, int x) const {
+    const float gv = r.g && x < g.X ? ld_l2(r.g + x) : 0.f;
+    return make_float2(gv, r.i ? ld_l2(r.i + x) : gv);
+  }
+  __device__ __forceinline__ float put(const Row& r, int x, float o, Pre p) {
+    if (!r.o) return 0.f;
+    const float v = upd(p.y, p.x, o);
+    r.o[x] = v;
+    return v;
+  }
     // padding rows / z planes where the result is known to be zero
   __device__ __forceinline__ bool zero_row(int, int) const { return false; }
   __device__ __forceinline__ bool zero_plane(int) const { return false; }
@@ -550,6 +694,11 @@ struct ModOTF {
     const float f = scale2 ? scale * *scale2 : scale;
     return make_float2(f * (v.x * h.x - v.y * h.y), f * (v.x * h.y + v.y * h.x));
   }
+  __device__ __forceinline__ c2 pair(float4 h, c2 v) const {
+    const float2 hr = make_float2(h.x, h.y), hi = make_float2(h.z, h.w), f = both(scale);
+    return c2{pmul(f, psub(pmul(v.re, hr), pmul(v.im, hi))),
+              pmul(f, pfma(v.im, hr, pmul(v.re, hi)))};
+  }
   // the same operation with the deferred factor read once (per thread)
   __device__ __forceinline__ ModOTF resolved() const {
     ModOTF r = *this;
@@ -578,11 +727,18 @@ struct ModWiener {
                         off + chunk <= total ? chunk : total - off);
   }
   __device__ __forceinline__ float2 apply(long long idx, float2 v) const {
-    const float2 h = CLARITY_LDG(&H[idx]);
+    return apply_h(CLARITY_LDG(&H[idx]), v);
+  }
+  __device__ __forceinline__ float2 apply_h(float2 h, float2 v) const {
     const float mag = h.x * h.x + h.y * h.y;
     const float f = 1.0f / (mag + eps);
     const float a = h.x * f, b = -h.y * f;
     return make_float2(scale * (a * v.x - b * v.y), scale * (a * v.y + b * v.x));
+  }
+  __device__ __forceinline__ c2 pair(float4 h, c2 v) const {
+    const float2 x = apply_h(make_float2(h.x, h.z), make_float2(v.re.x, v.im.x));
+    const float2 y = apply_h(make_float2(h.y, h.w), make_float2(v.re.y, v.im.y));
+    return c2{make_float2(x.x, y.x), make_float2(x.y, y.y)};
   }
   __device__ __forceinline__ ModWiener resolved() const { return *this; }
 };

@@ -75,6 +75,50 @@ struct VolPlan {
 #define CLARITY_HD
 #endif
 
+// Division of 0 <= n < 2^20 by a fixed 1 <= d < 2^11 as a multiply-high:
+// m = ceil(2^32 / d) is off by less than d, so n m / 2^32 is off by less than
+// n d / 2^32 < 1/d and its floor is exact.
+struct FDiv {
+  unsigned m, one;  // one: all bits set for d = 1, whose m would be 2^32
+};
+CLARITY_HD inline FDiv fdiv_by(int d) {
+  if (d <= 1) return FDiv{0u, ~0u};
+  return FDiv{0xFFFFFFFFu / (unsigned)d + 1u, 0u};
+}
+
+// Plan of the column-pair passes (passes_pair.cuh) for one work box.  The x
+// transforms run on pairs of real rows held as one complex row of full length
+// nx (no r2c split; odd nx costs what even nx does), two pairs per register
+// pass: a row quad.  The spectrum is stored as pairs of columns,
+//   S[k1][kg][z][y0] = float4 (re of kx = 2kg, re of 2kg+1, im, im),
+//   k1 < Ay, kg < KG = ceil((nx/2 + 1) / 2), y = y0 + By*j, y0 < By.
+struct PairAxis {
+  int n, npass;
+  int radix[kMaxPasses], len[kMaxPasses], span[kMaxPasses];
+  int plen[kMaxPasses], pspan[kMaxPasses];  // len and span in padded slots
+  int pad;     // one empty slot after every `pad` elements (0: none)
+  FDiv dspan[kMaxPasses], dper[kMaxPasses];  // by span and by n / radix
+  FDiv dpad;
+  int tw_off;  // the w_n^t table in the pair twiddle buffer
+};
+struct PairPlan {
+  int ok;
+  int nx, ny, nz;
+  int XS, KG;       // columns kx < XS, pairs of them
+  int Ay, By;       // ny = Ay * By
+  int TG;           // y0 lines per XY tile
+  int NQ;           // row quads per line, ceil(Ay / 4)
+  int rowlen;       // slots (float4) per row quad in shared memory
+  int BS;           // slots per z row in the z tile
+  PairAxis ax, ayB, az;
+  FDiv dBy, dTG;
+  int tw_ny_off;    // w_ny^t, t < ny
+  int twiddle_count;
+  int big_xy, big_z;  // a radix above 16: the kernels with more registers a thread
+  int xy_threads, z_threads, xy_smem, z_smem, z_blocks;
+  long long spec_elems;  // complex elements of S
+};
+
 // Twiddle table w_n^t = exp(-2 pi i t / n), t < count, at float2 offset off.
 struct TwTable {
   int off, n, count;
@@ -113,6 +157,14 @@ bool make_plan(int nx, int ny, int nz, VolPlan* out, std::string* why);
 // Up to max_out (<= 8) tilings of the box, best model score first (the first
 // is make_plan's); the autotuner times them.  Returns how many.
 int make_plan_candidates(int nx, int ny, int nz, VolPlan* out, int max_out, std::string* why);
+
+// Plans the column-pair passes; false for boxes they do not serve (a z tile
+// beyond shared memory, rows beyond kPairMaxNx, unsupported factors).
+constexpr int kPairMaxNx = 1280;
+bool make_pair_plan(int nx, int ny, int nz, PairPlan* out);
+// Tables of a pair plan: the padded shared-memory slot of every natural x
+// frequency, and the twiddle tables (x, y0, z, y split).
+void pair_tables(const PairPlan& P, std::vector<int>* slots, std::vector<TwTable>* tabs);
 
 // Kernel families of the launch accounting and timing probes.
 enum KernelKind { KK_XY_FORWARD = 0, KK_Z = 1, KK_XY_INV_FWD = 2, KK_XY_INVERSE = 3,

@@ -199,4 +199,200 @@ void plan_tables(const VolPlan& P, std::vector<int>* xrev, std::vector<TwTable>*
   tabs->assign(t, t + kPlanTwTables);
 }
 
+// ------------------------------------------------------- column-pair passes
+// Radix sequence of n with the fewest passes (then the smallest largest
+// radix), non-increasing, from the radices up to 16 and, where n has those
+// factors, 17 and 19.
+static void search_pair(int n, int depth, int* cur, int* best, int* best_len, int* best_max) {
+  if (n == 1) {
+    const int mx = depth ? cur[0] : 0;
+    if (depth < *best_len || (depth == *best_len && mx < *best_max)) {
+      *best_len = depth;
+      *best_max = mx;
+      for (int i = 0; i < depth; ++i) best[i] = cur[i];
+    }
+    return;
+  }
+  if (depth >= kMaxPasses || depth + 1 > *best_len) return;
+  for (int r = 19; r >= 2; --r) {
+    if (r == 18 || n % r) continue;
+    if (depth > 0 && r > cur[depth - 1]) continue;
+    cur[depth] = r;
+    search_pair(n / r, depth + 1, cur, best, best_len, best_max);
+  }
+}
+
+static bool pair_axis(int n, bool padded, PairAxis* A) {
+  std::memset(A, 0, sizeof(*A));
+  A->n = n;
+  if (n == 1) return true;
+  int cur[kMaxPasses], best[kMaxPasses];
+  int best_len = kMaxPasses + 1, best_max = INT_MAX;
+  search_pair(n, 0, cur, best, &best_len, &best_max);
+  if (best_len > kMaxPasses) return false;
+  A->npass = best_len;
+  const int rl = best[best_len - 1];
+  // the last pass's consecutive threads are rl slots apart: an even rl gets
+  // one empty slot per rl elements, so the stride is odd (no bank conflicts)
+  A->pad = padded && best_len > 1 && rl % 2 == 0 ? rl : 0;
+  int len = n;
+  for (int s = 0; s < best_len; ++s) {
+    A->radix[s] = best[s];
+    A->len[s] = len;
+    A->span[s] = len / best[s];
+    A->plen[s] = len + (A->pad ? len / A->pad : 0);
+    A->pspan[s] = A->span[s] + (A->pad ? A->span[s] / A->pad : 0);
+    A->dspan[s] = fdiv_by(A->span[s]);
+    A->dper[s] = fdiv_by(n / best[s]);
+    len /= best[s];
+  }
+  A->dpad = fdiv_by(A->pad);
+  return true;
+}
+
+static bool pair_big(const PairAxis& A) {
+  for (int s = 0; s < A.npass; ++s)
+    if (A.radix[s] > 16) return true;
+  return false;
+}
+
+// Rough cycles of a pass kernel on the chip's 148 SMs: `n` sweeps of items[s]
+// work items of radix r[s] by blocks of `threads`, as many blocks per SM as
+// shared memory and registers allow.  A round of a sweep costs its latency
+// (lat[s] and about 140 cycles per radix point: some 25 instructions at a
+// warp's 6 cycles each) or the issue slots of all resident warps, whichever is
+// more; both constants from the passes' profiles at the 320x320x96 box.
+static double pair_cost(const int* items, const int* r, const int* lat, int n, int threads,
+                        int smem, long long blocks, bool big) {
+  const int by_regs = (big ? 256 : 512) / threads, by_smem = kSmemPerSM / (smem + 1024);
+  int bps = std::min(by_regs, by_smem);
+  if (bps < 1) return 1e30;
+  const long long per_sm = (blocks + 147) / 148;
+  const long long waves = (per_sm + bps - 1) / bps;
+  bps = (int)((per_sm + waves - 1) / waves);
+  double t = 1500;
+  for (int s = 0; s < n; ++s) {
+    const int rounds = (items[s] + threads - 1) / threads;
+    t += rounds * std::max(lat[s] + 140.0 * r[s], bps * (threads / 32) * 10.0 * r[s]);
+  }
+  return t * (double)waves;
+}
+
+static int pair_threads(const int* items, const int* r, const int* lat, int n, int smem,
+                        long long blocks, bool big, double* cost) {
+  int best = 0;
+  *cost = 1e30;
+  for (int t = 32; t <= (big ? 128 : 256); t += 32) {
+    const double c = pair_cost(items, r, lat, n, t, smem, blocks, big);
+    if (c < *cost) {
+      *cost = c;
+      best = t;
+    }
+  }
+  return best;
+}
+
+bool make_pair_plan(int nx, int ny, int nz, PairPlan* out) {
+  PairPlan P;
+  std::memset(&P, 0, sizeof(P));
+  P.nx = nx;
+  P.ny = ny;
+  P.nz = nz;
+  P.XS = nx / 2 + 1;
+  P.KG = (P.XS + 1) / 2;
+  out->ok = 0;
+  if (nx < 2 || nz < 2 || nx > kPairMaxNx || (long long)nx * ny * nz >= (1ll << 31)) return false;
+  if (!pair_axis(nx, true, &P.ax) || !pair_axis(nz, false, &P.az)) return false;
+  P.rowlen = nx + (P.ax.pad ? nx / P.ax.pad : 0);
+  double best = 1e30;
+  for (int ay = 1; ay <= 19; ++ay) {
+    if (ny % ay || ay == 18) continue;
+    PairPlan c = P;
+    c.Ay = ay;
+    c.By = ny / ay;
+    if (!pair_axis(c.By, false, &c.ayB)) continue;
+    c.NQ = (ay + 3) / 4;
+    c.BS = c.By | 1;
+    c.spec_elems = 2ll * ay * c.KG * nz * c.By;
+    if (c.spec_elems >= (1ll << 31)) continue;
+    c.dBy = fdiv_by(c.By);
+    const long long zsm = ((long long)nz * c.BS + nz + c.By) * 16;
+    if (zsm > kSmemMax) continue;
+    c.z_smem = (int)zsm;
+    c.z_blocks = ay * c.KG;
+    c.big_z = pair_big(c.az) || pair_big(c.ayB);
+    c.big_xy = ay > 16 || pair_big(c.ax);
+    // a sweep's latency: shared memory only, or through L2 or HBM
+    constexpr int kSm = 500, kFar = 2000;
+    int items[4 * kMaxPasses], r[4 * kMaxPasses], lat[4 * kMaxPasses], n = 0;
+    for (int s = 0; s < c.ayB.npass; ++s)
+      for (int d = 0; d < 2; ++d, ++n) {
+        lat[n] = kSm;
+        r[n] = c.ayB.radix[s];
+        items[n] = nz * (c.By / r[n]);
+      }
+    for (int s = 0; s < c.az.npass; ++s)
+      for (int d = 0; d < 2; ++d, ++n) {
+        lat[n] = s == c.az.npass - 1 && d == 0 ? kFar : kSm;
+        r[n] = c.az.radix[s];
+        items[n] = c.By * (nz / r[n]);
+      }
+    double zc, xc;
+    c.z_threads = pair_threads(items, r, lat, n, c.z_smem, c.z_blocks, c.big_z, &zc);
+    if (!c.z_threads) continue;
+    for (int tg : {1, 2, 3, 4, 8}) {
+      if (c.By % tg) continue;
+      const long long xsm = ((long long)tg * c.NQ * c.rowlen + tg * ay) * 16 + nx * 8;
+      if (xsm > kSmemMax) continue;
+      c.TG = tg;
+      c.dTG = fdiv_by(tg);
+      c.xy_smem = (int)xsm;
+      n = 0;
+      for (int d = 0; d < 2; ++d, ++n) {
+        r[n] = ay + (tg == 1 ? 6 : 2);  // the column step, its global accesses wider for tg > 1
+        lat[n] = d == 0 ? kFar : kSm;
+        items[n] = tg * c.KG;
+      }
+      for (int s = 0; s < c.ax.npass; ++s)
+        for (int d = 0; d < (s == 0 ? 1 : 2); ++d, ++n) {
+          lat[n] = s == 0 ? kFar : kSm;
+          r[n] = s == 0 ? 2 * c.ax.radix[s] : c.ax.radix[s];  // the first and last pass in one
+          items[n] = tg * c.NQ * (nx / c.ax.radix[s]);
+        }
+      c.xy_threads = pair_threads(items, r, lat, n, c.xy_smem, (long long)nz * (c.By / tg), c.big_xy, &xc);
+      if (!c.xy_threads) continue;
+      // one line's columns are half sectors of the spectrum: 8% in the XY passes
+      // at the 320x320x96 box
+      if (tg == 1) xc *= 1.08;
+      if (zc + xc < best) {
+        best = zc + xc;
+        *out = c;
+        out->ok = 1;
+      }
+    }
+  }
+  if (!out->ok) return false;
+  int off = 0;
+  out->ax.tw_off = off; off += nx;
+  out->ayB.tw_off = off; off += out->By;
+  out->az.tw_off = off; off += nz;
+  out->tw_ny_off = off; off += ny;
+  out->twiddle_count = off;
+  return true;
+}
+
+void pair_tables(const PairPlan& P, std::vector<int>* slots, std::vector<TwTable>* tabs) {
+  slots->assign(P.nx, 0);
+  for (int k = 0; k < P.nx; ++k) {
+    int rem = k, e = 0;
+    for (int s = 0; s < P.ax.npass; ++s) {
+      e += (rem % P.ax.radix[s]) * P.ax.span[s];
+      rem /= P.ax.radix[s];
+    }
+    (*slots)[k] = e + (P.ax.pad ? e / P.ax.pad : 0);
+  }
+  *tabs = {TwTable{P.ax.tw_off, P.nx, P.nx}, TwTable{P.ayB.tw_off, P.By, P.By},
+           TwTable{P.az.tw_off, P.nz, P.nz}, TwTable{P.tw_ny_off, P.ny, P.ny}};
+}
+
 }  // namespace clarity

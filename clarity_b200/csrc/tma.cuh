@@ -178,6 +178,29 @@ inline int atomicExch(int* p, int v) {
 }
 #endif
 
+// Loads through L2 that stay behind CLARITY_PDL_WAIT (both are volatile): for
+// data the previous kernels on the stream may have written.
+__device__ __forceinline__ float ld_l2(const float* p) {
+#ifndef CLARITY_HOST_EMULATION
+  float v;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+#else
+  return *p;
+#endif
+}
+__device__ __forceinline__ float4 ld_l2(const float4* p) {
+#ifndef CLARITY_HOST_EMULATION
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p));
+  return v;
+#else
+  return *p;
+#endif
+}
+
 // L2 prefetch of the 16-byte-aligned part of [begin, begin+bytes): never
 // touches memory outside the range.
 __device__ __forceinline__ void prefetch_l2_range(const void* begin, size_t bytes) {

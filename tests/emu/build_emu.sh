@@ -17,3 +17,5 @@ for f in "$ROOT"/clarity_b200/csrc/*.cu "$ROOT"/clarity_b200/csrc/*.cpp \
 done
 for p in $pids; do wait $p; done
 $CXX -fsanitize=address "$OUT"/*.o -o "$OUT/emu_main"
+# the objects are hundreds of MB and always rebuilt
+rm -f "$OUT"/*.o

@@ -265,3 +265,40 @@ def test_emulated_single_pass_filters_with_uneven_split(emu, tmp_path, ishape, k
     assert rel_l2(run_emu(emu, tmp_path, "convolve_noalloc", img, psf, 0), want) <= 1e-6
     assert rel_l2(run_emu(emu, tmp_path, "wiener", img, psf, 1e-2),
                   oracle_lib.wiener(img, psf, 1e-2)) <= 2e-6
+
+
+@pytest.mark.parametrize("ishape,kshape", [
+    ((1, 1, 1), (1, 1, 1)),        # work 2x2x2: one radix-2 pass per axis
+    ((9, 20, 19), (5, 18, 15)),    # 34x38x14: radices 17, 19 and 14
+    ((3, 5, 31), (2, 2, 14)),      # 45x7x5: odd x as 15*3, Ay 7 with a dead row in its last quad
+    ((4, 10, 40), (6, 29, 47)),    # 87 has a factor 29: refused in x
+    ((4, 13, 60), (6, 26, 51)),    # 111 = 3*37: refused in x
+    ((5, 50, 27), (7, 70, 37)),    # 64x120x12: most rows and quads of a line dead
+    ((11, 26, 30), (2, 7, 25)),    # 55x33x13: prime radices 11 and 13, odd everywhere
+    ((1, 3, 640), (1, 1, 656)),    # 1296x4x2: rows too long for the column-pair passes
+])
+def test_emulated_column_pair_passes_match_the_general_path(emu, tmp_path, oracle_lib, ishape,
+                                                            kshape):
+    # boxes without compile-time kernels run the column-pair passes; with
+    # CLARITY_STATIC=0 every box runs the runtime-planned ones
+    r = syn.rng(11 + sum(ishape))
+    img = (r.random(ishape) * 100 + 1).astype(np.float32)
+    psf = syn.gaussian_psf(kshape, 1.5, 1.2).astype(np.float32)
+    if any((a + b) % p == 0 for a, b in zip(ishape, kshape) for p in (29, 37)):
+        with pytest.raises(AssertionError):  # no plan in either form
+            run_emu(emu, tmp_path, "convolve", img, psf, 0)
+        return
+    for op, prm, want, tol in (("convolve", 0, oracle_lib.convolve(img, psf), 1e-6),
+                               ("wiener", 1e-2, oracle_lib.wiener(img, psf, 1e-2), 2e-6),
+                               ("rl", 2, oracle_lib.rl(img, psf, 2), 2e-6),
+                               ("jvc", 2, oracle_lib.jvc(img, psf, 2), 2e-6),
+                               ("accel", 3, oracle_lib.rl_accel(img, psf, 3)[0], 2e-6),
+                               ("rlcorr", 2, oracle_lib.rl_correlate(img, psf, 2), 2e-6)):
+        got = run_emu(emu, tmp_path, op, img, psf, prm)
+        assert rel_l2(got, want) <= tol, op
+        os.environ["CLARITY_STATIC"] = "0"
+        try:
+            general = run_emu(emu, tmp_path, op, img, psf, prm)
+        finally:
+            del os.environ["CLARITY_STATIC"]
+        assert rel_l2(got, general) <= 2 * tol, op
