@@ -82,22 +82,70 @@ constexpr cs_pair root_cs(long k, long n) {
 }
 
 // ------------------------------------------------------------ complex ops
-// Complex add and subtract use sm_100's paired FP32 add (one FADD2 per complex
-// add instead of two FADDs; each lane rounds exactly as a scalar add), unless
-// CLARITY_NO_F32X2 is defined or the code is compiled for the host.
-#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000 && !defined(CLARITY_NO_F32X2)
-#define CLARITY_F32X2 1
+// Packed FP32 (sm_100's add/sub/mul/fma.f32x2): one instruction on both halves
+// of a float2, each rounded as the scalar instruction rounds it.  The
+// subtraction is an instruction of its own: written as an add of -b it costs
+// two more to negate b.
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+__device__ __forceinline__ unsigned long long f2_bits(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ float2 bits_f2(unsigned long long r) {
+  float2 a;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+  return a;
+}
+__device__ __forceinline__ float2 padd(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return bits_f2(r);
+}
+__device__ __forceinline__ float2 psub(float2 a, float2 b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return bits_f2(r);
+}
+__device__ __forceinline__ float2 pmul(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return bits_f2(r);
+}
+__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r)
+      : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
+  return bits_f2(r);
+}
+#else
+__device__ __forceinline__ float2 padd(float2 a, float2 b) {
+  return make_float2(a.x + b.x, a.y + b.y);
+}
+__device__ __forceinline__ float2 psub(float2 a, float2 b) {
+  return make_float2(a.x - b.x, a.y - b.y);
+}
+__device__ __forceinline__ float2 pmul(float2 a, float2 b) {
+  return make_float2(a.x * b.x, a.y * b.y);
+}
+__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) {
+  return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
+}
 #endif
+
+// Complex add and subtract as one packed instruction, unless CLARITY_NO_F32X2
+// is defined.
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) {
-#ifdef CLARITY_F32X2
-  return __fadd2_rn(a, b);
+#ifndef CLARITY_NO_F32X2
+  return padd(a, b);
 #else
   return make_float2(a.x + b.x, a.y + b.y);
 #endif
 }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) {
-#ifdef CLARITY_F32X2
-  return __fadd2_rn(a, make_float2(-b.x, -b.y));
+#ifndef CLARITY_NO_F32X2
+  return psub(a, b);
 #else
   return make_float2(a.x - b.x, a.y - b.y);
 #endif

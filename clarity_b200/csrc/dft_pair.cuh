@@ -18,53 +18,6 @@ struct c2 {
   float2 re, im;
 };
 
-#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
-__device__ __forceinline__ unsigned long long f2_bits(float2 a) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
-  return r;
-}
-__device__ __forceinline__ float2 bits_f2(unsigned long long r) {
-  float2 a;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
-  return a;
-}
-__device__ __forceinline__ float2 padd(float2 a, float2 b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
-  return bits_f2(r);
-}
-__device__ __forceinline__ float2 psub(float2 a, float2 b) {
-  unsigned long long r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
-  return bits_f2(r);
-}
-__device__ __forceinline__ float2 pmul(float2 a, float2 b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
-  return bits_f2(r);
-}
-__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(r)
-      : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
-  return bits_f2(r);
-}
-#else
-__device__ __forceinline__ float2 padd(float2 a, float2 b) {
-  return make_float2(a.x + b.x, a.y + b.y);
-}
-__device__ __forceinline__ float2 psub(float2 a, float2 b) {
-  return make_float2(a.x - b.x, a.y - b.y);
-}
-__device__ __forceinline__ float2 pmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x, a.y * b.y);
-}
-__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) {
-  return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
-}
-#endif
 __device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
 
 __device__ __forceinline__ c2 padd(c2 a, c2 b) { return c2{padd(a.re, b.re), padd(a.im, b.im)}; }

@@ -47,11 +47,9 @@ inline PdlLauncher<P...> pdl_launcher(void (*k)(P...), dim3 grid, dim3 block, si
   ::clarity::pdl_launcher((kernel), dim3(grid), dim3(block), (smem), (stream), (pdl))
 // First statement of a kernel launched by CLARITY_LAUNCH_PDL.
 #define CLARITY_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
-// Lets the next kernel's blocks be scheduled once every block of this one has
-// started (they wait in CLARITY_PDL_WAIT for its completion).  Only after this
-// kernel's own wait: the one before it has then completed, so nothing older
-// than one kernel runs beside the next.
-#define CLARITY_PDL_TRIGGER() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
+// (No kernel lets the next one start early with launch_dependents: waiting
+// blocks beside a small grid made RL on 64x64x32 slower, 31 -> 44 us an
+// iteration, and changed nothing at 256x256x64.)
 #define CLARITY_DYN_SMEM(T, name) extern __shared__ __align__(128) T name[]
 // Loop stride of a block-wide strided loop in kernels launched with a
 // compile-time block size.
@@ -65,7 +63,6 @@ inline PdlLauncher<P...> pdl_launcher(void (*k)(P...), dim3 grid, dim3 block, si
 #define CLARITY_LAUNCH_PDL(kernel, grid, block, smem, stream, pdl) \
   ::clarity_emu::launcher((grid), (smem))(kernel)
 #define CLARITY_PDL_WAIT() ((void)0)
-#define CLARITY_PDL_TRIGGER() ((void)0)
 #define CLARITY_DYN_SMEM(T, name) T* name = ::clarity_emu::dynamic_smem<T>()
 #define CLARITY_BLOCK_STRIDE(n) ((int)blockDim.x)
 #define CLARITY_ISSUE_LANES ((int)blockDim.x)

@@ -197,7 +197,6 @@ __global__ void __launch_bounds__(Cls<BIG>::MAXT, 2)
   for (int t = threadIdx.x; t < P.By; t += blockDim.x)
     twy[t] = twin(CLARITY_LDG(&tables[P.ayB.tw_off + t]));
   CLARITY_PDL_WAIT();  // the previous kernel's output is complete and visible
-  CLARITY_PDL_TRIGGER();
   // the OTF tile this block will multiply by, into L2
   if (threadIdx.x < 4) mod.prefetch_tile(gbase * 2u, P.nz * P.By * 2, threadIdx.x, 4);
   // plain 16-byte loads: a bulk copy per plane costs more issue slots than the
@@ -536,7 +535,6 @@ __global__ void __launch_bounds__(Cls<BIG>::MAXT, 2)
   const float4* twl = stage_tables(sm, P, y0base, tables);
   __syncthreads();
   CLARITY_PDL_WAIT();
-  CLARITY_PDL_TRIGGER();
   const XyCtx C = tile_of(sm, P, pro, pro.plane(pl), y0base, twl);
   with_radix<MAXR>(P.ax.radix[0], [&](auto r) { x_first<decltype(r)::value>(C, P, pro); });
   __syncthreads();
@@ -558,7 +556,6 @@ __global__ void __launch_bounds__(Cls<BIG>::MAXT, 2)
   const float4* twl = stage_tables(sm, P, y0base, tables);
   __syncthreads();
   CLARITY_PDL_WAIT();
-  CLARITY_PDL_TRIGGER();
   const XyCtx C = tile_of(sm, P, epi, z, y0base, twl);
   with_radix<MAXR>(P.Ay, [&](auto r) {
     cols_inverse<decltype(r)::value>(C, P, reinterpret_cast<const float4*>(S), twl, slots);

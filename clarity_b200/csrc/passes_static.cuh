@@ -64,10 +64,10 @@ struct Shape {
   static constexpr int TILE = NZ * BW;
   static constexpr int THREADS = T_;
   static constexpr int Z_THREADS = TZ_;
-  static_assert(T_ % 32 == 0 && T_ >= 256 && T_ <= 1024, "whole warps, 256..1024 threads");
+  static_assert(T_ % 32 == 0 && T_ >= 64 && T_ <= 1024, "whole warps, 64..1024 threads");
   // blocks per SM the register budget is sized for (__launch_bounds__)
-  static constexpr int XY_MINB = T_ == 256 ? CLARITY_XY_MINBLOCKS : 1;
-  static constexpr int Z_MINB = T_ == 256 ? 2 : 1;
+  static constexpr int XY_MINB = T_ <= 256 ? CLARITY_XY_MINBLOCKS : 1;
+  static constexpr int Z_MINB = T_ <= 256 ? 2 : 1;
   static constexpr int XY_SMEM = G * GSTRIDE * 8;
   static constexpr int Z_SMEM = TILE * 8;
   static constexpr int NGROUPS = BY / G;
@@ -796,48 +796,44 @@ template <class SH, class Mod>
 __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
     ks_z2(const Mod mod, const float2* __restrict__ Sin, float2* __restrict__ Sout,
           const Tables T) {
-  CLARITY_PDL_WAIT();  // the previous kernel's output is complete and visible
   CLARITY_DYN_SMEM(float2, sm);
   static_assert(SH::Y_PER_LINE, "y0 per-line Z kernel needs BY <= 32");
   constexpr int BY = SH::BY, W = SH::W, BW = SH::BW, NZ = SH::NZ, ZS = SH::ZS;
   // z rows of the tile are contiguous BW*8-byte runs in HBM and land at
-  // ZS*8-byte strides in shared memory: bulk copies when both are 16-byte
-  // multiples
+  // ZS*8-byte strides in shared memory: 16-byte asynchronous copies when both
+  // are 16-byte multiples
   constexpr bool BULK = (BW * 8) % 16 == 0 && (ZS * 8) % 16 == 0;
   using A = typename SH::Z;
   const unsigned gbase = blockIdx.x * (unsigned)SH::TILE;
   // planes zn <= z < zh are zero: the q-th live plane is q, or q + gap
   const int zn = mod.zn < NZ ? mod.zn : NZ;
   const int gap = (mod.zh < NZ ? mod.zh : NZ) - zn;
-  if (threadIdx.x < 16) mod.prefetch_tile(gbase, SH::TILE, threadIdx.x, 16);
-  // z twiddles in shared memory: a z-pass task's twiddle is the same for all
-  // lanes of a warp (a broadcast), where the table in global memory cost an
-  // L1 round trip per twiddle
+  // z twiddles in shared memory, before the previous kernel has finished: a
+  // z-pass task's twiddle is the same for all lanes of a warp (a broadcast),
+  // where the table in global memory cost an L1 round trip per twiddle
   float2* twz = sm + SH::Z2_TILE_BYTES / 8;
   for (int t = threadIdx.x; t < NZ; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) twz[t] = __ldg(&T.twz[t]);
-  __shared__ alignas(8) uint64_t bar;
+  CLARITY_PDL_WAIT();  // the previous kernel's output is complete and visible
   if constexpr (BULK) {
     static_assert((BW * 8) % 16 == 0 && (ZS * 8) % 16 == 0 && (SH::TILE * 8) % 16 == 0,
-                  "bulk copies need 16-byte sizes and offsets");
+                  "16-byte copies need 16-byte sizes and offsets");
     if (!smem_aligned16(sm)) {  // never expected: refuse rather than fault
       if (threadIdx.x == 0) raise_error(T.err, kErrMisaligned);
       return;
     }
-    if (threadIdx.x == 0) mbar_init(&bar, 1);
-    __syncthreads();
-    if ((int)threadIdx.x < CLARITY_ISSUE_LANES) {
-      if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, (uint32_t)((NZ - gap) * BW * 8));
-      __syncwarp();
-      for (int q = threadIdx.x; q < NZ - gap; q += CLARITY_ISSUE_LANES) {
-        const int z = q < zn ? q : q + gap;
-        bulk_load(sm + z * ZS, Sin + gbase + z * BW, BW * 8, &bar);
-      }
+    constexpr int CH = BW / 2;  // 16-byte chunks of a row
+#pragma unroll 4
+    for (int t = threadIdx.x; t < (NZ - gap) * CH; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
+      const int q = t / CH, c = 2 * (t - q * CH);
+      const int z = q < zn ? q : q + gap;
+      cp_async16(sm + z * ZS + c, Sin + gbase + z * BW + c);
     }
-    if (!mbar_wait(&bar, 0, T.err)) {
-      mbar_wait(&bar, 0, nullptr);  // give copies in flight a last chance
-      return;
-    }
+    if (threadIdx.x < 4) mod.prefetch_tile(gbase, SH::TILE, threadIdx.x, 4);
+    cp_async_wait_all();
+  } else {
+    if (threadIdx.x < 4) mod.prefetch_tile(gbase, SH::TILE, threadIdx.x, 4);
   }
+  __syncthreads();
   // y0 forward, one line (z, ki) per thread
 #pragma unroll 1
   for (int l = threadIdx.x; l < NZ * W; l += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
@@ -901,12 +897,13 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
       }
     }
     if constexpr (BULK) {
-      fence_smem_to_async();
       __syncthreads();
-      if ((int)threadIdx.x < CLARITY_ISSUE_LANES) {
-        for (int z = threadIdx.x; z < zo; z += CLARITY_ISSUE_LANES)
-          bulk_store(Sout + gbase + z * BW, sm + z * ZS, BW * 8);
-        bulk_store_commit_and_wait();
+      constexpr int CH = BW / 2;
+#pragma unroll 4
+      for (int t = threadIdx.x; t < zo * CH; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
+        const int z = t / CH, c = 2 * (t - z * CH);
+        *reinterpret_cast<float4*>(Sout + gbase + z * BW + c) =
+            *reinterpret_cast<const float4*>(sm + z * ZS + c);
       }
     }
   }

@@ -2,22 +2,21 @@
 // HBM traffic moved by the Tensor Memory Accelerator.
 //
 // One block owns the tile (z, y0base .. y0base+TG-1): all AY rows y = y0 +
-// BY*j of those TG y0 lines.  At block start one thread issues
-//   * one tiled tensor load of the tile's spectrum columns, the box
-//     S[k1 = 0..AY)[kg = 0..KG)[z][y0base .. +TG)[ki = 0..W) (33 KB for the
-//     512x512x128 box), and
-//   * one bulk copy per tile row of the real volume the epilogue reads (the
-//     RL estimate or the image),
-// both completing on mbarriers, so no thread waits on HBM inside the
-// transforms.  The column step then runs one length-AY DFT per thread out of
-// shared memory (every column a task of its own: the kx = 0 and kx = M columns
-// share one DFT as the real and imaginary parts of one complex column), the
-// x passes and the epilogue run as in passes_static.cuh, the epilogue's output
-// rows leave by bulk stores, and the forward column step writes the box back
-// into the same buffer for one tiled tensor store.
+// BY*j of those TG y0 lines.  At block start
+//   * one thread issues one tiled tensor load of the tile's spectrum columns,
+//     the box S[k1 = 0..AY)[kg = 0..KG)[z][y0base .. +TG)[ki = 0..W) (33 KB a
+//     line for the 512x512x128 box), completing on an mbarrier, and
+//   * all threads copy the rows of the real volume the epilogue reads (the RL
+//     estimate or the image) by 16-byte asynchronous copies.
+// The column step then runs one length-AY DFT per thread out of shared memory
+// (every column a task of its own: the kx = 0 and kx = M columns share one DFT
+// as the real and imaginary parts of one complex column), the x passes and the
+// epilogue run as in passes_static.cuh, the epilogue's results go straight to
+// memory, and the forward column step writes the box back into the same buffer
+// for one tiled tensor store.
 //
 // Shared memory per block: the column box, reused in place for the x rows,
-// plus the staged real rows (65 KB for 512x512x128, three blocks per SM).
+// plus the staged real rows.
 #pragma once
 #include "passes_static.cuh"
 #ifdef CLARITY_HOST_EMULATION
@@ -27,15 +26,17 @@
 namespace clarity {
 namespace st {
 
-template <class SH, int TG>
-using TileShape = Shape<typename SH::X, SH::AY, typename SH::Y, typename SH::Z, TG, SH::W>;
+template <class SH, int TG, int THR>
+using TileShape = Shape<typename SH::X, SH::AY, typename SH::Y, typename SH::Z, TG, SH::W, THR>;
 
-template <class SH>
+// Tile of TG y0 lines run by THR threads.  The box's innermost extent, TG*W
+// float2, must be a multiple of 16 bytes; a box of 16-byte runs moves at half
+// the rate of one of 32-byte runs (one sector each): at the 512x512x128 box
+// the loads and stores alone took 42 us of the product pass's 91.
+template <class SH, int TG_, int THR>
 struct XyTma {
-  // y0 lines per tile: the box's innermost extent TG*W float2 must be a
-  // multiple of 16 bytes
-  static constexpr int TG = (SH::W % 2 == 0) ? 1 : 2;
-  using T = TileShape<SH, TG>;
+  static constexpr int TG = TG_;
+  using T = TileShape<SH, TG, THR>;
   static constexpr int M = SH::M, NX = SH::NX, AY = SH::AY, W = SH::W, KG = SH::KG;
   static constexpr int BOXW = TG * W;  // float2 per (k1, kg) in the box
   static constexpr int BOX_F2 = AY * KG * BOXW;
@@ -43,19 +44,21 @@ struct XyTma {
   static constexpr int BUF_F2_RAW = BOX_F2 > ROWS_F2 ? BOX_F2 : ROWS_F2;
   static constexpr int BUF_F2 = (BUF_F2_RAW + 15) / 16 * 16;  // 128-byte multiple
   static constexpr int NROWS = TG * AY;
-  static constexpr int STG_F = NROWS * NX;
-  static constexpr int SMEM = BUF_F2 * 8 + STG_F * 4;
+  // staged rows: `stride` floats each, what the epilogue's longest row needs
+  static constexpr int stage_stride(int n) { return (n + 3) / 4 * 4; }
+  static constexpr int smem(int stride) { return BUF_F2 * 8 + NROWS * stride * 4; }
+  static constexpr int SMEM = smem(NX);
   static constexpr int TASKS = TG * M;  // column DFTs per tile
   // x twiddles (M) and the lines' y split twiddles (TG*AY) staged in shared
   // memory when three blocks per SM still fit beside the dynamic tile
   static constexpr int TW_F2 = M + TG * AY;
-  static constexpr bool TW_SMEM = 3 * (SMEM + TW_F2 * 8 + 2048 + 1024) <= 228 * 1024;
-  static constexpr int THREADS = SH::THREADS;
-  static constexpr int BLOCKS = SH::NZ * (SH::BY / TG);
-  // usable when the tile fits three 256-thread blocks per SM, every column
-  // task has a thread, the rows are whole 16-byte runs and the box is a legal
-  // TMA box
-  static constexpr bool OK = SMEM <= 72 * 1024 && THREADS == 256 && TASKS <= THREADS &&
+  static constexpr bool TW_SMEM = THR < 512 && 3 * (SMEM + TW_F2 * 8 + 2048 + 1024) <= 228 * 1024;
+  static constexpr int THREADS = THR;
+  // blocks per SM the registers are sized for (80 a thread at most)
+  static constexpr int MINB = THR <= 256 ? 768 / THR : 2;
+  // usable when every column task has a thread, the rows are whole 16-byte
+  // runs and the box is a legal TMA box
+  static constexpr bool OK = SMEM <= 200 * 1024 && SH::THREADS == 256 && TASKS <= THREADS &&
                              M % 2 == 0 && M >= 4 &&
                              AY % 2 == 0 &&
                              NX % 4 == 0 && SH::BY % TG == 0 && KG <= 256 && AY <= 256 &&
@@ -126,12 +129,11 @@ __device__ __forceinline__ void per_task_two_phase_pairs(const A& a, const B& b)
 // with the c2r pair combine of slots k and M - k done as the rows are
 // written (the pair's two columns are held by two lanes of one warp).  Only
 // rows j < L of each line are written (the later steps read no others).
-template <class SH>
+template <class SH, class X>
 __device__ __forceinline__ void cols_inverse_tma(float2* buf, int y0base,
                                                  const float2* __restrict__ twr,
                                                  const float2* twl,
-                                                 int L = XyTma<SH>::AY) {
-  using X = XyTma<SH>;
+                                                 int L = X::AY) {
   using T = typename X::T;
   constexpr int M = X::M, AY = X::AY, RS = T::ROWSTRIDE;
   auto load = [&](int c, float2* v) {
@@ -191,12 +193,11 @@ __device__ __forceinline__ void cols_inverse_tma(float2* buf, int y0base,
 // slots k and M - k happens as the columns are read: both tasks of a pair
 // read both slots and each keeps its own half.  Rows j >= L of each line
 // hold zeros, which the split maps to zeros.
-template <class SH>
+template <class SH, class X>
 __device__ __forceinline__ void cols_forward_tma(float2* buf, int y0base,
                                                  const float2* __restrict__ twr,
                                                  const float2* twl,
-                                                 int L = XyTma<SH>::AY) {
-  using X = XyTma<SH>;
+                                                 int L = X::AY) {
   using T = typename X::T;
   constexpr int M = X::M, AY = X::AY, RS = T::ROWSTRIDE;
   (void)L;
@@ -278,7 +279,7 @@ __device__ __forceinline__ void cols_forward_tma(float2* buf, int y0base,
   // padding slots kx = M+1 .. KG*W-1 of every (k1, g)
   constexpr int PADK = X::KG * X::W - (M + 1);
   if constexpr (PADK > 0) {
-    for (int f = threadIdx.x; f < AY * X::TG * PADK; f += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
+    for (int f = threadIdx.x; f < AY * X::TG * PADK; f += CLARITY_BLOCK_STRIDE(X::THREADS)) {
       const int kx = M + 1 + f % PADK;
       const int rest = f / PADK;
       buf[X::box(rest / X::TG, kx, rest % X::TG)] = make_float2(0.f, 0.f);
@@ -289,9 +290,9 @@ __device__ __forceinline__ void cols_forward_tma(float2* buf, int y0base,
 // Last inverse x pass into the epilogue with the tile row staged in shared
 // memory (srow, NX floats); FUSE re-applies forward pass 0.
 template <class T, class Epi, bool FUSE, class Skip, bool COMPACT>
-__device__ __forceinline__ void x_last_staged(float2* sm, float* stg, Epi& epi, int z, int y0base,
+__device__ __forceinline__ void x_last_staged(float2* sm, const float* stg, Epi& epi, int z, int y0base,
                                               const float2* tw, const Skip& skip,
-                                              const int* nf, int L) {
+                                              int L, int SS) {
   using X = typename T::X;
   constexpr int R = X::radix(0), span = X::span(0);
   const int total = visit_rows<T, COMPACT>(L) * span;
@@ -318,8 +319,8 @@ __device__ __forceinline__ void x_last_staged(float2* sm, float* stg, Epi& epi, 
       for (int k = 1; k < R; ++k) v[k] = cmulc(v[k], tw[i * k]);
     }
     dft<R, +1>(v);
-    float* srow = stg + r * T::NX;
-    const int n = nf[r];
+    const float* srow = stg + r * SS;
+    const int n = epi.in_row(y, z).nf;
 #pragma unroll
     for (int t = 0; t < R; ++t) v[t] = epi.apply_s(i + t * span, y, z, v[t], srow, n);
     if constexpr (FUSE) {
@@ -337,136 +338,89 @@ __device__ __forceinline__ void x_last_staged(float2* sm, float* stg, Epi& epi, 
 // The pass kernel.  S box in/out through the tensor map tm (float view of S:
 // dims {2*W*BY, NZ, KG, AY}); FUSE = false is the final inverse (no forward
 // transform, S is only read).
-template <class SH, class Epi, bool FUSE>
-__global__ void __launch_bounds__(256, 3)
-    ks_xy_tma(Epi epi, CLARITY_GRID_CONST TensorMap tm, const Tables T) {
-  CLARITY_PDL_WAIT();  // the previous pass's output is complete and visible
-  using X = XyTma<SH>;
+template <class SH, class X, class Epi, bool FUSE>
+__global__ void __launch_bounds__(X::THREADS, X::MINB)
+    ks_xy_tma(Epi epi, CLARITY_GRID_CONST TensorMap tm, const Tables T, const int SS) {
   using TS = typename X::T;
   static_assert(X::OK, "shape not supported by the TMA XY pass");
   CLARITY_DYN_SMEM(float2, buf);
   float* stg = reinterpret_cast<float*>(buf + X::BUF_F2);
-  __shared__ alignas(8) uint64_t bars[2];
-  __shared__ int nf[X::NROWS];
-  __shared__ int bulk_ok, bulk_out;
+  __shared__ alignas(8) uint64_t bar;
   constexpr int NB = SH::BY / X::TG;
   const int z = blockIdx.x / NB;
   const int y0base = (blockIdx.x - z * NB) * X::TG;
-  if (epi.zero_plane(z)) {  // neither read nor written (see Mod::zn)
-    if constexpr (requires { epi.finish_skipped(); }) epi.finish_skipped();
-    return;
-  }
   if (!smem_aligned128(buf)) {    // never expected: refuse rather than fault
     if (threadIdx.x == 0) raise_error(T.err, kErrMisaligned);
     return;
   }
-  if (threadIdx.x == 0) {
-    int ok = 1, out_ok = 1;
-    for (int r = 0; r < X::NROWS; ++r) {
-      const int g = r / X::AY, j = r - g * X::AY;
-      const RowRef rr = epi.in_row(y0base + g + SH::BY * j, z);
-      nf[r] = rr.nf;
-      if (rr.nf > 0 && (((uintptr_t)rr.p & 15u) != 0 || (rr.nf & 3) != 0)) ok = 0;
-      if constexpr (Epi::kStoreRows) {
-        // the output rows have the input rows' extent
-        const float* o = epi.out_row(y0base + g + SH::BY * j, z);
-        if (o && (((uintptr_t)o & 15u) != 0 || (rr.nf & 3) != 0)) out_ok = 0;
-      }
-    }
-    bulk_ok = ok;
-    bulk_out = out_ok;
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    mbar_arrive_expect_tx(&bars[0], (uint32_t)(X::BOX_F2 * 8));
-    tma_load_4d(buf, &tm, 2 * SH::W * y0base, z, 0, 0, &bars[0]);
-    uint32_t bytes = 0;
-    if (bulk_ok)
-      for (int r = 0; r < X::NROWS; ++r) bytes += 4u * (uint32_t)nf[r];
-    mbar_arrive_expect_tx(&bars[1], bytes);
-  }
-  __syncwarp();
-  if (threadIdx.x < 32 && bulk_ok) {
-    for (int r = threadIdx.x; r < X::NROWS; r += CLARITY_ISSUE_LANES) {
-      if (nf[r] <= 0) continue;
-      const int g = r / X::AY, j = r - g * X::AY;
-      const RowRef rr = epi.in_row(y0base + g + SH::BY * j, z);
-      bulk_load(stg + r * X::NX, rr.p, 4u * (uint32_t)rr.nf, &bars[1]);
-    }
-  }
-  if (!bulk_ok) {  // rows not 16-byte runs: plain loads
-    for (int t = threadIdx.x; t < X::STG_F; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
-      const int r = t / X::NX, x = t - r * X::NX;
-      if (x < nf[r]) {
-        const int g = r / X::AY, j = r - g * X::AY;
-        stg[t] = __ldg(epi.in_row(y0base + g + SH::BY * j, z).p + x);
-      }
-    }
-  }
-  // twiddles into shared memory while the tile is in flight: the lines'
-  // y split factors w_ny^(y0*k1) (1 for k1 = 0 or y0 = 0) and, when they fit,
-  // the x table w_M^t
+  if (threadIdx.x == 0) mbar_init(&bar, 1);
+  // twiddles into shared memory, before the previous pass has finished: the
+  // lines' y split factors w_ny^(y0*k1) (1 for k1 = 0 or y0 = 0) and, when they
+  // fit, the x table w_M^t
   __shared__ float2 s_twl[X::TG * X::AY];
   __shared__ float2 s_twx[X::TW_SMEM ? X::M : 1];
-  for (int t = threadIdx.x; t < X::TG * X::AY; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
+  for (int t = threadIdx.x; t < X::TG * X::AY; t += CLARITY_BLOCK_STRIDE(X::THREADS)) {
     const int g = t / X::AY, k1 = t - g * X::AY, y0 = y0base + g;
     s_twl[t] = (k1 != 0 && y0 != 0) ? __ldg(&T.twny[y0 * k1]) : make_float2(1.f, 0.f);
   }
   if constexpr (X::TW_SMEM)
-    for (int t = threadIdx.x; t < X::M; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) s_twx[t] = __ldg(&T.twx[t]);
+    for (int t = threadIdx.x; t < X::M; t += CLARITY_BLOCK_STRIDE(X::THREADS)) s_twx[t] = __ldg(&T.twx[t]);
   const float2* twx = X::TW_SMEM ? s_twx : T.twx;
+  CLARITY_PDL_WAIT();  // the previous pass's output is complete and visible
+  if (epi.zero_plane(z)) {  // neither read nor written (see Mod::zn)
+    if constexpr (requires { epi.finish_skipped(); }) epi.finish_skipped();
+    return;
+  }
+  // the spectrum box: the one tensor copy, issued before anything else
+  if (threadIdx.x == 0) {
+    mbar_arrive_expect_tx(&bar, (uint32_t)(X::BOX_F2 * 8));
+    tma_load_4d(buf, &tm, 2 * SH::W * y0base, z, 0, 0, &bar);
+  }
+  if constexpr (requires { epi.prepare(); }) epi.prepare();
+  // image rows an epilogue reads in place, into L2
+  if constexpr (requires { epi.prefetch_image(0, 0); })
+    if ((int)threadIdx.x < X::NROWS) {
+      const int g = threadIdx.x / X::AY, j = threadIdx.x - g * X::AY;
+      epi.prefetch_image(y0base + g + SH::BY * j, z);
+    }
+  // the real rows the epilogue reads, SS floats apart (SS a multiple of 4)
+  for (int t = threadIdx.x; t < X::NROWS * (SS / 4); t += CLARITY_BLOCK_STRIDE(X::THREADS)) {
+    const int r = t / (SS / 4), x = 4 * (t - r * (SS / 4));
+    const int g = r / X::AY, j = r - g * X::AY;
+    const RowRef rr = epi.in_row(y0base + g + SH::BY * j, z);
+    if (x + 4 <= rr.nf && ((uintptr_t)(rr.p + x) & 15u) == 0) {
+      cp_async16(stg + r * SS + x, rr.p + x);
+    } else {  // a row that is not a 16-byte run, or its end
+      for (int e = x; e < x + 4 && e < rr.nf; ++e) stg[r * SS + e] = ld_l2(rr.p + e);
+    }
+  }
   __syncthreads();
-  bool ok = mbar_wait(&bars[0], 0, T.err);
+  bool ok = mbar_wait(&bar, 0, T.err);
   if (!ok) {
-    mbar_wait(&bars[0], 0, nullptr);  // give copies in flight a last chance
-    mbar_wait(&bars[1], 0, nullptr);
+    mbar_wait(&bar, 0, nullptr);  // give the copy in flight a last chance
+    cp_async_wait_all();
     return;
   }
   // rows j >= L of every line are outside the image (zero for this epilogue)
   int L = SH::AY;
   if constexpr (Epi::has_zero_rows) L = epi.live_rows(y0base, SH::BY, SH::AY);
   constexpr bool CP = Epi::has_zero_rows;
-  cols_inverse_tma<SH>(buf, y0base, T.twr, s_twl, L);
+  if constexpr (TS::X::npass >= 2) cp_async_wait_all();  // a barrier follows
+  cols_inverse_tma<SH, X>(buf, y0base, T.twr, s_twl, L);
   const RowSkip<TS, Epi> skip{epi, z, y0base};
   x_inverse_down_to<TS, 1, RowSkip<TS, Epi>, CP>(buf, twx, skip, L);
-  if (!mbar_wait(&bars[1], 0, T.err)) {
-    mbar_wait(&bars[1], 0, nullptr);
-    return;
-  }
-  x_last_staged<TS, Epi, FUSE, RowSkip<TS, Epi>, CP>(buf, stg, epi, z, y0base, twx, skip,
-                                                     nf, L);
-  if constexpr (Epi::kStoreRows) {
-    // the epilogue's output rows, written in place of its input, leave by
-    // bulk stores while the forward transform runs
-    fence_smem_to_async();
+  if constexpr (TS::X::npass < 2) {  // no barrier since the rows were waited for
+    cp_async_wait_all();
     __syncthreads();
-    const bool rows_bulk = bulk_out != 0;
-    if (threadIdx.x < 32) {
-      for (int r = threadIdx.x; r < X::NROWS; r += CLARITY_ISSUE_LANES) {
-        const int g = r / X::AY, j = r - g * X::AY;
-        float* dst = epi.out_row(y0base + g + SH::BY * j, z);
-        if (dst && rows_bulk) bulk_store(dst, stg + r * X::NX, 4u * (uint32_t)nf[r]);
-      }
-      bulk_commit();
-    }
-    if (!rows_bulk) {  // rows that are not 16-byte runs: plain stores
-      for (int t = threadIdx.x; t < X::STG_F; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
-        const int r = t / X::NX, x = t - r * X::NX;
-        const int g = r / X::AY, j = r - g * X::AY;
-        float* dst = epi.out_row(y0base + g + SH::BY * j, z);
-        if (dst && x < nf[r]) dst[x] = stg[t];
-      }
-    }
   }
+  x_last_staged<TS, Epi, FUSE, RowSkip<TS, Epi>, CP>(buf, stg, epi, z, y0base, twx, skip, L, SS);
   if constexpr (FUSE) {
     if constexpr (CP) {
       zero_dead_rows<TS>(buf, L);
     }
     __syncthreads();
     x_forward_from<TS, 1, RowSkip<TS, Epi>, CP>(buf, twx, skip, L);
-    cols_forward_tma<SH>(buf, y0base, T.twr, s_twl, L);
+    cols_forward_tma<SH, X>(buf, y0base, T.twr, s_twl, L);
     fence_smem_to_async();
     __syncthreads();
     if (threadIdx.x == 0) {

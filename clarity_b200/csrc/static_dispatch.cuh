@@ -33,7 +33,7 @@ using ShapeW64 = st::Shape<st::Rad<8, 4>, 16, st::Rad<4>, st::Rad<8, 4>, 4, 1>;
 
 // The 512x512x128 box keeps its TMA XY pass with shared-memory twiddles and
 // three blocks per SM; a tile change that breaks this fails to compile.
-static_assert(st::XyTma<ShapeW512>::OK && st::XyTma<ShapeW512>::TW_SMEM,
+static_assert(st::XyTma<ShapeW512, 1, 256>::OK && st::XyTma<ShapeW512, 1, 256>::TW_SMEM,
               "the 512x512x128 XY tile no longer fits three TMA blocks per SM");
 
 template <class... SHs>
@@ -70,9 +70,8 @@ constexpr bool xy_staged() {
 
 // Tensor map of the spectrum S as floats {2*W*BY, NZ, KG, AY} with the box of
 // one XY tile.
-template <class SH>
+template <class SH, class X>
 inline bool encode_s_map(TensorMap* tm, const float2* S) {
-  using X = st::XyTma<SH>;
   const unsigned long long row = 2ull * SH::W * SH::BY;
   const unsigned long long dim[4] = {row, (unsigned long long)SH::NZ,
                                      (unsigned long long)SH::KG, (unsigned long long)SH::AY};
@@ -82,36 +81,61 @@ inline bool encode_s_map(TensorMap* tm, const float2* S) {
   return encode_tensor_f32_4d(tm, S, dim, stride, box);
 }
 
-// Launches the TMA XY pass when shape, epilogue and buffers allow it.
-template <class SH, bool FUSE, class F>
-inline bool try_xy_tma(const PlanEntry& pe, cudaStream_t st, const F& fn, const float2* S,
-                       int family, cudaError_t* err) {
-  using X = st::XyTma<SH>;
+// Launches the TMA XY pass on tiles X when shape, epilogue and buffers allow it.
+template <class SH, class X, bool FUSE, class F>
+inline bool try_xy_tma_tile(const PlanEntry& pe, cudaStream_t st, const F& fn, const float2* S,
+                            int family, cudaError_t* err) {
   if constexpr (X::OK && xy_staged<F>()) {
     if (!xy_tma_enabled()) return false;
     // the map depends only on S: encoded once per buffer
     static thread_local const float2* map_s = nullptr;
     static thread_local TensorMap tm;
     if (S != map_s) {
-      if (!encode_s_map<SH>(&tm, S)) {
+      if (!encode_s_map<SH, X>(&tm, S)) {
         map_s = nullptr;
         return false;
       }
       map_s = S;
     }
-    auto k = st::ks_xy_tma<SH, F, FUSE>;
+    auto k = st::ks_xy_tma<SH, X, F, FUSE>;
+    const int stride = X::stage_stride(fn.row_n());
+    const int smem = X::smem(stride);
     *err = allow_smem_st(k, X::SMEM);
     if (*err != cudaSuccess) return true;
     const st::Tables T = tables_of(pe);
     const int blocks = launch_planes(fn, SH::NZ) * (SH::BY / X::TG);
     if (blocks <= 0) return true;
     note_launch_begin(family, st);
-    CLARITY_LAUNCH_PDL(k, blocks, SH::THREADS, X::SMEM, st, pdl_enabled())(fn, tm, T);
+    CLARITY_LAUNCH_PDL(k, blocks, X::THREADS, smem, st, pdl_enabled())(fn, tm, T, stride);
     note_launch_end(family, st);
     *err = cudaGetLastError();
     return true;
   } else {
     (void)pe; (void)st; (void)fn; (void)S; (void)family; (void)err;
+    return false;
+  }
+}
+
+// The tiles of the TMA XY pass.  Boxes whose spectrum rows hold two columns
+// (16 bytes a line) take two lines and twice the threads where the staged rows
+// leave room for two such blocks per SM; one line otherwise.  Where a line has
+// few columns a block has as many threads as it has column tasks: the rest
+// only waited at barriers.
+template <class SH, bool FUSE, class F>
+inline bool try_xy_tma(const PlanEntry& pe, cudaStream_t st, const F& fn, const float2* S,
+                       int family, cudaError_t* err) {
+  if constexpr (xy_staged<F>()) {
+    constexpr int TG = SH::W % 2 == 0 ? 1 : 2;
+    constexpr int tasks = TG * SH::M;
+    constexpr int THR = tasks < 64 ? 64 : (tasks > 256 ? 256 : (tasks + 31) / 32 * 32);
+    if constexpr (SH::W == 2 && tasks == 256) {
+      using X2 = st::XyTma<SH, 2, 512>;
+      if (2 * (X2::smem(X2::stage_stride(fn.row_n())) + 4096) <= 228 * 1024 &&
+          try_xy_tma_tile<SH, X2, FUSE>(pe, st, fn, S, family, err))
+        return true;
+    }
+    return try_xy_tma_tile<SH, st::XyTma<SH, TG, THR>, FUSE>(pe, st, fn, S, family, err);
+  } else {
     return false;
   }
 }

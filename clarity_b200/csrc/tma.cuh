@@ -178,6 +178,26 @@ inline int atomicExch(int* p, int v) {
 }
 #endif
 
+// 16-byte copies from global to shared memory through L2 without registers,
+// complete after cp_async_wait_all (for the issuing thread) and a block
+// barrier.  All threads of a block issue them side by side; a bulk copy per
+// short row, issued by one warp, costs some 25 instructions a row in a chain
+// that the other warps wait for.
+__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src_gmem) {
+#ifndef CLARITY_HOST_EMULATION
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)),
+               "l"(src_gmem)
+               : "memory");
+#else
+  std::memcpy(dst_smem, src_gmem, 16);
+#endif
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+#ifndef CLARITY_HOST_EMULATION
+  asm volatile("cp.async.wait_all;" ::: "memory");
+#endif
+}
+
 // Loads through L2 that stay behind CLARITY_PDL_WAIT (both are volatile): for
 // data the previous kernels on the stream may have written.
 __device__ __forceinline__ float ld_l2(const float* p) {
