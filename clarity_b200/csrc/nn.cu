@@ -22,6 +22,7 @@
 // kernels are multiples of 16.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -663,125 +664,154 @@ __global__ void __launch_bounds__(kTmThreads, 1)
 }
 #endif
 
-// dW[co][tap][ci] += sum over this block's voxels of dy[v][co] in(v + tap)[ci]
-// (FP32 atomics; the caller zeroes dW).  GEMM M = cout (BM rows per block),
-// N = 27 cin (64 columns per block: four 16-channel groups, each one tap),
-// K = voxels (16 per step, kVoxChunk per block).  Warp w owns columns
-// [16w, 16w + 16) of the block for all BM rows.
-constexpr int kVoxChunk = 2048;
-constexpr int kWRow = 72;  // smem pitch (bf16) of the [voxel][64] tiles: conflict-free
+// dW[co][tap][ci] += sum_v dy[v][co] in(v + tap)[ci] (FP32 atomics; the caller
+// zeroes dW).  A block takes one 16-channel input chunk, BM output channels
+// and a run of 2x8x8 voxel tiles, and keeps all 27 taps' BM x 16 products in
+// registers over the whole run: warp w owns taps w, w + 4, ...  Per tile it
+// stages the chunk's 4x10x10 halo and the tile's dy once (two stages, copied
+// while the other is multiplied); per 16 voxels a warp loads its dy fragments
+// once and one input fragment per tap, at the halo's shifted rows.  What bounds
+// it is the fragment loads (one per two MMAs at BM = 16); the form it replaces
+// gathered every tap's shifted input from L2 anew, 16 voxels at a time.
+// Measured at 128x128x48, 16+32 -> 16 channels: see the launch below.
+constexpr int kWgTaps = 7;        // taps per warp (the last warp has 6)
+constexpr int kVoxTile = kTZ * kTY * kTX;  // 128
 
 template <int BM>
-__global__ void __launch_bounds__(128) k_conv3_wgrad(const Conv3Args a, const bf16* __restrict__ dy,
-                                                    float* __restrict__ dw) {
-  static_assert(BM % 16 == 0 && BM <= 64, "BM: 16, 32, 48 or 64");
-  __shared__ alignas(128) bf16 As[2][16 * kWRow];  // [voxel][co]
-  __shared__ alignas(128) bf16 Bs[2][16 * kWRow];  // [voxel][n]
-  const int cin = a.c1 + a.c2;
-  const int ngroups = 27 * (cin / 16);
-  const int N = 27 * cin;
-  const long long V = (long long)a.D * a.H * a.W;
-  const int nb = blockIdx.x;           // 64-column block
-  const int co0 = blockIdx.y * BM;
-  const long long vbeg = (long long)blockIdx.z * kVoxChunk;
-  const long long vend = vbeg + kVoxChunk < V ? vbeg + kVoxChunk : V;
-  const int nsteps = (int)((vend - vbeg + 15) / 16);
+struct WgradSmem {
+  static constexpr int DROW = BM + 8;  // pitch of a dy row: conflict-free ldmatrix
+  static constexpr int HALO = kHalo * kRow;
+  static constexpr int STAGE = HALO + kVoxTile * DROW;  // bf16 elements
+  static constexpr int BYTES = 2 * STAGE * 2;
+};
 
-  auto load = [&](int s, int stage) {
-    const long long vb = vbeg + (long long)s * 16;
-    // A: 16 voxels x BM channels of dy, BM/8 chunks per voxel
-    for (int q = threadIdx.x; q < 16 * (BM / 8); q += CLARITY_BLOCK_STRIDE(128)) {
-      const int r = q / (BM / 8), ch = q - r * (BM / 8);
-      const long long v = vb + r;
-      const bf16* src = v < vend ? dy + ((size_t)v * a.cout + co0 + ch * 8) : nullptr;
-      cp16(&As[stage][r * kWRow + ch * 8], src, dy);
+template <int BM>
+__global__ void __launch_bounds__(128, BM == 16 ? 4 : 3)
+    k_conv3_wgrad(const Conv3Args a, const bf16* __restrict__ dy, float* __restrict__ dw,
+                  int tilesx, int tilesy, int ntiles) {
+  static_assert(BM == 16 || BM == 32, "BM: 16 or 32");
+  using SMM = WgradSmem<BM>;
+  CLARITY_DYN_SMEM(bf16, sm);
+  const int cin = a.c1 + a.c2, N = 27 * cin;
+  const int c0 = blockIdx.x * 16, co0 = blockIdx.y * BM;
+  const int t0 = (int)((long long)ntiles * blockIdx.z / gridDim.z);
+  const int t1 = (int)((long long)ntiles * (blockIdx.z + 1) / gridDim.z);
+
+  auto load = [&](int tile, int stage) {
+    bf16* H = sm + stage * SMM::STAGE;
+    bf16* G = H + SMM::HALO;
+    const int txy = tile / tilesx, tx = tile - txy * tilesx;
+    const int tz = txy / tilesy, ty = txy - tz * tilesy;
+    const int z0 = tz * kTZ, y0 = ty * kTY, x0 = tx * kTX;
+    for (int q = threadIdx.x; q < kHalo * 2; q += CLARITY_BLOCK_STRIDE(128)) {
+      const int hv = q >> 1, half = q & 1;
+      const int hz = hv / (kHY * kHX), r = hv - hz * (kHY * kHX);
+      const int hy = r / kHX, hx = r - hy * kHX;
+      cp16(&H[hv * kRow + half * 8],
+           in_chunk(a, z0 + hz - 1, y0 + hy - 1, x0 + hx - 1, c0 + half * 8), a.x1);
     }
-    // B: 16 voxels x 4 groups x 2 halves of the shifted input
-    for (int q = threadIdx.x; q < 16 * 8; q += CLARITY_BLOCK_STRIDE(128)) {
-      const int r = q >> 3, gi = (q >> 1) & 3, half = q & 1;
-      const int gg = nb * 4 + gi;
-      const long long v = vb + r;
-      const bf16* src = nullptr;
-      if (v < vend && gg < ngroups) {
-        const int t = gg / (cin / 16), cc = gg - t * (cin / 16);
-        int dz, dyo, dx;
-        tap_offset(t, &dz, &dyo, &dx);
-        const int x = (int)(v % a.W);
-        const long long zy = v / a.W;
-        const int y = (int)(zy % a.H), z = (int)(zy / a.H);
-        src = in_chunk(a, z + dz, y + dyo, x + dx, cc * 16 + half * 8);
-      }
-      cp16(&Bs[stage][r * kWRow + gi * 16 + half * 8], src, a.x1);
+    for (int q = threadIdx.x; q < kVoxTile * (BM / 8); q += CLARITY_BLOCK_STRIDE(128)) {
+      const int v = q / (BM / 8), ch = q - v * (BM / 8);
+      const int z = z0 + v / (kTY * kTX), y = y0 + (v / kTX) % kTY, x = x0 + v % kTX;
+      const bf16* src = z < a.D && y < a.H && x < a.W
+                            ? dy + ((size_t)((z * a.H + y) * a.W + x) * a.cout + co0 + ch * 8)
+                            : nullptr;
+      cp16(&G[v * SMM::DROW + ch * 8], src, dy);
     }
     cp_commit();
   };
 
 #ifndef CLARITY_HOST_EMULATION
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float acc[BM / 16][2][4];
+  float acc[kWgTaps][BM / 16][2][4];
 #pragma unroll
-  for (int i = 0; i < BM / 16; ++i)
+  for (int t = 0; t < kWgTaps; ++t)
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int i = 0; i < BM / 16; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
-  if (nsteps > 0) load(0, 0);
-  for (int s = 0; s < nsteps; ++s) {
-    const int st = s & 1;
-    if (s + 1 < nsteps) {
-      load(s + 1, st ^ 1);
+      for (int e = 0; e < 8; ++e) acc[t][i][e >> 2][e & 3] = 0.f;
+  // halo row of the lane's voxel at k-step 0 and tap (0, 0, 0), and the taps'
+  // offsets (a missing 28th tap repeats the 27th and is not stored)
+  const int kr = lane & 15;
+  const int hrow = (kr >> 3) * kHX + (kr & 7);
+  int toff[kWgTaps];
+#pragma unroll
+  for (int t = 0; t < kWgTaps; ++t) {
+    const int tap = warp + 4 * t < 27 ? warp + 4 * t : 26;
+    toff[t] = ((tap / 9) * (kHY * kHX) + (tap / 3) % 3 * kHX + tap % 3) * kRow;
+  }
+  if (t0 < t1) load(t0, 0);
+  for (int tile = t0; tile < t1; ++tile) {
+    const int st = (tile - t0) & 1;
+    if (tile + 1 < t1) {
+      load(tile + 1, st ^ 1);
       cp_wait<1>();
     } else {
       cp_wait<0>();
     }
     __syncthreads();
-    // B fragments of the warp's two n8 tiles: stored [k][n], transposed load
-    uint32_t bfr[4];
-    ldm_x4_t(bfr, &Bs[st][((lane & 7) + ((lane >> 3) & 1) * 8) * kWRow + warp * 16 + (lane >> 4) * 8]);
+    const bf16* H = sm + st * SMM::STAGE;
+    const bf16* G = H + SMM::HALO;
+#pragma unroll 2
+    for (int ks = 0; ks < kVoxTile / 16; ++ks) {
+      // 16 voxels: two x rows of the tile
+      const int hz = ks / (kTY / 2), hy = 2 * (ks % (kTY / 2));
+      const bf16* hb = H + (hz * (kHY * kHX) + hy * kHX + hrow) * kRow + (lane >> 4) * 8;
+      uint32_t af[BM / 16][4];
 #pragma unroll
-    for (int i = 0; i < BM / 16; ++i) {
-      // A fragment (rows co, cols voxel) from the stored [voxel][co] tile
-      uint32_t af[4];
-      ldm_x4_t(af, &As[st][((lane & 7) + (lane >> 4) * 8) * kWRow + i * 16 + ((lane >> 3) & 1) * 8]);
-      mma16816(acc[i][0], af, bfr);
-      mma16816(acc[i][1], af, bfr + 2);
+      for (int i = 0; i < BM / 16; ++i)
+        ldm_x4_t(af[i], &G[(ks * 16 + (lane & 7) + (lane >> 4) * 8) * SMM::DROW + i * 16 +
+                           ((lane >> 3) & 1) * 8]);
+#pragma unroll
+      for (int t = 0; t < kWgTaps; ++t) {
+        uint32_t bfr[4];
+        ldm_x4_t(bfr, hb + toff[t]);
+#pragma unroll
+        for (int i = 0; i < BM / 16; ++i) {
+          mma16816(acc[t][i][0], af[i], bfr);
+          mma16816(acc[t][i][1], af[i], bfr + 2);
+        }
+      }
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < BM / 16; ++i)
+  for (int t = 0; t < kWgTaps; ++t) {
+    const int tap = warp + 4 * t;
+    if (tap >= 27 || t0 >= t1) continue;
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int i = 0; i < BM / 16; ++i)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int co = co0 + i * 16 + (lane >> 2) + h * 8;
-        const int nl = warp * 16 + j * 8 + (lane & 3) * 2;  // column in the block
-        const int gg = nb * 4 + (nl >> 4);
-        if (gg >= ngroups) continue;
-        const int n = nb * 64 + nl;
-        atomicAdd(&dw[(size_t)co * N + n], acc[i][j][2 * h]);
-        atomicAdd(&dw[(size_t)co * N + n + 1], acc[i][j][2 * h + 1]);
-      }
-#else
-  static thread_local float accs[64][64];
-  for (int m = 0; m < BM; ++m)
-    for (int n = 0; n < 64; ++n) accs[m][n] = 0.f;
-  for (int s = 0; s < nsteps; ++s) {
-    load(s, 0);
-    for (int m = 0; m < BM; ++m)
-      for (int n = 0; n < 64; ++n) {
-        float t = 0.f;
-        for (int k = 0; k < 16; ++k)
-          t += __bfloat162float(As[0][k * kWRow + m]) * __bfloat162float(Bs[0][k * kWRow + n]);
-        accs[m][n] += t;
-      }
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int co = co0 + i * 16 + (lane >> 2) + h * 8;
+          float* d = &dw[(size_t)co * N + tap * cin + c0 + j * 8 + (lane & 3) * 2];
+          atomicAdd(d, acc[t][i][j][2 * h]);
+          atomicAdd(d + 1, acc[t][i][j][2 * h + 1]);
+        }
   }
-  for (int m = 0; m < BM; ++m)
-    for (int n = 0; n < 64; ++n) {
-      const int gg = nb * 4 + (n >> 4);
-      if (gg >= ngroups) continue;
-      dw[(size_t)(co0 + m) * N + nb * 64 + n] += accs[m][n];
+#else
+  static thread_local float accs[27][BM][16];
+  std::memset(accs, 0, sizeof(accs));
+  for (int tile = t0; tile < t1; ++tile) {
+    load(tile, 0);
+    const bf16* H = sm;
+    const bf16* G = H + SMM::HALO;
+    for (int v = 0; v < kVoxTile; ++v) {
+      const int h0 = (v / (kTY * kTX) * kHY + (v / kTX) % kTY) * kHX + v % kTX;
+      for (int t = 0; t < 27; ++t) {
+        const bf16* h = H + (h0 + t / 9 * (kHY * kHX) + t / 3 % 3 * kHX + t % 3) * kRow;
+        for (int m = 0; m < BM; ++m)
+          for (int n = 0; n < 16; ++n)
+            accs[t][m][n] += __bfloat162float(G[v * SMM::DROW + m]) * __bfloat162float(h[n]);
+      }
     }
+  }
+  for (int t = 0; t < 27; ++t)
+    for (int m = 0; m < BM; ++m)
+      for (int n = 0; n < 16; ++n)
+        dw[(size_t)(co0 + m) * N + t * cin + c0 + n] += accs[t][m][n];
 #endif
 }
 
@@ -970,16 +1000,34 @@ __global__ void k_up_grad(const bf16* __restrict__ dxcat, int ccat, int c1, int 
   }
 }
 
-// db[co] += sum_v dy[v][co]
+// db[co] += sum_v dy[v][co].  A thread keeps one octet of channels (blockDim is
+// a multiple of cout/8, or less than that many), reads 16 bytes a voxel and
+// sums in registers; one shared-memory atomic per thread and channel and one
+// global per block and channel at the end.
 __global__ void k_bias_grad(const bf16* __restrict__ dy, long long V, int cout,
                             float* __restrict__ db) {
   CLARITY_DYN_SMEM(float, sb);
   for (int i = threadIdx.x; i < cout; i += blockDim.x) sb[i] = 0.f;
   __syncthreads();
-  const long long n = V * cout;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    atomicAdd(&sb[i % cout], __bfloat162float(dy[i]));
+  const int noct = cout / 8;
+  for (int o = threadIdx.x % noct; o < noct; o += blockDim.x) {
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const int lanes = blockDim.x < noct ? 1 : blockDim.x / noct;
+    for (long long v = blockIdx.x * (long long)lanes + threadIdx.x / noct; v < V;
+         v += (long long)gridDim.x * lanes) {
+      const uint4 q = *reinterpret_cast<const uint4*>(dy + v * cout + o * 8);
+      const unsigned w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        __nv_bfloat162 b;
+        memcpy(&b, &w[k], 4);
+        s[2 * k] += __bfloat162float(b.x);
+        s[2 * k + 1] += __bfloat162float(b.y);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) atomicAdd(&sb[o * 8 + k], s[k]);
+  }
   __syncthreads();
   for (int i = threadIdx.x; i < cout; i += blockDim.x) atomicAdd(&db[i], sb[i]);
 }
@@ -1241,21 +1289,37 @@ CLARITY_API ClarityResult_t clarityx_nn_conv3_wgrad(const void* x1, int c1, cons
                    D / 2, H / 2, W / 2, nullptr, nullptr, cout, 0, nullptr, nullptr};
   const long long V = (long long)D * H * W;
   const int cin = c1 + c2;
-  const int nblk = (27 * (cin / 16) + 3) / 4;
-  const int bm = cout % 64 == 0 ? 64 : (cout % 48 == 0 ? 48 : (cout % 32 == 0 ? 32 : 16));
-  const dim3 grid(nblk, cout / bm, (unsigned)((V + nnk::kVoxChunk - 1) / nnk::kVoxChunk));
+  // 32 output channels a block where they divide: twice the MMAs per input
+  // fragment; more would not leave registers for three blocks per SM
+  const int bm = cout % 32 == 0 ? 32 : 16;
+  const int tx = (W + nnk::kTX - 1) / nnk::kTX, ty = (H + nnk::kTY - 1) / nnk::kTY;
+  const int ntiles = tx * ty * ((D + nnk::kTZ - 1) / nnk::kTZ);
+  // runs of tiles: enough blocks for the SMs several times over, but at least
+  // four tiles each (once every SM has a block) so that a block's 27 * 16 * bm
+  // atomics stay a small part,
+  // and at most 12 (96 MMAs into one accumulator): the tensor cores' FP32 sums
+  // lose about an ulp a step, and with 31 tiles a run dW's error against 64 bits
+  // was 1.3e-6 where runs of 128 MMAs had 8e-7
+  const int cols = (cin / 16) * (cout / bm);
+  const int runs = std::max((ntiles + 11) / 12,
+                            std::min((148 * (bm == 16 ? 4 : 3) + cols - 1) / cols,
+                                     std::max(ntiles / 4, std::min(ntiles, 148 / cols + 1))));
+  const dim3 grid(cin / 16, cout / bm, runs);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bf16* d = static_cast<const bf16*>(dy);
+  auto kern = bm == 32 ? nnk::k_conv3_wgrad<32> : nnk::k_conv3_wgrad<16>;
+  const int smem = bm == 32 ? nnk::WgradSmem<32>::BYTES : nnk::WgradSmem<16>::BYTES;
+  const cudaError_t se = clarity::smem_opt_in(reinterpret_cast<const void*>(kern), smem);
+  if (se != cudaSuccess) return (ClarityResult_t)nn_err(se);
   clarity::note_launch_begin(clarity::KK_OTHER, st);
-  switch (bm) {
-    case 64: CLARITY_LAUNCH(nnk::k_conv3_wgrad<64>, grid, 128, 0, st)(a, d, dw); break;
-    case 48: CLARITY_LAUNCH(nnk::k_conv3_wgrad<48>, grid, 128, 0, st)(a, d, dw); break;
-    case 32: CLARITY_LAUNCH(nnk::k_conv3_wgrad<32>, grid, 128, 0, st)(a, d, dw); break;
-    default: CLARITY_LAUNCH(nnk::k_conv3_wgrad<16>, grid, 128, 0, st)(a, d, dw); break;
+  CLARITY_LAUNCH(kern, grid, 128, smem, st)(a, d, dw, tx, ty, ntiles);
+  if (dbias) {
+    const int noct = cout / 8;
+    const int bt = noct >= 256 ? 256 : 256 / noct * noct;
+    const long long per = 8 * std::max(1, bt / noct);  // voxels that keep a block busy
+    const int nb = (int)std::min<long long>(296, (V + per - 1) / per);
+    CLARITY_LAUNCH(nnk::k_bias_grad, nb, bt, cout * sizeof(float), st)(d, V, cout, dbias);
   }
-  if (dbias)
-    CLARITY_LAUNCH(nnk::k_bias_grad, nnk::grid_for(V * cout), 256, cout * sizeof(float), st)(
-        d, V, cout, dbias);
   clarity::note_launch_end(clarity::KK_OTHER, st);
   return (ClarityResult_t)nn_err(cudaGetLastError());
 }

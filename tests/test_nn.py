@@ -88,6 +88,43 @@ def test_conv3_forward_backward_vs_reference(clarity_gpu, c1, c2, cout, dims):
     _close(db, dy.to(torch.float64).sum(dim=(0, 1, 2)), rel=1e-2)
 
 
+@pytest.mark.parametrize("dims,c1,c2,cout", [
+    ((1, 1, 1), 16, 0, 16),       # one voxel: every neighbour is padding
+    ((3, 9, 17), 16, 0, 32),      # remainders of the 2x8x8 tile on every axis
+    ((6, 10, 14), 32, 16, 48),    # upsampled second input, 48 = 3 x 16 channels
+    ((4, 16, 24), 16, 32, 64),    # whole tiles
+    ((26, 40, 40), 16, 0, 16),    # runs of several tiles per block
+])
+def test_conv3_weight_gradient_at_tile_edges(clarity_gpu, dims, c1, c2, cout):
+    # BF16 products are exact in FP32; a sum is at most 96 MMA accumulations
+    # and 128 atomic additions long, each within an ulp of its partial sum
+    from clarity_b200 import unet
+    D, H, W = dims
+    g = torch.Generator().manual_seed(sum(dims) + cout)
+    rnd = lambda *s: torch.randn(s, generator=g).to(torch.bfloat16)  # noqa: E731
+    x1, dy = rnd(D, H, W, c1), rnd(D, H, W, cout)
+    x2 = rnd(D // 2, H // 2, W // 2, c2) if c2 else None
+    cin = c1 + c2
+    dw = torch.zeros(cout * 27 * cin, device="cuda")
+    db = torch.zeros(cout, device="cuda")
+    unet.conv3_wgrad(x1.cuda(), dy.cuda(), dw, db, x2=x2.cuda() if c2 else None)
+    torch.cuda.synchronize()
+    x = x1.double()
+    if c2:
+        up = x2.double()
+        for d in range(3):
+            up = up.repeat_interleave(2, d)
+        x = torch.cat([x, up], 3)
+    p = torch.nn.functional.pad(x, (0, 0, 1, 1, 1, 1, 1, 1))
+    f = dy.double().reshape(-1, cout)
+    bound = 256 * 2.0 ** -24
+    got = dw.cpu().double().reshape(cout, 27, cin)
+    for t in range(27):
+        sh = p[t // 9:t // 9 + D, t // 3 % 3:t // 3 % 3 + H, t % 3:t % 3 + W].reshape(-1, cin)
+        assert ((got[:, t] - f.T @ sh).abs() <= bound * (f.abs().T @ sh.abs()) + 1e-30).all(), t
+    assert ((db.cpu().double() - f.sum(0)).abs() <= bound * f.abs().sum(0) + 1e-30).all()
+
+
 _CROSS = """
 import sys, numpy as np, torch
 from clarity_b200 import unet
