@@ -139,7 +139,7 @@ struct ProWork {
 };
 
 // Rows y0base + by*j of a line group that lie below Y (j < the result).
-__device__ __forceinline__ int rows_below(int Y, int y0base, int by, int ay) {
+CLARITY_HD inline int rows_below(int Y, int y0base, int by, int ay) {
   const int l = (Y - y0base + by - 1) / by;
   return l < 0 ? 0 : (l > ay ? ay : l);
 }
@@ -194,7 +194,7 @@ struct ProAccel {
   int live_planes(int nz) const { return Z < nz ? Z : nz; }
   __device__ __forceinline__ int plane(int p) const { return p; }
   static constexpr bool has_zero_rows = true;
-  __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
+  CLARITY_HD inline int live_rows(int y0base, int by, int ay) const {
     return rows_below(Y, y0base, by, ay);
   }
   __device__ __forceinline__ void finish() const {}
@@ -257,7 +257,7 @@ struct ProImage {
   int live_planes(int nz) const { return p.Z < nz ? p.Z : nz; }
   __device__ __forceinline__ int plane(int q) const { return q; }
   static constexpr bool has_zero_rows = true;
-  __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
+  CLARITY_HD inline int live_rows(int y0base, int by, int ay) const {
     return rows_below(p.Y, y0base, by, ay);
   }
   __device__ __forceinline__ void finish() const {}
@@ -387,7 +387,7 @@ struct EpiClip {
   __device__ __forceinline__ bool zero_row(int y, int z) const { return y >= Y || z >= Z; }
   __device__ __forceinline__ bool zero_plane(int z) const { return z >= Z; }
   int live_planes(int nz) const { return Z < nz ? Z : nz; }
-  __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
+  CLARITY_HD inline int live_rows(int y0base, int by, int ay) const {
     return rows_below(Y, y0base, by, ay);
   }
   __device__ __forceinline__ void prefetch_row(int, int) const {}
@@ -454,14 +454,14 @@ struct EpiRLProduct {
   __device__ __forceinline__ bool zero_row(int y, int z) const { return y >= Y || z >= Z; }
   __device__ __forceinline__ bool zero_plane(int z) const { return z >= Z; }
   int live_planes(int nz) const { return Z < nz ? Z : nz; }
-  __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
+  CLARITY_HD inline int live_rows(int y0base, int by, int ay) const {
     return rows_below(Y, y0base, by, ay);
   }
   // the estimate row this block's epilogue will read, into L2
   __device__ __forceinline__ void prefetch_row(int y, int z) const {
     if (y < Y && z < Z) prefetch_l2_range(cur + at(0, y, z), sizeof(float) * (size_t)X);
   }
-  // Staged form (passes_xy_tma.cuh): row (y, z) of cur arrives in shared memory
+  // Staged form (passes_xy_rows.cuh): row (y, z) of cur arrives in shared memory
   // (n floats at sr).
   static constexpr bool kStaged = true;
   __device__ __forceinline__ st::RowRef in_row(int y, int z) const {
@@ -564,7 +564,7 @@ struct MidRLRatio {
   // planes a launch needs to cover (the rest are zero_plane)
   int live_planes(int nz) const { return g.Z < nz ? g.Z : nz; }
   // rows y0base + by*j with j < live_rows lie inside the image (y < Y)
-  __device__ __forceinline__ int live_rows(int y0base, int by, int ay) const {
+  CLARITY_HD inline int live_rows(int y0base, int by, int ay) const {
     return rows_below(g.Y, y0base, by, ay);
   }
   __device__ __forceinline__ void prefetch_row(int y, int z) const {

@@ -62,13 +62,6 @@ __device__ __forceinline__ float4 put(const c2& v) {
   return make_float4(v.re.x, v.re.y, v.im.x, v.im.y);
 }
 __device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
-__device__ __forceinline__ int quot(int n, FDiv D) {
-#ifndef CLARITY_HOST_EMULATION
-  return (int)(__umulhi((unsigned)n, D.m) + ((unsigned)n & D.one));
-#else
-  return (int)((((unsigned long long)(unsigned)n * D.m) >> 32) + ((unsigned)n & D.one));
-#endif
-}
 
 // v[k] *= w_n^(DIR k i) (DIR = -1 forward: the table's w; +1: conjugate); W:
 // float2 entries, or float4 with both parts twice

@@ -721,9 +721,14 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
 
 // ----------------------------------------------- Z kernel, y0 per line
 // z-axis register pass S over the padded tile: lines l0 < BW (adjacent in
-// memory), element e of line l0 at l0 + e*ZS.
-template <class SH, int S, int DIR>
-__device__ __forceinline__ void z2_pass(float2* sm, const float2* __restrict__ tw) {
+// memory), element e of line l0 at l0 + e*ZS.  With EDGE pass 0 knows the planes:
+// forward it reads planes z0 <= z < z1 as zeros, inverse it stores planes
+// z < z0 only.  (The test is the same for a whole warp, lanes sharing i; it pays
+// in ks_z3's long sweeps, while it made ks_z2 at the 512x512x128 box slower,
+// 70 -> 75 us.)
+template <class SH, int S, int DIR, bool EDGE = false>
+__device__ __forceinline__ void z2_pass(float2* sm, const float2* __restrict__ tw, int z0 = 0,
+                                        int z1 = 0) {
   using A = typename SH::Z;
   constexpr int R = A::radix(S), len = A::len(S), span = len / R;
   constexpr int per_line = A::n / R, twstep = A::n / len;
@@ -737,7 +742,12 @@ __device__ __forceinline__ void z2_pass(float2* sm, const float2* __restrict__ t
     const int base = l0 + (b * len + i) * SH::ZS;
     float2 v[R];
 #pragma unroll
-    for (int t = 0; t < R; ++t) v[t] = sm[base + t * span * SH::ZS];
+    for (int t = 0; t < R; ++t) {
+      if (EDGE && S == 0 && DIR < 0 && i + t * span >= z0 && i + t * span < z1)
+        v[t] = make_float2(0.f, 0.f);
+      else
+        v[t] = sm[base + t * span * SH::ZS];
+    }
     if constexpr (DIR < 0) {
       dft<R, -1>(v);
       if (span > 1 && i != 0) {
@@ -752,7 +762,8 @@ __device__ __forceinline__ void z2_pass(float2* sm, const float2* __restrict__ t
       dft<R, +1>(v);
     }
 #pragma unroll
-    for (int t = 0; t < R; ++t) sm[base + t * span * SH::ZS] = v[t];
+    for (int t = 0; t < R; ++t)
+      if (!(EDGE && S == 0 && DIR > 0) || i + t * span < z0) sm[base + t * span * SH::ZS] = v[t];
   }
 }
 
@@ -789,6 +800,32 @@ __device__ __forceinline__ void z2_last(float2* sm, const Mod& mod, unsigned gba
 #pragma unroll
       for (int t = 0; t < R; ++t) sm[sbase + t * SH::ZS] = v[t];
     }
+  }
+}
+
+// The z passes of a tile whose y0 lines are transformed: forward, spectral
+// operation, inverse (planes z < zo), with a barrier after each but a forward-
+// only last one.
+template <class SH, bool EDGE, class Mod>
+__device__ __forceinline__ void z2_spectral(float2* sm, const Mod& mod, unsigned gbase,
+                                            float2* __restrict__ out, const float2* twz, int z0,
+                                            int z1, int zo) {
+  using A = typename SH::Z;
+  z2_pass<SH, 0, -1, EDGE>(sm, twz, z0, z1);
+  __syncthreads();
+  if constexpr (A::npass >= 3) {
+    z2_pass<SH, 1, -1>(sm, twz);
+    __syncthreads();
+  }
+  z2_last<SH>(sm, mod, gbase, out);
+  if constexpr (!Mod::forward_only) {
+    __syncthreads();
+    if constexpr (A::npass >= 3) {
+      z2_pass<SH, 1, +1>(sm, twz);
+      __syncthreads();
+    }
+    z2_pass<SH, 0, +1, EDGE>(sm, twz, zo);
+    __syncthreads();
   }
 }
 
@@ -858,27 +895,10 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
     for (int k = 0; k < BY; ++k) d[k * W] = v[k];
   }
   __syncthreads();
-  if constexpr (A::npass >= 2) {
-    z2_pass<SH, 0, -1>(sm, twz);
-    __syncthreads();
-  }
-  if constexpr (A::npass >= 3) {
-    z2_pass<SH, 1, -1>(sm, twz);
-    __syncthreads();
-  }
-  z2_last<SH>(sm, mod, gbase, Sout);
+  const int zo = mod.zout < NZ ? mod.zout : NZ;
+  z2_spectral<SH, false>(sm, mod, gbase, Sout, twz, zn, zn + gap, zo);
   if constexpr (!Mod::forward_only) {
-    __syncthreads();
-    if constexpr (A::npass >= 3) {
-      z2_pass<SH, 1, +1>(sm, twz);
-      __syncthreads();
-    }
-    if constexpr (A::npass >= 2) {
-      z2_pass<SH, 0, +1>(sm, twz);
-      __syncthreads();
-    }
     // y0 inverse per line, for the planes the next pass reads (z < zo)
-    const int zo = mod.zout < NZ ? mod.zout : NZ;
 #pragma unroll 1
     for (int l = threadIdx.x; l < zo * W; l += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
       const int ki = l % W, z = l / W;
@@ -905,6 +925,97 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
         *reinterpret_cast<float4*>(Sout + gbase + z * BW + c) =
             *reinterpret_cast<const float4*>(sm + z * ZS + c);
       }
+    }
+  }
+}
+
+// ------------------------------------ Z kernel, y0 in several passes
+// y0 register pass S over `planes` live planes (the q-th is q, or q + gap
+// beyond zn), W = 1: consecutive threads take consecutive planes, ZS (odd)
+// apart.  In the unpadded tile of ks_z consecutive threads shared a line and
+// its accesses 8 elements apart fell on two banks.
+template <class SH, int S, int DIR>
+__device__ __forceinline__ void y3_pass(float2* sm, const float2* tw, int planes, FDiv dplanes,
+                                        int zn, int gap) {
+  using A = typename SH::Y;
+  constexpr int R = A::radix(S), len = A::len(S), span = len / R;
+  constexpr int per_line = A::n / R, twstep = A::n / len;
+  const int total = planes * per_line;
+#pragma unroll 1
+  for (int f = threadIdx.x; f < total; f += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
+    const int rem = quot(f, dplanes), q = f - rem * planes;
+    const int z = q < zn ? q : q + gap;
+    const int b = rem / span, i = rem - b * span;
+    float2* p = sm + z * SH::ZS + b * len + i;
+    float2 v[R];
+#pragma unroll
+    for (int t = 0; t < R; ++t) v[t] = p[t * span];
+    if constexpr (DIR < 0) dft<R, -1>(v);
+    if (span > 1 && i != 0) {
+#pragma unroll
+      for (int k = 1; k < R; ++k)
+        v[k] = DIR < 0 ? cmul(v[k], tw[i * k * twstep]) : cmulc(v[k], tw[i * k * twstep]);
+    }
+    if constexpr (DIR > 0) dft<R, +1>(v);
+#pragma unroll
+    for (int t = 0; t < R; ++t) p[t * span] = v[t];
+  }
+}
+
+// The FP32 z kernel of boxes with BY > 32 (W = 1): ks_z2 with the y0 axis in
+// two register passes over the live planes and every table in shared memory.
+// One padded tile (133 KB at the 1024x1024x256 box) and 1024 threads per SM;
+// there a pass that reads and wants half the planes went from 1334 to 751 us.
+template <class SH>
+struct Z3 {
+  static constexpr bool OK = !SH::Y_PER_LINE && SH::W == 1 && SH::Y::npass == 2 &&
+                             SH::Z::npass >= 2 && SH::BY % 2 == 0 && (SH::ZS & 1) == 1;
+  static constexpr int SMEM = SH::Z2_TILE_BYTES + (SH::NZ + SH::BY) * 8;
+};
+template <class SH, class Mod>
+__global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
+    ks_z3(const Mod mod, const float2* __restrict__ Sin, float2* __restrict__ Sout,
+          const Tables T) {
+  CLARITY_DYN_SMEM(float2, sm);
+  constexpr int BW = SH::BW, NZ = SH::NZ, ZS = SH::ZS;
+  static_assert(Z3<SH>::OK, "shape not supported by ks_z3");
+  float2* twz = sm + SH::Z2_TILE_BYTES / 8;
+  float2* twy = twz + NZ;
+  for (int t = threadIdx.x; t < NZ; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) twz[t] = __ldg(&T.twz[t]);
+  for (int t = threadIdx.x; t < BW; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) twy[t] = __ldg(&T.twy[t]);
+  CLARITY_PDL_WAIT();  // the previous kernel's output is complete and visible
+  const unsigned gbase = blockIdx.x * (unsigned)SH::TILE;
+  const int zn = mod.zn < NZ ? mod.zn : NZ;
+  const int gap = (mod.zh < NZ ? mod.zh : NZ) - zn;
+  const int zo = mod.zout < NZ ? mod.zout : NZ;
+  if (threadIdx.x < 4) mod.prefetch_tile(gbase, SH::TILE, threadIdx.x, 4);
+  constexpr int CH = BW / 2;  // 16-byte pieces of a plane's row
+#pragma unroll 4
+  for (int t = threadIdx.x; t < (NZ - gap) * CH; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
+    const int q = t / CH, c = 2 * (t - q * CH);
+    const int z = q < zn ? q : q + gap;
+    const float4 v = ld_l2(reinterpret_cast<const float4*>(Sin + gbase + z * BW + c));
+    sm[z * ZS + c] = make_float2(v.x, v.y);
+    sm[z * ZS + c + 1] = make_float2(v.z, v.w);
+  }
+  __syncthreads();
+  const FDiv dlive = fdiv_by(NZ - gap);
+  y3_pass<SH, 0, -1>(sm, twy, NZ - gap, dlive, zn, gap);
+  __syncthreads();
+  y3_pass<SH, 1, -1>(sm, twy, NZ - gap, dlive, zn, gap);
+  __syncthreads();
+  z2_spectral<SH, true>(sm, mod, gbase, Sout, twz, zn, zn + gap, zo);
+  if constexpr (!Mod::forward_only) {
+    const FDiv dout = fdiv_by(zo);
+    y3_pass<SH, 1, +1>(sm, twy, zo, dout, zo, 0);
+    __syncthreads();
+    y3_pass<SH, 0, +1>(sm, twy, zo, dout, zo, 0);
+    __syncthreads();
+#pragma unroll 4
+    for (int t = threadIdx.x; t < zo * CH; t += CLARITY_BLOCK_STRIDE(SH::THREADS)) {
+      const int z = t / CH, c = 2 * (t - z * CH);
+      const float2 a = sm[z * ZS + c], b = sm[z * ZS + c + 1];
+      *reinterpret_cast<float4*>(Sout + gbase + z * BW + c) = make_float4(a.x, a.y, b.x, b.y);
     }
   }
 }

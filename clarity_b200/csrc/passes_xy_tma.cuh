@@ -39,6 +39,14 @@ struct XyTma {
   using T = TileShape<SH, TG, THR>;
   static constexpr int M = SH::M, NX = SH::NX, AY = SH::AY, W = SH::W, KG = SH::KG;
   static constexpr int BOXW = TG * W;  // float2 per (k1, kg) in the box
+  // a TMA box is at most 256 wide: KB boxes of KGB column groups side by side
+  static constexpr int boxes() {
+    int n = 1;
+    while (KG % n != 0 || KG / n > 256) ++n;
+    return n;
+  }
+  static constexpr int KB = boxes(), KGB = KG / KB;
+  static constexpr int KB_F2 = AY * KGB * BOXW;  // float2 of one box
   static constexpr int BOX_F2 = AY * KG * BOXW;
   static constexpr int ROWS_F2 = TG * T::GSTRIDE;
   static constexpr int BUF_F2_RAW = BOX_F2 > ROWS_F2 ? BOX_F2 : ROWS_F2;
@@ -52,20 +60,25 @@ struct XyTma {
   // x twiddles (M) and the lines' y split twiddles (TG*AY) staged in shared
   // memory when three blocks per SM still fit beside the dynamic tile
   static constexpr int TW_F2 = M + TG * AY;
-  static constexpr bool TW_SMEM = THR < 512 && 3 * (SMEM + TW_F2 * 8 + 2048 + 1024) <= 228 * 1024;
+  static constexpr bool TW_SMEM =
+      THR >= 512 || 3 * (SMEM + TW_F2 * 8 + 2048 + 1024) <= 228 * 1024;
+  // static shared memory and the system's share of a block
+  static constexpr int EXTRA = (TW_SMEM ? TW_F2 : TG * AY) * 8 + 2048;
+  // blocks per SM that rows of `stride` staged floats allow
+  static constexpr int blocks_per_sm(int stride) { return 228 * 1024 / (smem(stride) + EXTRA); }
   static constexpr int THREADS = THR;
   // blocks per SM the registers are sized for (80 a thread at most)
-  static constexpr int MINB = THR <= 256 ? 768 / THR : 2;
+  static constexpr int MINB = THR <= 256 ? 768 / THR : 1024 / THR;
   // usable when every column task has a thread, the rows are whole 16-byte
   // runs and the box is a legal TMA box
-  static constexpr bool OK = SMEM <= 200 * 1024 && SH::THREADS == 256 && TASKS <= THREADS &&
-                             M % 2 == 0 && M >= 4 &&
+  static constexpr bool OK = TASKS <= THREADS && KB_F2 * 8 % 128 == 0 && M % 2 == 0 && M >= 4 &&
                              AY % 2 == 0 &&
-                             NX % 4 == 0 && SH::BY % TG == 0 && KG <= 256 && AY <= 256 &&
+                             NX % 4 == 0 && SH::BY % TG == 0 && AY <= 256 &&
                              (BOXW * 8) % 16 == 0;
   // box float2 index of column kx of tile line g at k1
   __device__ __forceinline__ static int box(int k1, int kx, int g) {
-    return (k1 * KG + kx / W) * BOXW + g * W + kx % W;
+    const int kg = kx / W;
+    return ((kg / KGB * AY + k1) * KGB + kg % KGB) * BOXW + g * W + kx % W;
   }
 };
 
@@ -322,7 +335,11 @@ __device__ __forceinline__ void x_last_staged(float2* sm, const float* stg, Epi&
     const float* srow = stg + r * SS;
     const int n = epi.in_row(y, z).nf;
 #pragma unroll
-    for (int t = 0; t < R; ++t) v[t] = epi.apply_s(i + t * span, y, z, v[t], srow, n);
+    for (int t = 0; t < R; ++t) {
+      // beyond the longest row, for every thread alike: zero, nothing to do
+      if (2 * t * span >= epi.row_n()) v[t] = make_float2(0.f, 0.f);
+      else v[t] = epi.apply_s(i + t * span, y, z, v[t], srow, n);
+    }
     if constexpr (FUSE) {
       dft<R, -1>(v);
       if (i != 0) {
@@ -371,10 +388,12 @@ __global__ void __launch_bounds__(X::THREADS, X::MINB)
     if constexpr (requires { epi.finish_skipped(); }) epi.finish_skipped();
     return;
   }
-  // the spectrum box: the one tensor copy, issued before anything else
+  // the spectrum box, issued before anything else
   if (threadIdx.x == 0) {
     mbar_arrive_expect_tx(&bar, (uint32_t)(X::BOX_F2 * 8));
-    tma_load_4d(buf, &tm, 2 * SH::W * y0base, z, 0, 0, &bar);
+#pragma unroll
+    for (int b = 0; b < X::KB; ++b)
+      tma_load_4d(buf + b * X::KB_F2, &tm, 2 * SH::W * y0base, z, b * X::KGB, 0, &bar);
   }
   if constexpr (requires { epi.prepare(); }) epi.prepare();
   // image rows an epilogue reads in place, into L2
@@ -424,7 +443,9 @@ __global__ void __launch_bounds__(X::THREADS, X::MINB)
     fence_smem_to_async();
     __syncthreads();
     if (threadIdx.x == 0) {
-      tma_store_4d(&tm, 2 * SH::W * y0base, z, 0, 0, buf);
+#pragma unroll
+      for (int b = 0; b < X::KB; ++b)
+        tma_store_4d(&tm, 2 * SH::W * y0base, z, b * X::KGB, 0, buf + b * X::KB_F2);
       bulk_commit();
     }
   }

@@ -86,6 +86,14 @@ CLARITY_HD inline FDiv fdiv_by(int d) {
   return FDiv{0xFFFFFFFFu / (unsigned)d + 1u, 0u};
 }
 
+CLARITY_HD inline int quot(int n, FDiv D) {
+#ifdef __CUDA_ARCH__
+  return (int)(__umulhi((unsigned)n, D.m) + ((unsigned)n & D.one));
+#else
+  return (int)((((unsigned long long)(unsigned)n * D.m) >> 32) + ((unsigned)n & D.one));
+#endif
+}
+
 // Plan of the column-pair passes (passes_pair.cuh) for one work box.  The x
 // transforms run on pairs of real rows held as one complex row of full length
 // nx (no r2c split; odd nx costs what even nx does), two pairs per register

@@ -11,6 +11,7 @@
 #include "engine.hpp"
 #include "ops.cuh"
 #include "passes_static.cuh"
+#include "passes_xy_rows.cuh"
 #include "passes_xy_tma.cuh"
 
 namespace clarity {
@@ -30,11 +31,6 @@ using ShapeW128 = st::Shape<st::Rad<8, 8>, 16, st::Rad<8>, st::Rad<8, 8>, 1, 4>;
 using ShapeW1024 = st::Shape<st::Rad<8, 8, 8>, 16, st::Rad<8, 8>, st::Rad<16, 16>, 2, 1,
                              CLARITY_W1024_THREADS, CLARITY_W1024_Z_THREADS>;
 using ShapeW64 = st::Shape<st::Rad<8, 4>, 16, st::Rad<4>, st::Rad<8, 4>, 4, 1>;
-
-// The 512x512x128 box keeps its TMA XY pass with shared-memory twiddles and
-// three blocks per SM; a tile change that breaks this fails to compile.
-static_assert(st::XyTma<ShapeW512, 1, 256>::OK && st::XyTma<ShapeW512, 1, 256>::TW_SMEM,
-              "the 512x512x128 XY tile no longer fits three TMA blocks per SM");
 
 template <class... SHs>
 struct ShapeList {};
@@ -59,8 +55,8 @@ inline cudaError_t allow_smem_st(K kernel, int smem) {
   return smem_opt_in(reinterpret_cast<const void*>(kernel), smem);
 }
 
-// The TMA XY pass (passes_xy_tma.cuh) serves epilogues with a staged form
-// unless CLARITY_XY_TMA=0.
+// The staged XY passes (passes_xy_tma.cuh, passes_xy_rows.cuh) serve epilogues
+// with a staged form unless CLARITY_XY_TMA=0.
 bool xy_tma_enabled();
 template <class F>
 constexpr bool xy_staged() {
@@ -77,67 +73,94 @@ inline bool encode_s_map(TensorMap* tm, const float2* S) {
                                      (unsigned long long)SH::KG, (unsigned long long)SH::AY};
   const unsigned long long stride[3] = {row * 4, row * 4 * SH::NZ,
                                         row * 4 * SH::NZ * SH::KG};
-  const unsigned box[4] = {2u * X::BOXW, 1u, (unsigned)SH::KG, (unsigned)SH::AY};
+  const unsigned box[4] = {2u * X::BOXW, 1u, (unsigned)X::KGB, (unsigned)SH::AY};
   return encode_tensor_f32_4d(tm, S, dim, stride, box);
 }
 
-// Launches the TMA XY pass on tiles X when shape, epilogue and buffers allow it.
+// Launches the TMA XY pass on tiles X; false when its rows do not fit or the
+// buffer cannot be mapped.
 template <class SH, class X, bool FUSE, class F>
 inline bool try_xy_tma_tile(const PlanEntry& pe, cudaStream_t st, const F& fn, const float2* S,
                             int family, cudaError_t* err) {
-  if constexpr (X::OK && xy_staged<F>()) {
-    if (!xy_tma_enabled()) return false;
-    // the map depends only on S: encoded once per buffer
-    static thread_local const float2* map_s = nullptr;
-    static thread_local TensorMap tm;
-    if (S != map_s) {
-      if (!encode_s_map<SH, X>(&tm, S)) {
-        map_s = nullptr;
-        return false;
-      }
-      map_s = S;
+  static_assert(X::OK, "shape not supported by the TMA XY pass");
+  const int stride = X::stage_stride(fn.row_n());
+  if (X::blocks_per_sm(stride) < 1) return false;
+  // the map depends only on S: encoded once per buffer
+  static thread_local const float2* map_s = nullptr;
+  static thread_local TensorMap tm;
+  if (S != map_s) {
+    if (!encode_s_map<SH, X>(&tm, S)) {
+      map_s = nullptr;
+      return false;
     }
-    auto k = st::ks_xy_tma<SH, X, F, FUSE>;
-    const int stride = X::stage_stride(fn.row_n());
-    const int smem = X::smem(stride);
-    *err = allow_smem_st(k, X::SMEM);
-    if (*err != cudaSuccess) return true;
-    const st::Tables T = tables_of(pe);
-    const int blocks = launch_planes(fn, SH::NZ) * (SH::BY / X::TG);
-    if (blocks <= 0) return true;
-    note_launch_begin(family, st);
-    CLARITY_LAUNCH_PDL(k, blocks, X::THREADS, smem, st, pdl_enabled())(fn, tm, T, stride);
-    note_launch_end(family, st);
-    *err = cudaGetLastError();
-    return true;
-  } else {
-    (void)pe; (void)st; (void)fn; (void)S; (void)family; (void)err;
-    return false;
+    map_s = S;
   }
+  auto k = st::ks_xy_tma<SH, X, F, FUSE>;
+  const int smem = X::smem(stride);
+  *err = allow_smem_st(k, smem);
+  if (*err != cudaSuccess) return true;
+  const int blocks = launch_planes(fn, SH::NZ) * (SH::BY / X::TG);
+  if (blocks <= 0) return true;
+  note_launch_begin(family, st);
+  CLARITY_LAUNCH_PDL(k, blocks, X::THREADS, smem, st, pdl_enabled())(fn, tm, tables_of(pe), stride);
+  note_launch_end(family, st);
+  *err = cudaGetLastError();
+  return true;
 }
 
-// The tiles of the TMA XY pass.  Boxes whose spectrum rows hold two columns
-// (16 bytes a line) take two lines and twice the threads where the staged rows
-// leave room for two such blocks per SM; one line otherwise.  Where a line has
-// few columns a block has as many threads as it has column tasks: the rest
-// only waited at barriers.
+// Launches the pass of passes_xy_rows.cuh on tiles X; false when its rows do
+// not fit.
+template <class SH, class X, bool FUSE, class F>
+inline bool try_xy_rows_tile(const PlanEntry& pe, cudaStream_t st, const F& fn, float2* S,
+                             int family, cudaError_t* err) {
+  const int stride = X::stage_stride(fn.row_n());
+  if (!X::fits(stride)) return false;
+  auto k = st::ks_xy_rows<SH, X, F, FUSE>;
+  const int smem = X::smem(stride);
+  *err = allow_smem_st(k, smem);
+  if (*err != cudaSuccess) return true;
+  const int blocks = launch_planes(fn, SH::NZ) * (SH::BY / X::TG);
+  if (blocks <= 0) return true;
+  note_launch_begin(family, st);
+  CLARITY_LAUNCH_PDL(k, blocks, X::THREADS, smem, st, pdl_enabled())(fn, S, tables_of(pe), stride);
+  note_launch_end(family, st);
+  *err = cudaGetLastError();
+  return true;
+}
+
+// The tiles of the staged XY passes.
+//   * Rows of fewer than 256 complex: passes_xy_rows.cuh, 64 threads, keeping
+//     half the rows where no line has more than AY/2 live ones (the image is at
+//     most half the box).
+//   * Else the TMA pass.  Boxes whose spectrum rows hold two columns (16 bytes a
+//     line) take two lines and 512 threads where the staged rows leave room for
+//     two such blocks per SM (whole sectors: product pass 91 -> 87 us); one line
+//     otherwise.  The 1024x1024x256 box's two lines of 512 columns are one block
+//     of 1024 threads per SM (ratio pass 1122 -> 950 us); rows too long to stage
+//     beside them (a work-box volume's) keep the passes without staging.
 template <class SH, bool FUSE, class F>
-inline bool try_xy_tma(const PlanEntry& pe, cudaStream_t st, const F& fn, const float2* S,
-                       int family, cudaError_t* err) {
+inline bool try_xy_staged(const PlanEntry& pe, cudaStream_t st, const F& fn, float2* S, int family,
+                          cudaError_t* err) {
   if constexpr (xy_staged<F>()) {
-    constexpr int TG = SH::W % 2 == 0 ? 1 : 2;
-    constexpr int tasks = TG * SH::M;
-    constexpr int THR = tasks < 64 ? 64 : (tasks > 256 ? 256 : (tasks + 31) / 32 * 32);
-    if constexpr (SH::W == 2 && tasks == 256) {
+    if (!xy_tma_enabled()) return false;
+    if constexpr (SH::M < 256) {
+      constexpr int TG = SH::W >= 4 ? 1 : 2;
+      if constexpr (F::has_zero_rows)
+        if (fn.live_rows(0, SH::BY, SH::AY) <= SH::AY / 2)
+          return try_xy_rows_tile<SH, st::XyRows<SH, TG, 64, SH::AY / 2>, FUSE>(pe, st, fn, S,
+                                                                               family, err);
+      return try_xy_rows_tile<SH, st::XyRows<SH, TG, 64, SH::AY>, FUSE>(pe, st, fn, S, family, err);
+    } else if constexpr (SH::W == 2 && SH::M == 256) {
       using X2 = st::XyTma<SH, 2, 512>;
-      if (2 * (X2::smem(X2::stage_stride(fn.row_n())) + 4096) <= 228 * 1024 &&
+      if (X2::blocks_per_sm(X2::stage_stride(fn.row_n())) >= 2 &&
           try_xy_tma_tile<SH, X2, FUSE>(pe, st, fn, S, family, err))
         return true;
+      return try_xy_tma_tile<SH, st::XyTma<SH, 1, 256>, FUSE>(pe, st, fn, S, family, err);
+    } else if constexpr (SH::W == 1 && SH::M == 512) {
+      return try_xy_tma_tile<SH, st::XyTma<SH, 2, 1024>, FUSE>(pe, st, fn, S, family, err);
     }
-    return try_xy_tma_tile<SH, st::XyTma<SH, TG, THR>, FUSE>(pe, st, fn, S, family, err);
-  } else {
-    return false;
   }
+  return false;
 }
 
 // Kernel families that may use the specialised kernels: bit KIND of the
@@ -170,23 +193,34 @@ inline bool try_static(const PlanEntry& pe, cudaStream_t st, const F& fn, float2
                                                                                      Sa, T);
       note_launch_end(KK_Z, st);
     } else {
-      auto k = st::ks_z<st::ZThreads<SH>, F>;
-      int threads = SH::Z_THREADS;
+      using Z3 = st::Z3<st::ZThreads<SH>>;
+      static_assert(Z3::OK, "a box with BY > 32 needs the W = 1 z kernel");
+      int prec = st::kDftF32;
       if constexpr (st::kTcZ<SH> && !F::forward_only) {
         // the precision form: tensor-core first z stage (the OTF stays FP32)
-        const int prec = dft_precision();
-        if (prec == st::kDftF16Split) k = st::ks_z<SH, F, st::kDftF16Split>;
-        if (prec == st::kDftBF16Split) k = st::ks_z<SH, F, st::kDftBF16Split>;
-        if (prec != st::kDftF32) threads = SH::THREADS;
+        prec = dft_precision();
+        if (prec != st::kDftF32) {
+          auto k = prec == st::kDftF16Split ? st::ks_z<SH, F, st::kDftF16Split>
+                                            : st::ks_z<SH, F, st::kDftBF16Split>;
+          *err = allow_smem_st(k, SH::Z_SMEM);
+          if (*err != cudaSuccess) return true;
+          note_launch_begin(KK_Z, st);
+          CLARITY_LAUNCH(k, pe.P.z_blocks, SH::THREADS, SH::Z_SMEM, st)(fn, Sb, Sa, T);
+          note_launch_end(KK_Z, st);
+        }
       }
-      *err = allow_smem_st(k, SH::Z_SMEM);
-      if (*err != cudaSuccess) return true;
-      note_launch_begin(KK_Z, st);
-      CLARITY_LAUNCH(k, pe.P.z_blocks, threads, SH::Z_SMEM, st)(fn, Sb, Sa, T);
-      note_launch_end(KK_Z, st);
+      if (prec == st::kDftF32) {
+        auto k = st::ks_z3<st::ZThreads<SH>, F>;
+        *err = allow_smem_st(k, Z3::SMEM);
+        if (*err != cudaSuccess) return true;
+        note_launch_begin(KK_Z, st);
+        CLARITY_LAUNCH_PDL(k, pe.P.z_blocks, SH::Z_THREADS, Z3::SMEM, st, pdl_enabled())(fn, Sb, Sa,
+                                                                                      T);
+        note_launch_end(KK_Z, st);
+      }
     }
   } else if constexpr (KIND == 2) {
-    if (try_xy_tma<SH, true>(pe, st, fn, Sa, family_of<F, KK_XY_INV_FWD>(), err)) return true;
+    if (try_xy_staged<SH, true>(pe, st, fn, Sa, family_of<F, KK_XY_INV_FWD>(), err)) return true;
     auto k = st::ks_xy_inv_fwd<SH, F>;
     *err = allow_smem_st(k, SH::XY_SMEM);
     if (*err != cudaSuccess) return true;
@@ -195,7 +229,7 @@ inline bool try_static(const PlanEntry& pe, cudaStream_t st, const F& fn, float2
     (fn, Sa, T);
     note_launch_end(family_of<F, KK_XY_INV_FWD>(), st);
   } else {
-    if (try_xy_tma<SH, false>(pe, st, fn, Sb, KK_XY_INVERSE, err)) return true;
+    if (try_xy_staged<SH, false>(pe, st, fn, const_cast<float2*>(Sb), KK_XY_INVERSE, err)) return true;
     auto k = st::ks_xy_inverse<SH, F>;
     *err = allow_smem_st(k, SH::XY_SMEM);
     if (*err != cudaSuccess) return true;

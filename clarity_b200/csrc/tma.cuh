@@ -209,6 +209,15 @@ __device__ __forceinline__ float ld_l2(const float* p) {
   return *p;
 #endif
 }
+__device__ __forceinline__ float2 ld_l2(const float2* p) {
+#ifndef CLARITY_HOST_EMULATION
+  float2 v;
+  asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+#else
+  return *p;
+#endif
+}
 __device__ __forceinline__ float4 ld_l2(const float4* p) {
 #ifndef CLARITY_HOST_EMULATION
   float4 v;

@@ -475,3 +475,46 @@ def test_correlation_opt_ins_vs_oracle(clarity_gpu, oracle_lib, case):
     assert rel_l2(out.cpu().numpy(), oracle_lib.rl_correlate(img, psf, 4)) <= TOL_ITER
     plain = clarity_gpu.maximum_likelihood_deconvolve(img, psf, 4)
     assert rel_l2(plain, oracle_lib.rl(img, psf, 4)) <= TOL_ITER
+
+
+@pytest.mark.parametrize("image_zyx,psf_zyx", [
+    ((101, 333, 517), (155, 691, 507)),   # 1024x1024x256 box: rows that are no 16-byte runs
+    ((128, 512, 300), (128, 512, 724)),   # the same with whole tiles
+    ((50, 417, 301), (78, 95, 211)),      # 512x512x128: more than half of a line's rows live
+    ((64, 100, 256), (64, 412, 256)),     # 512x512x128: few live rows
+])
+def test_specialised_boxes_with_uneven_splits(clarity_gpu, image_zyx, psf_zyx):
+    # the compile-time boxes reached from other extents than half and half,
+    # against the padded circular convolution in FP64 (plain torch)
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(sum(image_zyx))
+    img = torch.rand(image_zyx, generator=gen, device="cuda") * 100 + 1
+    psf = torch.from_numpy(syn.gaussian_psf(psf_zyx, 2.0, 3.0).astype(np.float32)).cuda()
+    box = tuple(a + b for a, b in zip(image_zyx, psf_zyx))
+
+    def pad(a):
+        p = torch.zeros(box, dtype=torch.float64, device="cuda")
+        p[tuple(slice(0, n) for n in a.shape)] = a.double()
+        return p
+
+    otf = torch.fft.rfftn(torch.roll(pad(psf), tuple(-(k // 2) for k in psf_zyx), (0, 1, 2)))
+    blur = lambda u: torch.fft.irfftn(torch.fft.rfftn(u) * otf, s=box)  # noqa: E731
+    inside = tuple(slice(0, n) for n in image_zyx)
+    g = pad(img)
+    out = torch.empty_like(img)
+    clarity_gpu.convolve_device(img, psf, out)
+    want = blur(g)[inside]
+    assert ((out.double() - want).norm() / want.norm()).item() <= 1e-6
+    u = g
+    for _ in range(2):
+        b = blur(u)
+        v = u * blur(torch.where(b.abs() < 1e-5, torch.zeros_like(b), g / b))
+        u = v * (g.sum() / v.sum())
+    clarity_gpu.ml_device(img, psf, out, 2)
+    want = u[inside]
+    assert ((out.double() - want).norm() / want.norm()).item() <= 2e-6
+    A = 0.5 * g.max()
+    o = blur(g)
+    want = (g + (1 - (o - A) ** 2 / A ** 2) * (g - o)).clamp_min(0)[inside]
+    clarity_gpu.jvc_device(img, psf, out, 1)
+    assert ((out.double() - want).norm() / want.norm()).item() <= 2e-6
