@@ -374,9 +374,22 @@ def _stream_ptr(stream):
     return C.c_void_p(stream.cuda_stream)
 
 
+_torch = None
+
+
+def _is_f32_cuda(t) -> bool:
+    """Contiguous float32 CUDA tensor (the dtype by identity: formatting it
+    costs more than the rest of the check)."""
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    return t.is_cuda and t.is_contiguous() and t.dtype is _torch.float32
+
+
 def _dev(name, image, kernel, out, extra, stream):
     for t in (image, kernel, out):
-        if not (t.is_cuda and t.is_contiguous() and str(t.dtype) == "torch.float32"):
+        if not _is_f32_cuda(t):
             raise ValueError("device variants need contiguous float32 CUDA tensors")
     _check(getattr(load(), name)(C.c_void_p(image.data_ptr()), dim3(image),
                                  C.c_void_p(kernel.data_ptr()), dim3(kernel),
@@ -435,7 +448,7 @@ def ml_batch_device(images, kernels, outs, iterations, graph=True, stream=None,
     if len(kernels) != n or len(outs) != n:
         raise ValueError("images, kernels and outs must have the same length")
     for t in list(images) + list(kernels) + list(outs):
-        if not (t.is_cuda and t.is_contiguous() and str(t.dtype) == "torch.float32"):
+        if not _is_f32_cuda(t):
             raise ValueError("batch volumes must be contiguous float32 CUDA tensors")
     vp = C.c_void_p
     imgs = (vp * n)(*[t.data_ptr() for t in images])
@@ -471,7 +484,7 @@ def ml_ex_device(image, kernel, out, iterations, start=None, idiv=None, stream=N
     device tensor of `iterations` + 1 entries: the estimate at the start of each
     iteration, then the result)."""
     for t in (image, kernel, out) + ((start,) if start is not None else ()):
-        if not (t.is_cuda and t.is_contiguous() and str(t.dtype) == "torch.float32"):
+        if not _is_f32_cuda(t):
             raise ValueError("device variants need contiguous float32 CUDA tensors")
     if start is not None and tuple(start.shape) != tuple(image.shape):
         raise ValueError("start must have the image's shape")
@@ -494,7 +507,7 @@ def ml_accel_device(image, kernel, out, iterations, idiv=None, stream=None, star
     if start is not None and tuple(start.shape) != tuple(image.shape):
         raise ValueError("start must have the image's shape")
     for t in (image, kernel, out) + ((start,) if start is not None else ()):
-        if not (t.is_cuda and t.is_contiguous() and str(t.dtype) == "torch.float32"):
+        if not _is_f32_cuda(t):
             raise ValueError("device variants need contiguous float32 CUDA tensors")
     if idiv is not None and not (idiv.is_cuda and str(idiv.dtype) == "torch.float64"
                                  and idiv.numel() >= max(int(iterations), 0) + 1):
@@ -514,7 +527,7 @@ def ml_learned_device(image, kernel, params, out, pre, post, idiv=None, stream=N
     resumed for `post` iterations (optional float64 trace of post + 1
     entries)."""
     for t in (image, kernel, out, params):
-        if not (t.is_cuda and t.is_contiguous() and str(t.dtype) == "torch.float32"):
+        if not _is_f32_cuda(t):
             raise ValueError("device variants need contiguous float32 CUDA tensors")
     if idiv is not None and not (idiv.is_cuda and str(idiv.dtype) == "torch.float64"
                                  and idiv.numel() >= max(int(post), 0) + 1):
@@ -532,7 +545,7 @@ def nn_predict(params, x, out, stream=None):
     from the volume x (domain transforms fused into its first and last
     kernels)."""
     for t in (params, x, out):
-        if not (t.is_cuda and t.is_contiguous() and str(t.dtype) == "torch.float32"):
+        if not _is_f32_cuda(t):
             raise ValueError("nn_predict needs contiguous float32 CUDA tensors")
     vp = C.c_void_p
     _check(load().clarityx_nn_predict(vp(params.data_ptr()), params.numel(), vp(x.data_ptr()),
@@ -567,7 +580,7 @@ def blind_ml_psf_device(image, kernel, out, iterations, psf_subiterations=5, psf
     `psf_subiterations` PSF steps per iteration; psf_out (kernel-shaped) gets
     the PSF estimate."""
     for t in (image, kernel, out) + ((psf_out,) if psf_out is not None else ()):
-        if not (t.is_cuda and t.is_contiguous() and str(t.dtype) == "torch.float32"):
+        if not _is_f32_cuda(t):
             raise ValueError("device variants need contiguous float32 CUDA tensors")
     vp = C.c_void_p
     _check(load().clarityx_blind_ml_psf_device(

@@ -14,6 +14,7 @@
 #include <cstring>
 #include <algorithm>
 #include <mutex>
+#include <thread>
 #include <vector>
 #include <string>
 
@@ -45,15 +46,20 @@ struct Staging {
 
 // Library-owned pinned bounce buffers for callers whose host buffers are
 // pageable (every reference caller allocates with malloc or new,
-// src/Memory.cxx:97-156 copies from them synchronously).  A copy is cut
-// into chunks that alternate between two pinned buffers: the host copies
-// chunk k into one while the DMA engine moves chunk k-1 out of the other.
-// Buffers the caller pinned itself (cudaHostAlloc, cudaHostRegister) are
-// copied directly.
+// src/Memory.cxx:97-156 copies from them synchronously).  A copy is cut into
+// chunks that alternate between two pinned slots: the host copies chunk k into
+// one while the DMA engine moves chunk k-1 out of the other.  One thread copies
+// at some 8 GB/s, and a result's fresh pages fault in as it is written, so a
+// large copy is cut into slices for several threads with two slots each; they
+// live for the copy only.  Buffers the caller pinned itself (cudaHostAlloc,
+// cudaHostRegister) are copied directly.
 struct PinnedBounce {
-  static constexpr size_t kChunk = size_t(8) << 20;
-  void* buf[2] = {nullptr, nullptr};
-  cudaEvent_t ev[2] = {nullptr, nullptr};
+  static constexpr size_t kSlot = size_t(1) << 20;
+  static constexpr int kMaxThreads = 8;
+  static constexpr int kSlots = 2 * kMaxThreads;
+  static constexpr size_t kSlice = size_t(2) << 20;  // at least this much per thread
+  char* buf = nullptr;                               // kSlots slots
+  cudaEvent_t ev[kSlots] = {};
 } g_bounce;
 
 bool host_is_pinned(const void* p) {
@@ -66,25 +72,101 @@ bool host_is_pinned(const void* p) {
 }
 
 cudaError_t bounce_ready() {
-  for (int i = 0; i < 2; ++i) {
-    if (!g_bounce.buf[i]) {
-      cudaError_t e = cudaHostAlloc(&g_bounce.buf[i], PinnedBounce::kChunk, cudaHostAllocPortable);
-      if (e != cudaSuccess) return e;
-    }
-    if (!g_bounce.ev[i]) {
-      cudaError_t e = cudaEventCreateWithFlags(&g_bounce.ev[i], cudaEventDisableTiming);
-      if (e != cudaSuccess) return e;
-    }
+  if (!g_bounce.buf) {
+    void* b = nullptr;
+    const cudaError_t e = cudaHostAlloc(&b, PinnedBounce::kSlots * PinnedBounce::kSlot,
+                                        cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+    g_bounce.buf = static_cast<char*>(b);
   }
+  for (cudaEvent_t& ev : g_bounce.ev)
+    if (!ev) {
+      const cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+      if (e != cudaSuccess) return e;
+    }
   return cudaSuccess;
 }
 
 void free_bounce() {
-  for (int i = 0; i < 2; ++i) {
-    if (g_bounce.buf[i]) cudaFreeHost(g_bounce.buf[i]);
-    if (g_bounce.ev[i]) cudaEventDestroy(g_bounce.ev[i]);
-  }
+  if (g_bounce.buf) cudaFreeHost(g_bounce.buf);
+  for (cudaEvent_t ev : g_bounce.ev)
+    if (ev) cudaEventDestroy(ev);
   g_bounce = PinnedBounce();
+}
+
+// One thread's slice host -> device through its slots (2*t, 2*t + 1).
+cudaError_t upload_slice(char* d, const char* s, size_t bytes, int t, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  for (size_t off = 0, k = 0; off < bytes && e == cudaSuccess; off += PinnedBounce::kSlot, ++k) {
+    const int i = 2 * t + (int)(k & 1);
+    char* slot = g_bounce.buf + (size_t)i * PinnedBounce::kSlot;
+    const size_t n = std::min(PinnedBounce::kSlot, bytes - off);
+    if ((e = cudaEventSynchronize(g_bounce.ev[i])) != cudaSuccess) break;  // slot free
+    std::memcpy(slot, s + off, n);
+    e = cudaMemcpyAsync(d + off, slot, n, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaEventRecord(g_bounce.ev[i], st);
+  }
+  return e;
+}
+
+// One thread's slice device -> host; written completely when it returns.
+cudaError_t download_slice(char* d, const char* s, size_t bytes, int t, cudaStream_t st) {
+  const size_t nch = (bytes + PinnedBounce::kSlot - 1) / PinnedBounce::kSlot;
+  auto issue = [&](size_t k) -> cudaError_t {
+    const int i = 2 * t + (int)(k & 1);
+    const size_t off = k * PinnedBounce::kSlot, n = std::min(PinnedBounce::kSlot, bytes - off);
+    cudaError_t r = cudaEventSynchronize(g_bounce.ev[i]);
+    if (r == cudaSuccess)
+      r = cudaMemcpyAsync(g_bounce.buf + (size_t)i * PinnedBounce::kSlot, s + off, n,
+                          cudaMemcpyDeviceToHost, st);
+    if (r == cudaSuccess) r = cudaEventRecord(g_bounce.ev[i], st);
+    return r;
+  };
+  cudaError_t e = issue(0);
+  for (size_t k = 0; k < nch && e == cudaSuccess; ++k) {
+    if (k + 1 < nch && (e = issue(k + 1)) != cudaSuccess) break;
+    const int i = 2 * t + (int)(k & 1);
+    const size_t off = k * PinnedBounce::kSlot, n = std::min(PinnedBounce::kSlot, bytes - off);
+    if ((e = cudaEventSynchronize(g_bounce.ev[i])) != cudaSuccess) break;
+    std::memcpy(d + off, g_bounce.buf + (size_t)i * PinnedBounce::kSlot, n);
+  }
+  return e;
+}
+
+// Runs slice(offset, bytes, thread) over [0, bytes), on this thread and, for
+// large copies, a few more.  A thread that cannot be started leaves its slice
+// to this one.
+template <class F>
+cudaError_t in_slices(size_t bytes, const F& slice) {
+  const unsigned hw = std::thread::hardware_concurrency();
+  const size_t most = std::min<size_t>(PinnedBounce::kMaxThreads, hw > 2 ? hw / 2 : 1);
+  const int n = (int)std::max<size_t>(1, std::min(most, bytes / PinnedBounce::kSlice));
+  const size_t part = (bytes / n + 4095) / 4096 * 4096;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaError_t err[PinnedBounce::kMaxThreads] = {};
+  auto run = [&](int t) {
+    const size_t off = std::min(bytes, part * t), end = t + 1 == n ? bytes : std::min(bytes, off + part);
+    if (end > off) err[t] = slice(off, end - off, t);
+  };
+  std::thread th[PinnedBounce::kMaxThreads];
+  for (int t = 1; t < n; ++t) {
+    try {
+      th[t] = std::thread([&, t] {
+        cudaSetDevice(dev);
+        run(t);
+      });
+    } catch (...) {
+    }
+  }
+  run(0);
+  for (int t = 1; t < n; ++t) {
+    if (th[t].joinable()) th[t].join();
+    else run(t);
+  }
+  for (int t = 0; t < n; ++t)
+    if (err[t] != cudaSuccess) return err[t];
+  return cudaSuccess;
 }
 
 // host -> device on `st`, asynchronous for pinned sources; a pageable source
@@ -92,21 +174,12 @@ void free_bounce() {
 cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   if (bytes == 0) return cudaSuccess;
   if (host_is_pinned(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-  cudaError_t e = bounce_ready();
+  const cudaError_t e = bounce_ready();
   if (e != cudaSuccess) return e;
-  const char* s = static_cast<const char*>(src);
-  char* d = static_cast<char*>(dst);
-  for (size_t off = 0, k = 0; off < bytes; off += PinnedBounce::kChunk, ++k) {
-    const int i = (int)(k & 1);
-    const size_t n = std::min(PinnedBounce::kChunk, bytes - off);
-    if ((e = cudaEventSynchronize(g_bounce.ev[i])) != cudaSuccess) return e;  // buffer free
-    std::memcpy(g_bounce.buf[i], s + off, n);
-    if ((e = cudaMemcpyAsync(d + off, g_bounce.buf[i], n, cudaMemcpyHostToDevice, st)) !=
-        cudaSuccess)
-      return e;
-    if ((e = cudaEventRecord(g_bounce.ev[i], st)) != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  return in_slices(bytes, [&](size_t off, size_t n, int t) {
+    return upload_slice(static_cast<char*>(dst) + off, static_cast<const char*>(src) + off, n, t,
+                        st);
+  });
 }
 
 // device -> host on `st`; complete (the host buffer written) when it returns
@@ -116,27 +189,13 @@ cudaError_t download(void* dst, const void* src, size_t bytes, cudaStream_t st) 
   if (host_is_pinned(dst)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
   cudaError_t e = bounce_ready();
   if (e != cudaSuccess) return e;
-  const char* s = static_cast<const char*>(src);
-  char* d = static_cast<char*>(dst);
-  const size_t nch = (bytes + PinnedBounce::kChunk - 1) / PinnedBounce::kChunk;
-  auto issue = [&](size_t k) -> cudaError_t {
-    const int i = (int)(k & 1);
-    const size_t off = k * PinnedBounce::kChunk, n = std::min(PinnedBounce::kChunk, bytes - off);
-    cudaError_t r = cudaEventSynchronize(g_bounce.ev[i]);
-    if (r == cudaSuccess) r = cudaMemcpyAsync(g_bounce.buf[i], s + off, n,
-                                              cudaMemcpyDeviceToHost, st);
-    if (r == cudaSuccess) r = cudaEventRecord(g_bounce.ev[i], st);
-    return r;
-  };
-  if ((e = issue(0)) != cudaSuccess) return e;
-  for (size_t k = 0; k < nch; ++k) {
-    if (k + 1 < nch && (e = issue(k + 1)) != cudaSuccess) return e;
-    const int i = (int)(k & 1);
-    const size_t off = k * PinnedBounce::kChunk, n = std::min(PinnedBounce::kChunk, bytes - off);
-    if ((e = cudaEventSynchronize(g_bounce.ev[i])) != cudaSuccess) return e;
-    std::memcpy(d + off, g_bounce.buf[i], n);
-  }
-  return cudaSuccess;
+  // the threads wait for their copies on the host: better one wait for the
+  // solve here than all of them spinning through it
+  if (bytes >= 2 * PinnedBounce::kSlice && (e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+  return in_slices(bytes, [&](size_t off, size_t n, int t) {
+    return download_slice(static_cast<char*>(dst) + off, static_cast<const char*>(src) + off, n, t,
+                          st);
+  });
 }
 
 bool g_implicit = false;         // the context was created by a call, not by Register
