@@ -599,6 +599,7 @@ Status Context::build_entry(const VolPlan& P0, bool pair, std::unique_ptr<PlanEn
     pair_tables(pe->pair, &slots, &tabs);
     CL_TRY(upload_tables(slots, tabs, pe->pair.twiddle_count, st, &pe->pair_tw, &pe->pair_slots));
   }
+  pe->z_folds = pe->pair.ok || (static_family_mask() == 0xF && static_z_folds(P0));
   *out = std::move(pe);
   return Status::Ok();
 }
@@ -1067,12 +1068,28 @@ static Status rl_core(Context& ctx, const PlanEntry& pe, Workspace& ws,
     }
   }
   CL_TRY(xy_forward(ctx, pe, ProImage{u0, P.xmode}, ws.S));
+  // The flux rescale s = E / sum u' is a launch of its own between P5 and the
+  // next P2 -- or P2's blocks each add the partials up themselves, where that
+  // is little work: RL on 64x64x32 (70 thousand additions over all blocks) went
+  // from 26.4 to 25.2 us an iteration, a 171x147x49 box (228 thousand) from 81.1
+  // to 82.4.
+  const long long parts = (long long)sd.z * (pe.pair.ok ? pe.pair.By / pe.pair.TG : P.By);
+  const long long zb = pe.pair.ok ? pe.pair.z_blocks : P.z_blocks;
+  const bool fold = rescale && pe.z_folds && parts * zb <= (1ll << 17);
   for (int k = 0; k < iters; ++k) {
     const float* sk = (k == 0 || !rescale) ? nullptr : sdev;
     // the estimate is zero in planes z >= its extent, and P3 reads only planes
     // z < Z (the image is zero beyond): no other plane is read, or
     // inverse-transformed along y0, or stored
-    CL_TRY(z_pass(ctx, pe, otf_between(H, scale_n, sd.z, id.z, sk), ws.S, ws.S));
+    ModOTF m2 = otf_between(H, scale_n, sd.z, id.z, sk);
+    if (fold && k > 0) {
+      m2.partial = ws.partial;
+      m2.np = ws.iscal;
+      m2.energy = ws.dscal + 0;
+      m2.sum_out = ws.dscal + 1;
+      m2.scale_out = sdev;
+    }
+    CL_TRY(z_pass(ctx, pe, m2, ws.S, ws.S));
     MidRLRatio ratio{g, P.xmode};
     if (idiv) {
       ratio.idiv_partial = ws.partial;
@@ -1104,7 +1121,7 @@ static Status rl_core(Context& ctx, const PlanEntry& pe, Workspace& ws,
       CL_TRY(xy_inv_fwd(ctx, pe, epi, ws.S));
     else
       CL_TRY(xy_inverse(ctx, pe, epi, ws.S));
-    if (rescale) {
+    if (rescale && (!fold || k + 1 == iters)) {
       // s = E / sum u' by one block in a fixed order.  A last-block ticket
       // in the product pass itself cost more: each of its blocks then waited
       // for an atomic's round trip before it could exit.

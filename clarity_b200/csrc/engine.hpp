@@ -44,6 +44,8 @@ struct PlanEntry {
   PairPlan pair = {};
   float2* pair_tw = nullptr;
   int* pair_slots = nullptr;
+  // The box's z kernel can fold the flux rescale in (ModOTF::late).
+  bool z_folds = false;
   // The same box on the passes of P (the persistent batched launch, whose
   // tiles run those bodies).
   PlanEntry classic() const {
@@ -57,6 +59,8 @@ struct PlanEntry {
 };
 // Whether compile-time kernels exist for the plan's box (kern_static_z.cu).
 bool has_static_shape(const VolPlan& P);
+// ... and whether its z kernel can fold the flux rescale in (ModOTF::late).
+bool static_z_folds(const VolPlan& P);
 
 
 // Device allocation that honours the host-side fault injector.

@@ -10,6 +10,9 @@ static bool any_shape(ShapeList<SHs...>, const VolPlan& P) {
   return (st::matches<SHs>(P) || ...);
 }
 bool has_static_shape(const VolPlan& P) { return any_shape(StaticShapes{}, P); }
+bool static_z_folds(const VolPlan& P) {
+  return has_static_shape(P) && st::fold_small(P.nz, P.By);
+}
 template bool static_z<ModOTF>(const PlanEntry&, cudaStream_t, const ModOTF&, const float2*, float2*, cudaError_t*);
 template bool static_z<ModWiener>(const PlanEntry&, cudaStream_t, const ModWiener&, const float2*, float2*, cudaError_t*);
 template bool static_z<ModForward>(const PlanEntry&, cudaStream_t, const ModForward&, const float2*, float2*, cudaError_t*);

@@ -330,6 +330,7 @@ struct EpiWork {
     float* o = nullptr;
   };
   __device__ __forceinline__ Row row(int y, int z) const { return Row{out + w.idx(0, y, z)}; }
+  __host__ __device__ __forceinline__ int row_n() const { return w.nx; }
   struct Pre {};
   __device__ __forceinline__ Pre pre(const Row&, int) const { return Pre{}; }
   __device__ __forceinline__ float put(const Row& r, int x, float v, Pre) {
@@ -377,6 +378,7 @@ struct EpiClip {
     if (y >= Y || z >= Z) return Row{};
     return Row{out + ((long long)z * Y + y) * X, scale ? ld_l2(scale) : 1.f};
   }
+  __host__ __device__ __forceinline__ int row_n() const { return X; }
   struct Pre {};
   __device__ __forceinline__ Pre pre(const Row&, int) const { return Pre{}; }
   __device__ __forceinline__ float put(const Row& r, int x, float v, Pre) {
@@ -705,6 +707,15 @@ struct ModOTF {
   const float2* CLARITY_RESTRICT H;
   float scale;
   const float* CLARITY_RESTRICT scale2 = nullptr;
+  // The flux rescale folded in (partial != nullptr; kernels that call late()):
+  // every block forms s = energy / sum of the *np partials itself and uses it
+  // in place of *scale2; block 0 stores it to scale_out and the sum to sum_out
+  // for the passes that follow.
+  const double* CLARITY_RESTRICT partial = nullptr;
+  const int* CLARITY_RESTRICT np = nullptr;
+  const double* CLARITY_RESTRICT energy = nullptr;
+  double* CLARITY_RESTRICT sum_out = nullptr;
+  float* CLARITY_RESTRICT scale_out = nullptr;
   // only the z planes z < zn and z >= zh of the input spectrum are nonzero
   // (the rest were never written and are read as zeros); no plane lies at or
   // beyond the default zh
@@ -730,6 +741,24 @@ struct ModOTF {
     const float2 hr = make_float2(h.x, h.y), hi = make_float2(h.z, h.w), f = both(scale);
     return c2{pmul(f, psub(pmul(v.re, hr), pmul(v.im, hi))),
               pmul(f, pfma(v.im, hr, pmul(v.re, hi)))};
+  }
+  // Called by every thread of a block before resolved(), with a barrier inside.
+  __device__ __forceinline__ void late() {
+    if (!partial) return;  // the same for every thread
+    __shared__ float s_late;
+    const double t = block_total(partial, *np);
+    if (threadIdx.x == 0) {
+      const float s = (float)energy[0] / (float)t;
+      s_late = s;
+      if (CLARITY_BLOCK_ID() == 0) {
+        *sum_out = t;
+        *scale_out = s;
+      }
+    }
+    __syncthreads();
+    scale *= s_late;
+    scale2 = nullptr;
+    partial = nullptr;
   }
   // the same operation with the deferred factor read once (per thread)
   __device__ __forceinline__ ModOTF resolved() const {
@@ -772,6 +801,7 @@ struct ModWiener {
     const float2 y = apply_h(make_float2(h.y, h.w), make_float2(v.re.y, v.im.y));
     return c2{make_float2(x.x, y.x), make_float2(x.y, y.y)};
   }
+  __device__ __forceinline__ void late() {}
   __device__ __forceinline__ ModWiener resolved() const { return *this; }
 };
 
@@ -782,6 +812,7 @@ struct ModForward {
   int zout = 1 << 30;
   __device__ __forceinline__ void prefetch_tile(unsigned, int, int, int) const {}
   __device__ __forceinline__ float2 apply(long long, float2 v) const { return v; }
+  __device__ __forceinline__ void late() {}
   __device__ __forceinline__ ModForward resolved() const { return *this; }
 };
 

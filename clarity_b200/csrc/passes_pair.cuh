@@ -176,7 +176,7 @@ __device__ __forceinline__ void z_mod(float4* sm, const PairPlan& P, const Mod& 
 // memory (dead planes zeroed there).
 template <class Mod, bool BIG>
 __global__ void __launch_bounds__(Cls<BIG>::MAXT, 2)
-    kp_z(CLARITY_GRID_CONST PairPlan P, const ZSpan Z, const Mod mod, const float2* Sin_,
+    kp_z(CLARITY_GRID_CONST PairPlan P, const ZSpan Z, Mod mod, const float2* Sin_,
          float2* Sout_, const float2* CLARITY_RESTRICT tables) {
   CLARITY_DYN_SMEM(float4, sm);
   constexpr int MAXR = Cls<BIG>::MAXR;
@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(Cls<BIG>::MAXT, 2)
     const int z = quot(f, P.dBy);
     sm[f + z * (P.BS - P.By)] = z < Z.zn || z >= Z.zn + Z.gap ? ld_l2(&Sin[f]) : zero4();
   }
+  mod.late();
   __syncthreads();
   const int nlive = P.nz - Z.gap;
   for (int s = 0; s < P.ayB.npass; ++s) {
@@ -314,7 +315,7 @@ __device__ __forceinline__ void x_first(const XyCtx& C, const PairPlan& P, const
 template <int R, class Epi, bool FUSE>
 __device__ __forceinline__ void x_last(const XyCtx& C, const PairPlan& P, Epi& epi) {
   const int span = P.ax.span[0], ps = P.ax.pspan[0];
-  const int total = P.TG * C.nql * span;
+  const int total = P.TG * C.nql * span, xn = epi.row_n();
   const FDiv Ds = P.ax.dspan[0];
   for (int f = threadIdx.x; f < total; f += blockDim.x) {
     const int r = quot(f, Ds), i = f - r * span;
@@ -329,7 +330,7 @@ __device__ __forceinline__ void x_last(const XyCtx& C, const PairPlan& P, Epi& e
 #pragma unroll
       for (int t = 0; t < CH; ++t) {
         const int x = i + (t0 + t) * span;
-        if (t0 + t < R) {
+        if (t0 + t < R && (t0 + t) * span < xn) {
           a[t] = epi.pre(w.a, x);
           b[t] = epi.pre(w.b, x);
           c[t] = epi.pre(w.c, x);
@@ -349,7 +350,9 @@ __device__ __forceinline__ void x_last(const XyCtx& C, const PairPlan& P, Epi& e
 #pragma unroll
       for (int u = 0; u < CH; ++u) {
         const int t = t0 + u, x = i + t * span;
-        if (t < R) {
+        if (t < R && t * span >= xn) {
+          v[t] = get(zero4());  // beyond the longest row, for every thread alike
+        } else if (t < R) {
           v[t].re.x = epi.put(w.a, x, v[t].re.x, a[u]);
           v[t].im.x = epi.put(w.b, x, v[t].im.x, b[u]);
           v[t].re.y = epi.put(w.c, x, v[t].re.y, c[u]);

@@ -38,6 +38,8 @@ constexpr int ctz_c(int v) {
   return c;
 }
 
+constexpr bool fold_small(int nz, int by) { return by <= 32 && nz * by <= 1024; }
+
 // Even nx only (half-length complex rows).  T_ threads per block: 256 where
 // several blocks fit an SM; the boxes whose XY and z tiles take most of an
 // SM's shared memory (one block per SM) use more threads, so the SM still
@@ -71,6 +73,8 @@ struct Shape {
   static constexpr int XY_SMEM = G * GSTRIDE * 8;
   static constexpr int Z_SMEM = TILE * 8;
   static constexpr int NGROUPS = BY / G;
+  // boxes small enough for ks_z2's blocks to add up the flux partials themselves
+  static constexpr bool Z_FOLDS = fold_small(NZ, BY);
   // Z kernel with one register pass per y0 line (BY <= 32): padded z stride
   // ZS = BW + W keeps both the per-line y0 accesses and the z passes free of
   // bank conflicts.
@@ -831,7 +835,7 @@ __device__ __forceinline__ void z2_spectral(float2* sm, const Mod& mod, unsigned
 
 template <class SH, class Mod>
 __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
-    ks_z2(const Mod mod, const float2* __restrict__ Sin, float2* __restrict__ Sout,
+    ks_z2(Mod mod, const float2* __restrict__ Sin, float2* __restrict__ Sout,
           const Tables T) {
   CLARITY_DYN_SMEM(float2, sm);
   static_assert(SH::Y_PER_LINE, "y0 per-line Z kernel needs BY <= 32");
@@ -866,9 +870,11 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
       cp_async16(sm + z * ZS + c, Sin + gbase + z * BW + c);
     }
     if (threadIdx.x < 4) mod.prefetch_tile(gbase, SH::TILE, threadIdx.x, 4);
+    if constexpr (SH::Z_FOLDS) mod.late();
     cp_async_wait_all();
   } else {
     if (threadIdx.x < 4) mod.prefetch_tile(gbase, SH::TILE, threadIdx.x, 4);
+    if constexpr (SH::Z_FOLDS) mod.late();
   }
   __syncthreads();
   // y0 forward, one line (z, ki) per thread
