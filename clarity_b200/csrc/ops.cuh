@@ -470,7 +470,8 @@ struct EpiRLProduct {
     if (y < Y && z < Z) return {cur + at(0, y, z), X};
     return {nullptr, 0};
   }
-  __host__ __device__ __forceinline__ int row_n() const { return X; }  // floats of a staged row
+  __host__ __device__ __forceinline__ int row_n() const { return X; }
+  __host__ __device__ __forceinline__ int stage_n() const { return X; }  // floats of a staged row
   float s_ = 1.f;  // the deferred scale, read once the previous pass is done
   __device__ __forceinline__ void prepare() {
     if (scale) s_ = ld_l2(scale);
@@ -580,6 +581,7 @@ struct MidRLRatio {
     return {nullptr, 0};
   }
   __host__ __device__ __forceinline__ int row_n() const { return g.X; }
+  __host__ __device__ __forceinline__ int stage_n() const { return g.X; }
   __device__ __forceinline__ float2 apply_s(int m, int, int, float2 b, const float* sr, int n) {
     const int x = 2 * m;
     const float a0 = x < n ? sr[x] : 0.f, a1 = x + 1 < n ? sr[x + 1] : 0.f;
@@ -670,27 +672,31 @@ struct EpiJVC {
     if (y < g.Y && z < g.Z)
       prefetch_l2_range(g.src + ((unsigned)z * g.Y + y) * g.X, sizeof(float) * (size_t)g.X);
   }
-  // Staged form: the estimate's row (the image's on the first update) arrives
-  // in shared memory.  The image is read in place: an eighth of the work box has it.  At
-  // the 512x512x128 box the pass went from 292 to 184 us.
-  __device__ __forceinline__ void prefetch_image(int y, int z) const {
-    if (cur && y < g.Y && z < g.Z)
-      prefetch_l2_range(g.src + ((unsigned)z * g.Y + y) * g.X, sizeof(float) * (size_t)g.X);
-  }
+  // Staged pass, reading both volumes in place: with a work-box row staged beside
+  // each tile row only one-line tiles fit (512x512x128 box: 187 us staged, 172 in
+  // place in two-line tiles; 292 before either).
   static constexpr bool kStaged = true;
-  __device__ __forceinline__ st::RowRef in_row(int y, int z) const {
-    if (cur) return {cur + w.idx(0, y, z), w.nx};
-    if (y < g.Y && z < g.Z) return {g.src + ((unsigned)z * g.Y + y) * g.X, g.X};
-    return {nullptr, 0};
-  }
+  __device__ __forceinline__ void prefetch_image(int y, int z) const { prefetch_row(y, z); }
+  __device__ __forceinline__ st::RowRef in_row(int, int) const { return {nullptr, 0}; }
   __host__ __device__ __forceinline__ int row_n() const { return w.nx; }
-  __device__ __forceinline__ float2 apply_s(int m, int y, int z, float2 o, const float* sr, int n) {
+  __host__ __device__ __forceinline__ int stage_n() const { return 0; }
+  struct InPlace {
+    float2 i, g;
+  };
+  __device__ __forceinline__ InPlace read(int m, int y, int z) const {
     const int x = 2 * m;
-    const float i0 = x < n ? sr[x] : 0.f, i1 = x + 1 < n ? sr[x + 1] : 0.f;
-    const float g0 = cur ? g.at(x, y, z) : i0, g1 = cur ? g.at(x + 1, y, z) : i1;
-    const float2 r = make_float2(upd(i0, g0, o.x), upd(i1, g1, o.y));
-    store2(inext + w.idx(x, y, z), r.x, r.y);
+    InPlace q;
+    q.g = make_float2(g.at(x, y, z), g.at(x + 1, y, z));
+    q.i = cur ? ld_l2(reinterpret_cast<const float2*>(cur + w.idx(x, y, z))) : q.g;
+    return q;
+  }
+  __device__ __forceinline__ float2 apply_q(int m, int y, int z, float2 o, const InPlace& q) {
+    const float2 r = make_float2(upd(q.i.x, q.g.x, o.x), upd(q.i.y, q.g.y, o.y));
+    *reinterpret_cast<float2*>(inext + w.idx(2 * m, y, z)) = r;
     return r;
+  }
+  __device__ __forceinline__ float2 apply_s(int m, int y, int z, float2 o, const float*, int) {
+    return apply_q(m, y, z, o, read(m, y, z));
   }
   __device__ __forceinline__ void finish() {}
 };

@@ -334,6 +334,19 @@ __device__ __forceinline__ void x_last_staged(float2* sm, const float* stg, Epi&
     dft<R, +1>(v);
     const float* srow = stg + r * SS;
     const int n = epi.in_row(y, z).nf;
+    if constexpr (requires { typename Epi::InPlace; }) {
+      // the epilogue reads its volumes in place: four elements' loads at a time
+      constexpr int CH = R % 4 == 0 ? 4 : 1;
+#pragma unroll
+      for (int t0 = 0; t0 < R; t0 += CH) {
+        typename Epi::InPlace q[CH];
+#pragma unroll
+        for (int t = 0; t < CH; ++t) q[t] = epi.read(i + (t0 + t) * span, y, z);
+#pragma unroll
+        for (int t = 0; t < CH; ++t)
+          v[t0 + t] = epi.apply_q(i + (t0 + t) * span, y, z, v[t0 + t], q[t]);
+      }
+    } else
 #pragma unroll
     for (int t = 0; t < R; ++t) {
       // beyond the longest row, for every thread alike: zero, nothing to do

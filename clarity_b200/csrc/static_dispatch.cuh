@@ -83,7 +83,7 @@ template <class SH, class X, bool FUSE, class F>
 inline bool try_xy_tma_tile(const PlanEntry& pe, cudaStream_t st, const F& fn, const float2* S,
                             int family, cudaError_t* err) {
   static_assert(X::OK, "shape not supported by the TMA XY pass");
-  const int stride = X::stage_stride(fn.row_n());
+  const int stride = X::stage_stride(fn.stage_n());
   if (X::blocks_per_sm(stride) < 1) return false;
   // the map depends only on S: encoded once per buffer
   static thread_local const float2* map_s = nullptr;
@@ -113,7 +113,7 @@ inline bool try_xy_tma_tile(const PlanEntry& pe, cudaStream_t st, const F& fn, c
 template <class SH, class X, bool FUSE, class F>
 inline bool try_xy_rows_tile(const PlanEntry& pe, cudaStream_t st, const F& fn, float2* S,
                              int family, cudaError_t* err) {
-  const int stride = X::stage_stride(fn.row_n());
+  const int stride = X::stage_stride(fn.stage_n());
   if (!X::fits(stride)) return false;
   auto k = st::ks_xy_rows<SH, X, F, FUSE>;
   const int smem = X::smem(stride);
@@ -152,7 +152,7 @@ inline bool try_xy_staged(const PlanEntry& pe, cudaStream_t st, const F& fn, flo
       return try_xy_rows_tile<SH, st::XyRows<SH, TG, 64, SH::AY>, FUSE>(pe, st, fn, S, family, err);
     } else if constexpr (SH::W == 2 && SH::M == 256) {
       using X2 = st::XyTma<SH, 2, 512>;
-      if (X2::blocks_per_sm(X2::stage_stride(fn.row_n())) >= 2 &&
+      if (X2::blocks_per_sm(X2::stage_stride(fn.stage_n())) >= 2 &&
           try_xy_tma_tile<SH, X2, FUSE>(pe, st, fn, S, family, err))
         return true;
       return try_xy_tma_tile<SH, st::XyTma<SH, 1, 256>, FUSE>(pe, st, fn, S, family, err);
