@@ -285,30 +285,39 @@ __global__ void __launch_bounds__(128) k_conv3(const Conv3Args a) {
 //   * the load warp brings, by TMA, the unit's input slab (the plane z + dz - 1,
 //     rows y0 - 1 .. y0 + R ty, columns x0 - 1 .. x0 + tx, 16 channels; zero
 //     outside the volume; for a chunk of the half-resolution input the
-//     matching coarse slab) and the 9 taps' weights of that dz into a stage;
+//     matching coarse slab) and the 9 taps' weights of that dz into a stage.
+//     Where every item uses the same weights and they fit, all units' weights
+//     are copied to shared memory once instead;
 //   * eight window warps (two per TMEM lane quarter) turn the slab into the A
 //     operands in TMEM: thread m (TMEM lane m = MMA row m) reads its voxel's 16
-//     channels from the slab and its x neighbours arrive by warp shuffles, so
-//     every tap's shifted window (3 x shifts by S start rows) is written once
-//     with tcgen05.st;
+//     channels and its x neighbours' from the slab, and every tap's shifted
+//     window (3 x shifts by S start rows) is written once with tcgen05.st;
 //   * one issuing thread per MMA tile (R of them) issues that tile's 9 MMAs
 //     (A from TMEM, B = the taps' weights from shared memory) and commits them
 //     to the barriers that free the stage and the window buffer.  A single
 //     thread issues one tcgen05.mma about every 46 cycles whatever N is, so
 //     with N = 16 only several issuers keep the tensor cores busy;
-//   * four epilogue warps read a finished item's accumulators (tcgen05.ld),
-//     add bias, apply ReLU or the mask and store BF16, while the MMAs of the
-//     next item run into the other accumulator buffer.
+//   * eight epilogue warps read a finished item's accumulators (tcgen05.ld),
+//     add bias, apply ReLU and pack to BF16, release the accumulators to the
+//     next item's MMAs (with one buffer they would wait for the stores
+//     otherwise), then apply the mask and store.
+// Measured on one B200, 32 -> 32 channels at 128x128x32: 65.4 -> 55.4 us by the
+// direct slab reads, the early release and the resident weights; 16 -> 16 at
+// 256x256x64: 249 -> 169 us.  What bounds it now is the MMAs' A operand: one
+// takes about 50 cycles at N = 16 and 32 alike, at most a third of them math.
 // Shared memory holds kTmStages stages; TMEM holds two window buffers and one
 // or two accumulator buffers.  Every wait is bounded: a wait that runs out
 // records a timeout in the error word and sets the block's abort flag, the
 // other roles stop at their next wait, in-flight copies and MMAs are waited
 // for (again bounded) and the TMEM is freed.
 #ifndef CLARITY_HOST_EMULATION
-// warps 0-3 epilogue, 4-11 windows (two per TMEM lane quarter), 12 loads,
-// 13-16 MMA issue (one per MMA tile of an item)
-constexpr int kTmWinWarps = 8;
-constexpr int kTmLoadWarp = 4 + kTmWinWarps;
+// warps 0-7 epilogue, 8-15 windows (each two per TMEM lane quarter), 16 loads,
+// 17-20 MMA issue (one per MMA tile of an item)
+constexpr int kTmEpiParts = 2;  // per TMEM lane quarter
+constexpr int kTmEpiWarps = 4 * kTmEpiParts;
+constexpr int kTmWinParts = 2;  // per TMEM lane quarter; three measured the same
+constexpr int kTmWinWarps = 4 * kTmWinParts;
+constexpr int kTmLoadWarp = kTmEpiWarps + kTmWinWarps;
 constexpr int kTmIssueWarp = kTmLoadWarp + 1;
 constexpr int kTmIssuers = 4;
 constexpr int kTmThreads = 32 * (kTmIssueWarp + kTmIssuers);
@@ -323,6 +332,8 @@ struct TmGeom {
   int na;                    // accumulator buffers (1 or 2)
   int cw1, cw2;              // slab row lengths (voxels) of the full- and half-resolution inputs
   uint32_t stage, wofs;      // bytes of a stage; offset of its weights
+  uint32_t wres;             // 0, or offset of all units' weights, kept in shared memory
+  uint32_t bars;             // offset of the mbarriers
   uint32_t tx1, tx2;         // bytes a stage receives for a full- / half-resolution chunk
   uint32_t acc_cols, win_cols;
 };
@@ -398,6 +409,15 @@ __device__ __forceinline__ bool tm_wait(uint64_t* bar, uint32_t parity, volatile
 struct TmItem {
   int z, y0, x0, co0;
 };
+// 16-channel chunks of an item's accumulators at most, for BN channels: what
+// R tiles (R a power of two up to 4) of them leave room for beside two window
+// buffers.
+constexpr int tm_max_chunks(int bn) {
+  int best = 0;
+  for (int r = 1; r <= 4; r *= 2)
+    if (r * bn + 2 * 24 * (r + 2) <= kTmCols) best = r * bn / 16;
+  return best;
+}
 __device__ __forceinline__ TmItem tm_item(const TmGeom& g, int item, int bn) {
   int r = item;
   const int nb = r % g.nnb;
@@ -435,7 +455,7 @@ __global__ void __launch_bounds__(kTmThreads, 1)
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 128, "BN: a multiple of 16 up to 128");
   extern __shared__ unsigned char tm_raw[];
   unsigned char* base = tm_raw + ((1024u - (su32(tm_raw) & 1023u)) & 1023u);
-  uint64_t* full = reinterpret_cast<uint64_t*>(base + kTmStages * g.stage);
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + g.bars);
   uint64_t* empty = full + kTmStages;
   uint64_t* wfull = empty + kTmStages;  // [2] window buffer written
   uint64_t* wempty = wfull + 2;         // [2] window buffer read by its MMAs
@@ -460,10 +480,22 @@ __global__ void __launch_bounds__(kTmThreads, 1)
       mbar_init(&wfull[b], kTmWinWarps);
       mbar_init(&wempty[b], g.R);
       mbar_init(&afull[b], g.R);
-      mbar_init(&aempty[b], 4);
+      mbar_init(&aempty[b], kTmEpiWarps);
     }
     for (int i = 0; i < kTmIssuers; ++i) mbar_init(&drain[i], 1);
     *abort = 0;
+  }
+  if (g.wres) {
+    // unit u's weights as the stages hold them: [8-channel half][tap][BN] rows
+    const int cin = a.c1 + a.c2;
+    for (int e = threadIdx.x; e < nunits * 18 * BN; e += kTmThreads) {
+      const int h = e & 1, co = (e >> 1) % BN, k = (e >> 1) / BN, t9 = k % 9, u = k / 9;
+      const bf16* w = a.w + ((size_t)co * 27 + (u % 3) * 9 + t9) * cin + (u / 3) * 16 + 8 * h;
+      cp16(base + g.wres + ((u * 2 + h) * 9 * BN + t9 * BN + co) * 16, w, w);
+    }
+    cp_commit();
+    cp_wait<0>();
+    fence_smem_to_async();
   }
   tc_fence_before();
   __syncthreads();
@@ -493,8 +525,10 @@ __global__ void __launch_bounds__(kTmThreads, 1)
           else
             tma_load_4d(st, &m2, cc * 16 - a.c1, (it.x0 - 1) >> 1, (it.y0 - 1) >> 1,
                         (it.z + dz - 1) >> 1, &full[s]);
-          tma_load_4d(st + g.wofs, &mw, cc * 16, it.co0, dz * 9, 0, &full[s]);
-          tma_load_4d(st + g.wofs + 9 * BN * 16, &mw, cc * 16 + 8, it.co0, dz * 9, 0, &full[s]);
+          if (!g.wres) {
+            tma_load_4d(st + g.wofs, &mw, cc * 16, it.co0, dz * 9, 0, &full[s]);
+            tma_load_4d(st + g.wofs + 9 * BN * 16, &mw, cc * 16 + 8, it.co0, dz * 9, 0, &full[s]);
+          }
         }
       }
       // the copies of the last stages have landed before the block exits
@@ -525,7 +559,7 @@ __global__ void __launch_bounds__(kTmThreads, 1)
             break;
           }
           tc_fence_after();
-          const uint32_t sw = su32(base + s * g.stage + g.wofs);
+          const uint32_t sw = su32(base + (g.wres ? g.wres + u * (18 * BN * 16) : s * g.stage + g.wofs));
           const uint32_t win = win0 + b * g.win_cols + wrow * 24;
 #pragma unroll
           for (int t9 = 0; t9 < 9; ++t9) {
@@ -545,10 +579,10 @@ __global__ void __launch_bounds__(kTmThreads, 1)
       mbar_wait_bounded(&drain[i], 0, a.err, kTmWaitLimit);
     }
     __syncwarp();
-  } else if (warp >= 4) {
+  } else if (warp >= kTmEpiWarps) {
     // ---- windows: TMEM lane m = MMA row m = voxel (row m / tx, column m % tx);
     // two warps per lane quarter take alternate window rows
-    const int quarter = warp & 3, part = (warp - 4) >> 2;
+    const int quarter = warp & 3, part = (warp - kTmEpiWarps) >> 2;
     const int m = quarter * 32 + lane;
     const int tr = m / g.tx, tc = m - tr * g.tx;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
@@ -571,22 +605,15 @@ __global__ void __launch_bounds__(kTmThreads, 1)
         const bool fullres = cc * 16 < a.c1;
         const uint32_t win = lane_addr + win0 + b * g.win_cols;
 #pragma unroll 1
-        for (int sr = part; sr < g.S; sr += 2) {
+        for (int sr = part; sr < g.S; sr += kTmWinParts) {
           const int hr = sr + tr;
-          uint32_t c[8], e[8], w0[8], w2[8];
-          tm_slab(st, g, fullres, it.y0, it.x0, hr, tc + 1, c);
-          // the warp's edge lanes fetch the neighbour outside the warp
-          tm_slab(st, g, fullres, it.y0, it.x0, hr, lane == 0 ? tc : tc + 2, e);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            w0[k] = __shfl_up_sync(kFull, c[k], 1);
-            w2[k] = __shfl_down_sync(kFull, c[k], 1);
-            if (lane == 0) w0[k] = e[k];
-            if (lane == 31) w2[k] = e[k];
-          }
+          uint32_t w0[8], w1[8], w2[8];
+          tm_slab(st, g, fullres, it.y0, it.x0, hr, tc, w0);
+          tm_slab(st, g, fullres, it.y0, it.x0, hr, tc + 1, w1);
+          tm_slab(st, g, fullres, it.y0, it.x0, hr, tc + 2, w2);
           const uint32_t col = win + (uint32_t)(sr * 3 * 8);
           tc_st8(col, w0);
-          tc_st8(col + 8, c);
+          tc_st8(col + 8, w1);
           tc_st8(col + 16, w2);
         }
         tc_wait_st();
@@ -600,10 +627,16 @@ __global__ void __launch_bounds__(kTmThreads, 1)
       if (!ok) break;
     }
   } else {
-    // ---- epilogue: thread m reads TMEM lane m
-    const int m = threadIdx.x;
+    // ---- epilogue: TMEM lane m = MMA row m; the two warps of a lane quarter
+    // take alternate 16-channel chunks of the item's accumulators
+    const int m = (warp & 3) * 32 + lane, half = warp >> 2;
     const int tr = m / g.tx, tc = m - tr * g.tx;
-    const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+    const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+    constexpr int kPer = BN / 16;              // chunks of a tile
+    // chunks a warp holds at a time (8 registers each), rounds of them if need be
+    constexpr int kMost = tm_max_chunks(BN) / kTmEpiParts;
+    constexpr int kHold = kMost < 8 / kTmEpiParts ? kMost : 8 / kTmEpiParts;
+    const int chunks = g.R * kPer;
     uint32_t j = 0;
     for (int item = blockIdx.x; item < g.items; item += gridDim.x, ++j) {
       const TmItem it = tm_item(g, item, BN);
@@ -611,49 +644,68 @@ __global__ void __launch_bounds__(kTmThreads, 1)
       if (!__all_sync(kFull, tm_wait(&afull[ab], (j / g.na) & 1, abort, a.err))) break;
       tc_fence_after();
       const uint32_t acc = lane_addr + acc0 + ab * g.acc_cols;
-      for (int i = 0; i < g.R; ++i) {
-        const int y = it.y0 + i * g.ty + tr, x = it.x0 + tc;
-        const size_t o0 = (((size_t)it.z * a.H + y) * a.W + x) * a.cout + it.co0;
+      for (int c0 = 0; c0 < chunks; c0 += kTmEpiParts * kHold) {
+        uint32_t pk[kHold][8];
 #pragma unroll
-        for (int c0 = 0; c0 < BN; c0 += 16) {
-          uint32_t r[16];
-          tc_ld16(acc + (uint32_t)(i * BN + c0), r);
-          uint32_t mk[8];
-          if (a.mask) {
-            const uint4 m0 = *reinterpret_cast<const uint4*>(a.mask + o0 + c0);
-            const uint4 m1v = *reinterpret_cast<const uint4*>(a.mask + o0 + c0 + 8);
-            mk[0] = m0.x; mk[1] = m0.y; mk[2] = m0.z; mk[3] = m0.w;
-            mk[4] = m1v.x; mk[5] = m1v.y; mk[6] = m1v.z; mk[7] = m1v.w;
+        for (int n = 0; n < kHold; ++n) {
+          const int c = c0 + kTmEpiParts * n + half;
+          if (c < chunks) {
+            float bv[16];
+            const float* bias = a.bias + it.co0 + (c % kPer) * 16;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) bv[k] = a.bias ? bias[k] : 0.f;
+            uint32_t r[16];
+            tc_ld16(acc + (uint32_t)(c * 16), r);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              float v0 = __uint_as_float(r[2 * k]), v1 = __uint_as_float(r[2 * k + 1]);
+              if (a.bias) {
+                v0 += bv[2 * k];
+                v1 += bv[2 * k + 1];
+              }
+              if (a.relu) {
+                v0 = fmaxf(v0, 0.f);
+                v1 = fmaxf(v1, 0.f);
+              }
+              const __nv_bfloat162 o = __floats2bfloat162_rn(v0, v1);
+              memcpy(&pk[n][k], &o, 4);
+            }
           }
-          uint32_t pk[8];
+        }
+        // all read out: the next item's MMAs may start while this one is stored
+        if (c0 + kTmEpiParts * kHold >= chunks) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tm_arrive(&aempty[ab]);
+        }
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int co = it.co0 + c0 + 2 * k;
-            float v0 = __uint_as_float(r[2 * k]), v1 = __uint_as_float(r[2 * k + 1]);
-            if (a.bias) {
-              v0 += a.bias[co];
-              v1 += a.bias[co + 1];
-            }
-            if (a.relu) {
-              v0 = fmaxf(v0, 0.f);
-              v1 = fmaxf(v1, 0.f);
-            }
+        for (int n = 0; n < kHold; ++n) {
+          const int c = c0 + kTmEpiParts * n + half;
+          if (c < chunks) {
+            const int y = it.y0 + (c / kPer) * g.ty + tr, x = it.x0 + tc;
+            const size_t o =
+                (((size_t)it.z * a.H + y) * a.W + x) * a.cout + it.co0 + (c % kPer) * 16;
             if (a.mask) {
-              __nv_bfloat162 mb;
-              memcpy(&mb, &mk[k], 4);
-              if (!(__bfloat162float(mb.x) > 0.f)) v0 = 0.f;
-              if (!(__bfloat162float(mb.y) > 0.f)) v1 = 0.f;
+              uint32_t mk[8];
+              const uint4 m0 = *reinterpret_cast<const uint4*>(a.mask + o);
+              const uint4 m1v = *reinterpret_cast<const uint4*>(a.mask + o + 8);
+              mk[0] = m0.x; mk[1] = m0.y; mk[2] = m0.z; mk[3] = m0.w;
+              mk[4] = m1v.x; mk[5] = m1v.y; mk[6] = m1v.z; mk[7] = m1v.w;
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                __nv_bfloat162 mb;
+                memcpy(&mb, &mk[k], 4);
+                if (!(__bfloat162float(mb.x) > 0.f)) pk[n][k] &= 0xffff0000u;
+                if (!(__bfloat162float(mb.y) > 0.f)) pk[n][k] &= 0x0000ffffu;
+              }
             }
-            const __nv_bfloat162 o = __floats2bfloat162_rn(v0, v1);
-            memcpy(&pk[k], &o, 4);
+            *reinterpret_cast<uint4*>(a.y + o) =
+                make_uint4(pk[n][0], pk[n][1], pk[n][2], pk[n][3]);
+            *reinterpret_cast<uint4*>(a.y + o + 8) =
+                make_uint4(pk[n][4], pk[n][5], pk[n][6], pk[n][7]);
           }
-          *reinterpret_cast<uint4*>(a.y + o0 + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          *reinterpret_cast<uint4*>(a.y + o0 + c0 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) tm_arrive(&aempty[ab]);
     }
   }
   tc_fence_before();
@@ -673,7 +725,8 @@ __global__ void __launch_bounds__(kTmThreads, 1)
 // once and one input fragment per tap, at the halo's shifted rows.  What bounds
 // it is the fragment loads (one per two MMAs at BM = 16); the form it replaces
 // gathered every tap's shifted input from L2 anew, 16 voxels at a time.
-// Measured at 128x128x48, 16+32 -> 16 channels: see the launch below.
+// Measured on one B200 at 128x128x48: the largest layer, 16+32 -> 16 channels,
+// 952 -> 177 us; the 13 layers of a training step together 2860 -> 770 us.
 constexpr int kWgTaps = 7;        // taps per warp (the last warp has 6)
 constexpr int kVoxTile = kTZ * kTY * kTX;  // 128
 
@@ -1101,6 +1154,14 @@ static int nn_bad(const char* m) {
 }
 
 #ifndef CLARITY_HOST_EMULATION
+static int tm_sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+    return 148;
+  return n;
+}
+
 // Geometry of the tcgen05 convolution for one call, or false when the shape
 // does not suit it (width not a multiple of 32, rows not divisible).
 static bool tm_geometry(const nnk::Conv3Args& a, int* bn_out, nnk::TmGeom* g, int* smem) {
@@ -1145,28 +1206,33 @@ static bool tm_geometry(const nnk::Conv3Args& a, int* bn_out, nnk::TmGeom* g, in
   const uint32_t halo1 = (uint32_t)((tx + 2) * (rows + 2) * 32);
   const uint32_t halo2 = (uint32_t)((tx / 2 + 2) * (rows / 2 + 2) * 32);
   const uint32_t wb = (uint32_t)(2 * 9 * bn * 16);
-  G.wofs = (halo1 + 1023) / 1024 * 1024;
-  G.stage = G.wofs + (wb + 1023) / 1024 * 1024;
-  G.tx1 = halo1 + wb;
-  G.tx2 = halo2 + wb;
+  const uint32_t slab = (halo1 + 1023) / 1024 * 1024;
+  // barriers, alignment slack; at least 120 KB so one block holds an SM (and
+  // its 512 TMEM columns) at a time
+  const int rest = 512 + 1024;
+  // The weights of a stage are 16-byte rows, as slow for a tensor copy as the
+  // slab's 32-byte ones: where every item has the same weights and they fit
+  // beside the stages, they are loaded once (16 -> 16 channels at 256x256x64,
+  // 55 items a block: 249 -> 169 us; 32 -> 32 at 128x128x32, 6.9 items: 58.5 ->
+  // 55.4).  Nothing overlaps that load, so blocks of a few items stream them
+  // (96 -> 32 at 64x64x24, 2.6 items: 47.4 us against 53.4).
+  const long long all = 3ll * ((a.c1 + a.c2) / 16) * wb;
+  const bool res = G.nnb == 1 && items >= 4ll * tm_sm_count() &&
+                   nnk::kTmStages * (long long)slab + all + rest <= 227 * 1024;
+  G.wofs = slab;
+  G.stage = slab + (res ? 0 : (wb + 1023) / 1024 * 1024);
+  G.wres = res ? nnk::kTmStages * G.stage : 0;
+  G.bars = nnk::kTmStages * G.stage + (res ? (uint32_t)all : 0);
+  G.tx1 = halo1 + (res ? 0 : wb);
+  G.tx2 = halo2 + (res ? 0 : wb);
   G.acc_cols = (uint32_t)(R * bn);
   G.win_cols = (uint32_t)(24 * G.S);
-  // stages, barriers, alignment slack; at least 120 KB so one block holds an SM
-  // (and its 512 TMEM columns) at a time
-  int bytes = nnk::kTmStages * (int)G.stage + 512 + 1024;
+  int bytes = (int)G.bars + rest;
   if (bytes < 120 * 1024) bytes = 120 * 1024;
   if (bytes > 227 * 1024) return false;
   *smem = bytes;
   *bn_out = bn;
   return true;
-}
-
-static int tm_sm_count() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-    return 148;
-  return n;
 }
 
 // Launches the tcgen05 convolution.  Returns -1 when the call does not suit

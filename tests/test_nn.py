@@ -191,6 +191,33 @@ def test_conv3_relu_mask_epilogue(clarity_gpu, dims):
     assert torch.equal(ym, torch.where(m > 0, y, torch.zeros_like(y)))
 
 
+@pytest.mark.parametrize("dims,cin,cout", [
+    ((3, 8, 128), 16, 48),    # 12 chunks of 16 channels an item: the epilogue reads them in two rounds
+    ((2, 3, 128), 16, 48),    # one MMA tile of 3 chunks: the epilogue's warps share them unevenly
+    ((2, 2, 128), 16, 128),   # two tiles of 8 chunks
+    ((2, 2, 64), 128, 64),    # two rows of 64 columns a tile
+    ((2, 8, 32), 16, 256),    # two channel blocks: an item's weights differ from the next one's
+    ((170, 4, 128), 32, 32),  # more items than blocks, one accumulator buffer
+    ((600, 4, 128), 16, 16),  # several items a block: weights resident, two buffers
+    ((600, 4, 128), 16, 48),  # the same with one buffer
+    ((600, 2, 64), 32, 32),   # the same, two rows of 64 columns a tile
+])
+def test_conv3_tcgen05_item_shapes(clarity_gpu, dims, cin, cout):
+    from clarity_b200 import unet
+    g = torch.Generator().manual_seed(29 + cin + cout)
+    x = _rand((*dims, cin), g)
+    w = _rand((cout * 27 * cin,), g, 1.0 / np.sqrt(27 * cin))
+    m = _rand((*dims, cout), g).cuda()
+    b = torch.linspace(-0.5, 0.5, cout)
+    y = unet.conv3(x.cuda(), w.cuda(), cout, bias=b.cuda(), relu=False)
+    ym = unet.conv3(x.cuda(), w.cuda(), cout, bias=b.cuda(), relu=False, mask=m)
+    torch.cuda.synchronize()
+    ref = R.conv3(x.to(torch.float64), w.to(torch.float64).reshape(cout, 27, cin), cout,
+                  bias=b.to(torch.float64), relu=False)
+    _close(y.cpu(), ref)
+    assert torch.equal(ym, torch.where(m > 0, y, torch.zeros_like(y)))
+
+
 def test_pool_and_skip_merge(clarity_gpu):
     from clarity_b200 import unet
     g = torch.Generator().manual_seed(4)
