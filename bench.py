@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -165,28 +166,27 @@ def run_reference_arm(args, rank, world):
 
 
 # --------------------------------------------------------------- GPU arm
-def family_bytes(work, img_vox, ker_vox, iters):
-    """Algorithmic HBM bytes of one RL solve, per kernel family.
-    C = complex half spectrum 8*nz*ny*(nx/2+1); R = real work box 4*N; the
-    image and kernel are read unpadded (Ri, Rk).  Schedule per solve: OTF
-    (xy forward + z forward), one xy forward of the image, then per iteration
+def family_bytes(work, img_shape, ker_shape, iters):
+    """Algorithmic HBM bytes of one RL solve, per kernel family, of volumes
+    (z, y, x).  C = complex half spectrum 8*nz*ny*(nx/2+1), Cl and Ck = its part
+    in the image's and the kernel's planes; the image, the estimate (both Ri) and
+    the kernel (Rk) are read and written at their own sizes.  Schedule per solve:
+    OTF (xy forward + z forward), one xy forward of the image, then per iteration
     z (h*cur), xy inverse+forward (ratio), z (h*r) and the product step, which
     also transforms u' for the next iteration except on the last one."""
     nz, ny, nx = work
-    N = nx * ny * nz
     C = 8 * nz * ny * (nx // 2 + 1)
-    R = 4 * N
-    Ri, Rk = 4 * img_vox, 4 * ker_vox
-    cur0 = Ri                       # first iteration reads the image
-    prod_merged = [(C + (cur0 if k == 0 else R) + R + C) for k in range(iters - 1)]
-    last = C + (cur0 if iters == 1 else R) + R
+    Cl, Ck = C * img_shape[0] // nz, C * ker_shape[0] // nz
+    R = 4 * nx * ny * nz
+    Ri, Rk = 4 * math.prod(img_shape), 4 * math.prod(ker_shape)
+    z = C + 2 * Cl  # OTF read, live planes read and written
     return {
-        "xy_forward": (Rk + C) + (Ri + C),
-        "z": 2 * C + 2 * iters * 3 * C,
-        "xy_inv_fwd": iters * (2 * C + Ri),
-        "xy_product": sum(prod_merged),
-        "xy_inverse": last,
-        "per_iteration": 2 * R + Ri + 10 * C,
+        "xy_forward": (Rk + Ck) + (Ri + Cl),
+        "z": Ck + C + 2 * iters * z,
+        "xy_inv_fwd": iters * (2 * Cl + Ri),
+        "xy_product": (iters - 1) * (2 * Cl + 2 * Ri),
+        "xy_inverse": Cl + 2 * Ri,
+        "per_iteration": 2 * C + 8 * Cl + 3 * Ri,
         "per_iteration_survey": 4 * R + 10 * C,
     }
 
@@ -195,8 +195,8 @@ def family_bytes(work, img_vox, ker_vox, iters):
 # measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum) on the
 # steady launches of this workload's iteration 2 (z: the mean of its two
 # launches, P2 and P4).
-NCU_TRAFFIC = {"xy_product": 152.1e6 + 215.7e6, "xy_inv_fwd": 84.5e6 + 20.9e6,
-               "z": (270.7e6 + 46.0e6 + 203.5e6 + 82.6e6) / 2}
+NCU_TRAFFIC = {"xy_product": 84.5e6 + 33.1e6, "xy_inv_fwd": 84.5e6 + 23.8e6,
+               "z": (203.0e6 + 37.4e6 + 202.9e6 + 37.0e6) / 2}
 
 
 def max_over_ranks(value, dist, device):
@@ -461,12 +461,10 @@ def other_configs(api, torch, stream, n_batch=64, batch_iters=30, cfg3_iters=10)
     psfs = [torch.from_numpy(b).cuda() for _, b in cases]
     outs = [torch.empty_like(a) for a in imgs]
     vox = sum(a.numel() for a in imgs)
-    # the schedule's bytes per RL iteration over the batch (2R + Ri + 10C per
-    # volume, as the headline's schedule_bytes), for a bandwidth figure
-    sched = 0
-    for a in imgs:
-        z, y, x = (2 * d for d in a.shape)
-        sched += 2 * 4 * x * y * z + 4 * a.numel() + 10 * 8 * z * y * (x // 2 + 1)
+    # the schedule's bytes per RL iteration over the batch (as the headline's
+    # schedule_bytes), for a bandwidth figure
+    sched = sum(family_bytes(tuple(2 * d for d in a.shape), a.shape, a.shape, 1)["per_iteration"]
+                for a in imgs)
     peak = peaks()[0]
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     desc = (f"{n_batch} volumes of uneven sizes (x, y in 16*{{6..20}}, z in 8*{{2..12}}), "
@@ -499,7 +497,7 @@ def other_configs(api, torch, stream, n_batch=64, batch_iters=30, cfg3_iters=10)
                 "image_voxels": int(vox), "ms": ms,
                 "value": vox * batch_iters / (ms / 1e3) / 1e9, "unit": "Gvoxel-iter/s",
                 "schedule_GBps": gbps, "schedule_frac": gbps / peak,
-                "plans": ("autotuned (fastest of the planner's best four tilings per work box)"
+                "plans": ("autotuned (fastest of the planner's plans per work box)"
                           if tuned else "planner default")}
 
     res["batched_rl"] = timed(False, False)
@@ -520,7 +518,7 @@ def other_configs(api, torch, stream, n_batch=64, batch_iters=30, cfg3_iters=10)
     ms = e0.elapsed_time(e1)
     # the survey's per-iteration bytes (4R + 10C) of the work box, as the
     # headline's survey_frac
-    fb = family_bytes(tuple(2 * d for d in img.shape), img.size, psf.size, cfg3_iters)
+    fb = family_bytes(tuple(2 * d for d in img.shape), img.shape, psf.shape, cfg3_iters)
     large_gbps = fb["per_iteration_survey"] * cfg3_iters / (ms / 1e3) / 1e9
     res["large_rl"] = {"workload": f"RL 512x512x128 fp32 (work box 1024x1024x256), {cfg3_iters} "
                                    "iterations, FP32 SIMT FFT", "ms": ms,
@@ -638,7 +636,7 @@ def run_gpu_arm(args, rank, world):
 
     # roofline of the dominant kernel family
     work = tuple(2 * s for s in IMAGE_ZYX)
-    fb = family_bytes(work, vox, vox, ITERS)
+    fb = family_bytes(work, img.shape, psf.shape, ITERS)
     peak, peak_kind = peaks()
     fam_ms = {k: v for k, v in fam.items() if k != "other" and v[1] > 0}
     dom = max(fam_ms, key=lambda k: fam_ms[k][0]) if fam_ms else None
@@ -677,7 +675,7 @@ def run_gpu_arm(args, rank, world):
             "config": {"workload": WORKLOAD, "image_xyz": [256, 256, 64],
                        "psf_xyz": [256, 256, 64], "work_box_xyz": [512, 512, 128],
                        "iterations_per_step": ITERS, "parallelism": f"replicas x{world}",
-                       "l2": "inputs and working set (~0.7 GB) larger than L2"},
+                       "l2": "inputs and working set (~0.3 GB) larger than L2"},
             "e2e": {"value": e2e_value, "unit": UNIT,
                     "h2d_bytes_per_step": int(img_h.nbytes + psf_h.nbytes),
                     "d2h_bytes_per_step": int(out_h.nbytes), "ms_per_step": e2e_ms},

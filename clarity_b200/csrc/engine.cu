@@ -7,7 +7,7 @@
 // src/BlindMaximumLikelihoodDeconvolve.cxx:102-148, which allocate, plan and
 // free on every call and synchronise after every kernel.  Here plans and
 // buffers are cached per work box, every step is a fused FFT pass, and an
-// RL iteration is five kernel launches with no host round trip.
+// RL iteration is four or five kernel launches with no host round trip.
 #include <algorithm>
 #include <atomic>
 #include <climits>

@@ -17,6 +17,12 @@
 //   * programmatic dependent launch: a kernel's blocks are placed while the one
 //     before drains.  What an earlier kernel may have written is read through
 //     L2 (ld_l2, bulk copies), never through the read-only cache.
+//
+// Measured on one B200 against the runtime-planned passes (passes.cuh), which
+// run 128 registers at two blocks per SM and scalar arithmetic: RL, 20
+// iterations, 256x256x64 with a 64x64x32 PSF (320x320x96 box) 11.7 -> 5.3 ms;
+// 140x126x36 with 31x21x13 (171x147x49) 4.3 -> 1.7 ms; 12 uneven volumes, 5
+// iterations, 35.2 -> 17.7 ms.
 #pragma once
 #include "launch_macro.cuh"
 

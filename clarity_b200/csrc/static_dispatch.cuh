@@ -19,9 +19,10 @@ namespace clarity {
 using ShapeW512 = st::Shape<st::Rad<16, 16>, 16, st::Rad<8, 4>, st::Rad<16, 8>, 2, 2>;
 using ShapeW128 = st::Shape<st::Rad<8, 8>, 16, st::Rad<8>, st::Rad<8, 8>, 1, 4>;
 // The 1024x1024x256 box's XY and z tiles (133 and 128 KB) leave room for one
-// block per SM, so its XY blocks run CLARITY_W1024_THREADS threads and its
-// FP32 z blocks CLARITY_W1024_Z_THREADS (both measured against 256; more XY
-// threads spill registers).  The tensor-core z form keeps the XY count.
+// block per SM, so its XY blocks without staged rows run CLARITY_W1024_THREADS
+// threads and its FP32 z blocks CLARITY_W1024_Z_THREADS (both measured against
+// 256; more threads in those XY passes spill registers; the staged ones, below,
+// run 1024).  The tensor-core z form keeps the XY count.
 #ifndef CLARITY_W1024_THREADS
 #define CLARITY_W1024_THREADS 512
 #endif
@@ -136,7 +137,7 @@ inline bool try_xy_rows_tile(const PlanEntry& pe, cudaStream_t st, const F& fn, 
 //     line) take two lines and 512 threads where the staged rows leave room for
 //     two such blocks per SM (whole sectors: product pass 91 -> 87 us); one line
 //     otherwise.  The 1024x1024x256 box's two lines of 512 columns are one block
-//     of 1024 threads per SM (ratio pass 1122 -> 950 us); rows too long to stage
+//     of 1024 threads per SM (ratio pass 1122 -> 965 us); rows too long to stage
 //     beside them (a work-box volume's) keep the passes without staging.
 template <class SH, bool FUSE, class F>
 inline bool try_xy_staged(const PlanEntry& pe, cudaStream_t st, const F& fn, float2* S, int family,
