@@ -130,7 +130,7 @@ void set_dft_precision(int mode) { g_dft_precision.store(mode); }
 int dft_precision() { return g_dft_precision.load(); }
 
 cudaError_t smem_opt_in(const void* kernel, int smem) {
-  if (smem <= 48 * 1024) return cudaSuccess;
+  if (smem <= kSmemNoOptIn) return cudaSuccess;
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, int> done;  // (kernel, device) -> bytes
   int dev = 0;

@@ -252,9 +252,12 @@ void note_launch_begin(int kind, cudaStream_t st);
 void note_launch_end(int kind, cudaStream_t st);
 void set_capturing(bool on);
 bool pdl_enabled();
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) for kernels above 48 KB,
-// issued once per kernel, device and size (the attribute call is not free, and
-// a solve launches each kernel hundreds of times).
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize), issued once per kernel, device
+// and size (the attribute call is not free, and a solve launches each kernel
+// hundreds of times).  Without it a launch may use 48 KB, the kernel's static
+// shared memory included (the kernels hold up to 4.7 KB of it), so it is left out
+// only for dynamic sizes up to kSmemNoOptIn.
+constexpr int kSmemNoOptIn = 40 * 1024;
 cudaError_t smem_opt_in(const void* kernel, int smem);
 long long launch_count();
 // Counts one kernel launch that note_launch_begin/end do not bracket.

@@ -94,7 +94,7 @@ cudaError_t scratch_address(void** out) {
 
 template <class K>
 cudaError_t allow_smem(K kernel, int smem) {
-  if (smem > 48 * 1024)
+  if (smem > kSmemNoOptIn)
     return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   return cudaSuccess;

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdio>
 #include <cstdlib>
 #include <cstring>
 
@@ -17,6 +18,12 @@ namespace clarity_emu {
 extern thread_local uint3 tIdx, bIdx;
 extern thread_local dim3 bDim, gDim;
 extern thread_local void* smem_ptr;
+
+// A launch without cudaFuncSetAttribute(MaxDynamicSharedMemorySize) may use 48 KB
+// of static and dynamic shared memory together.  The host compiler does not tell a
+// kernel's static share: every kernel is taken to hold kStaticShare.
+constexpr size_t kStaticShare = 1024;
+size_t smem_allowed(const void* kernel);  // dynamic bytes opted in to (0: none)
 
 template <class T>
 T* dynamic_smem() {
@@ -37,6 +44,10 @@ struct Launcher {
         const char* v = std::getenv("EMU_BLOCK_ORDER");
         return v && v[0] == 'r';
       }();
+      if (s + kStaticShare > 48 * 1024 && s > smem_allowed(reinterpret_cast<const void*>(kernel))) {
+        std::fprintf(stderr, "launch with %zu bytes of dynamic shared memory, not opted in to\n", s);
+        std::abort();
+      }
       const unsigned long long nb = (unsigned long long)g.x * g.y * g.z;
       for (unsigned long long q = 0; q < nb; ++q) {
         const unsigned long long b = reverse ? nb - 1 - q : q;

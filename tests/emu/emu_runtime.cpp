@@ -3,6 +3,8 @@
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
 
 #include "emu_cuda.hpp"
 
@@ -10,6 +12,14 @@ namespace clarity_emu {
 thread_local uint3 tIdx, bIdx;
 thread_local dim3 bDim, gDim;
 thread_local void* smem_ptr = nullptr;
+
+static std::mutex g_smem_mu;
+static std::map<const void*, size_t> g_smem;
+size_t smem_allowed(const void* kernel) {
+  std::lock_guard<std::mutex> lk(g_smem_mu);
+  const auto it = g_smem.find(kernel);
+  return it == g_smem.end() ? 0 : it->second;
+}
 }  // namespace clarity_emu
 
 extern "C" {
@@ -97,7 +107,13 @@ cudaError_t cudaGetSymbolAddress(void** p, const void* symbol) {
 const char* cudaGetErrorString(cudaError_t e) {
   return e == cudaSuccess ? "no error" : "emulated error";
 }
-cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
+  if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
+    std::lock_guard<std::mutex> lk(clarity_emu::g_smem_mu);
+    clarity_emu::g_smem[f] = (size_t)v;
+  }
+  return cudaSuccess;
+}
 cudaError_t cudaEventCreate(cudaEvent_t* e) {
   *e = reinterpret_cast<cudaEvent_t>(new double(0));
   return cudaSuccess;

@@ -302,3 +302,16 @@ def test_emulated_column_pair_passes_match_the_general_path(emu, tmp_path, oracl
         finally:
             del os.environ["CLARITY_STATIC"]
         assert rel_l2(got, general) <= 2 * tol, op
+
+
+@pytest.mark.parametrize("ishape,kshape", [((60, 70, 1), (57, 55, 1)),     # z tile of 49072 bytes
+                                           ((20, 9, 200), (15, 8, 180))])  # XY tile of 48912
+def test_emulated_tiles_just_below_48_kb(emu, tmp_path, oracle_lib, ishape, kshape):
+    # the limit of a launch that has not opted in counts a kernel's static
+    # shared memory too (the emulated launch refuses what the device would)
+    r = syn.rng(3 + sum(ishape))
+    img = (r.random(ishape) * 100 + 1).astype(np.float32)
+    psf = syn.gaussian_psf(kshape, 1.5, 1.2).astype(np.float32)
+    assert rel_l2(run_emu(emu, tmp_path, "convolve", img, psf, 0),
+                  oracle_lib.convolve(img, psf)) <= 1e-6
+    assert rel_l2(run_emu(emu, tmp_path, "rl", img, psf, 2), oracle_lib.rl(img, psf, 2)) <= 2e-6

@@ -518,3 +518,19 @@ def test_specialised_boxes_with_uneven_splits(clarity_gpu, image_zyx, psf_zyx):
     want = (g + (1 - (o - A) ** 2 / A ** 2) * (g - o)).clamp_min(0)[inside]
     clarity_gpu.jvc_device(img, psf, out, 1)
     assert ((out.double() - want).norm() / want.norm()).item() <= 2e-6
+
+
+@pytest.mark.parametrize("image_zyx,psf_zyx", [
+    ((36, 220, 144), (36, 220, 144)),  # 288x440x72: z tile of 49024 bytes
+    ((34, 255, 160), (34, 255, 160)),  # 320x510x68: XY tile of 49120 bytes
+    ((60, 70, 1), (57, 55, 1)),        # the smallest boxes with such tiles
+    ((20, 9, 200), (15, 8, 180)),
+])
+def test_boxes_with_tiles_just_below_48_kb(clarity_gpu, oracle_lib, image_zyx, psf_zyx):
+    # dynamic and static shared memory together are beyond 48 KB there
+    r = syn.rng(5 + sum(image_zyx))
+    img = (r.random(image_zyx) * 100 + 1).astype(np.float32)
+    psf = syn.gaussian_psf(psf_zyx, 1.5, 1.2).astype(np.float32)
+    assert rel_l2(clarity_gpu.convolve(img, psf), oracle_lib.convolve(img, psf)) <= 1e-6
+    assert rel_l2(clarity_gpu.maximum_likelihood_deconvolve(img, psf, 2),
+                  oracle_lib.rl(img, psf, 2)) <= 2e-6
