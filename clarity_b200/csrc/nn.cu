@@ -26,6 +26,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "engine.hpp"
 #include "launch_macro.cuh"
@@ -722,7 +723,9 @@ __global__ void __launch_bounds__(kTmThreads, 1)
 // registers over the whole run: warp w owns taps w, w + 4, ...  Per tile it
 // stages the chunk's 4x10x10 halo and the tile's dy once (two stages, copied
 // while the other is multiplied); per 16 voxels a warp loads its dy fragments
-// once and one input fragment per tap, at the halo's shifted rows.  What bounds
+// once and one input fragment per tap, at the halo's shifted rows (a voxel beyond
+// the volume takes zeros: its neighbours can be inside, and its zero gradient
+// times an infinity there would be a NaN).  What bounds
 // it is the fragment loads (one per two MMAs at BM = 16); the form it replaces
 // gathered every tap's shifted input from L2 anew, 16 voxels at a time.
 // Measured on one B200 at 128x128x48: the largest layer, 16+32 -> 16 channels,
@@ -750,12 +753,14 @@ __global__ void __launch_bounds__(128, BM == 16 ? 4 : 3)
   const int t0 = (int)((long long)ntiles * blockIdx.z / gridDim.z);
   const int t1 = (int)((long long)ntiles * (blockIdx.z + 1) / gridDim.z);
 
-  auto load = [&](int tile, int stage) {
+  // origin of the tile to load next
+  int z0 = t0 / tilesx / tilesy * kTZ, y0 = t0 / tilesx % tilesy * kTY, x0 = t0 % tilesx * kTX;
+  // loads that tile, steps to the next one and returns the loaded one's extents
+  // inside the volume, four bits each
+  constexpr int kWhole = kTZ << 8 | kTY << 4 | kTX;
+  auto load = [&](int stage) {
     bf16* H = sm + stage * SMM::STAGE;
     bf16* G = H + SMM::HALO;
-    const int txy = tile / tilesx, tx = tile - txy * tilesx;
-    const int tz = txy / tilesy, ty = txy - tz * tilesy;
-    const int z0 = tz * kTZ, y0 = ty * kTY, x0 = tx * kTX;
     for (int q = threadIdx.x; q < kHalo * 2; q += CLARITY_BLOCK_STRIDE(128)) {
       const int hv = q >> 1, half = q & 1;
       const int hz = hv / (kHY * kHX), r = hv - hz * (kHY * kHX);
@@ -772,6 +777,16 @@ __global__ void __launch_bounds__(128, BM == 16 ? 4 : 3)
       cp16(&G[v * SMM::DROW + ch * 8], src, dy);
     }
     cp_commit();
+    const int inside = (a.D - z0 < kTZ ? a.D - z0 : kTZ) << 8 |
+                       (a.H - y0 < kTY ? a.H - y0 : kTY) << 4 | (a.W - x0 < kTX ? a.W - x0 : kTX);
+    if ((x0 += kTX) >= a.W) {
+      x0 = 0;
+      if ((y0 += kTY) >= a.H) {
+        y0 = 0;
+        z0 += kTZ;
+      }
+    }
+    return inside;
   };
 
 #ifndef CLARITY_HOST_EMULATION
@@ -793,23 +808,20 @@ __global__ void __launch_bounds__(128, BM == 16 ? 4 : 3)
     const int tap = warp + 4 * t < 27 ? warp + 4 * t : 26;
     toff[t] = ((tap / 9) * (kHY * kHX) + (tap / 3) % 3 * kHX + tap % 3) * kRow;
   }
-  if (t0 < t1) load(t0, 0);
-  for (int tile = t0; tile < t1; ++tile) {
-    const int st = (tile - t0) & 1;
-    if (tile + 1 < t1) {
-      load(tile + 1, st ^ 1);
-      cp_wait<1>();
-    } else {
-      cp_wait<0>();
-    }
-    __syncthreads();
-    const bf16* H = sm + st * SMM::STAGE;
+  // zeros in the unused end of the first halo row, never written by load
+  bf16* const zeros = sm + 16;
+  if (threadIdx.x < 8) zeros[threadIdx.x] = __float2bfloat16_rn(0.f);
+  // EDGE: the tile reaches beyond the volume
+  auto multiply = [&](const bf16* H, auto edge, int inside) {
+    constexpr bool EDGE = decltype(edge)::value;
     const bf16* G = H + SMM::HALO;
 #pragma unroll 2
     for (int ks = 0; ks < kVoxTile / 16; ++ks) {
       // 16 voxels: two x rows of the tile
       const int hz = ks / (kTY / 2), hy = 2 * (ks % (kTY / 2));
       const bf16* hb = H + (hz * (kHY * kHX) + hy * kHX + hrow) * kRow + (lane >> 4) * 8;
+      const bool in = !EDGE || (hz < inside >> 8 && hy + (kr >> 3) < (inside >> 4 & 15) &&
+                                (kr & 7) < (inside & 15));
       uint32_t af[BM / 16][4];
 #pragma unroll
       for (int i = 0; i < BM / 16; ++i)
@@ -818,7 +830,7 @@ __global__ void __launch_bounds__(128, BM == 16 ? 4 : 3)
 #pragma unroll
       for (int t = 0; t < kWgTaps; ++t) {
         uint32_t bfr[4];
-        ldm_x4_t(bfr, hb + toff[t]);
+        ldm_x4_t(bfr, in ? hb + toff[t] : zeros);
 #pragma unroll
         for (int i = 0; i < BM / 16; ++i) {
           mma16816(acc[t][i][0], af[i], bfr);
@@ -826,6 +838,22 @@ __global__ void __launch_bounds__(128, BM == 16 ? 4 : 3)
         }
       }
     }
+  };
+  int next = t0 < t1 ? load(0) : 0;
+  for (int tile = t0; tile < t1; ++tile) {
+    const int st = (tile - t0) & 1, inside = next;
+    if (tile + 1 < t1) {
+      next = load(st ^ 1);
+      cp_wait<1>();
+    } else {
+      cp_wait<0>();
+    }
+    __syncthreads();
+    const bf16* H = sm + st * SMM::STAGE;
+    if (inside == kWhole)
+      multiply(H, std::false_type{}, inside);
+    else
+      multiply(H, std::true_type{}, inside);
     __syncthreads();
   }
 #pragma unroll
@@ -848,10 +876,13 @@ __global__ void __launch_bounds__(128, BM == 16 ? 4 : 3)
   static thread_local float accs[27][BM][16];
   std::memset(accs, 0, sizeof(accs));
   for (int tile = t0; tile < t1; ++tile) {
-    load(tile, 0);
+    const int inside = load(0);
     const bf16* H = sm;
     const bf16* G = H + SMM::HALO;
     for (int v = 0; v < kVoxTile; ++v) {
+      if (v / (kTY * kTX) >= inside >> 8 || (v / kTX) % kTY >= (inside >> 4 & 15) ||
+          v % kTX >= (inside & 15))
+        continue;
       const int h0 = (v / (kTY * kTX) * kHY + (v / kTX) % kTY) * kHX + v % kTX;
       for (int t = 0; t < 27; ++t) {
         const bf16* h = H + (h0 + t / 9 * (kHY * kHX) + t / 3 % 3 * kHX + t % 3) * kRow;

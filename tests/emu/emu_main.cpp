@@ -38,7 +38,8 @@ static void dump(const std::string& path, const std::vector<float>& v) {
   std::fwrite(v.data(), sizeof(float), v.size(), f);
   std::fclose(f);
 }
-static int nn_conv_case(Clarity_Dim3 id, Clarity_Dim3 kd, int relu, const char* prefix) {
+// inf: infinite inputs at the last voxel and at the last column of the first row.
+static int nn_conv_case(Clarity_Dim3 id, Clarity_Dim3 kd, int relu, const char* prefix, bool inf) {
   const int W = id.x, H = id.y, D = id.z, c1 = kd.x, c2 = kd.y, co = kd.z, cin = c1 + c2;
   const size_t V = (size_t)D * H * W, V2 = c2 ? V / 8 : 0;
   auto mk = [](size_t n, uint32_t seed, float scale, std::vector<__nv_bfloat16>* b,
@@ -54,6 +55,11 @@ static int nn_conv_case(Clarity_Dim3 id, Clarity_Dim3 kd, int relu, const char* 
   std::vector<float> fx1, fx2, fw, fdy, fb(co);
   mk(V * c1, 1, 1.0f, &x1, &fx1);
   mk(V2 * c2, 2, 1.0f, &x2, &fx2);
+  if (inf)
+    for (size_t i : {(V - 1) * c1 + 3, (size_t)(W - 1) * c1 + 5}) {
+      fx1[i] = INFINITY;
+      x1[i] = __float2bfloat16_rn(INFINITY);
+    }
   mk((size_t)co * 27 * cin, 3, 0.1f, &wq, &fw);
   mk(V * co, 4, 1.0f, &dy, &fdy);
   for (int i = 0; i < co; ++i) fb[i] = hval(100 + i, 0.2f);
@@ -87,7 +93,8 @@ int main(int argc, char** argv) {
   Clarity_Dim3 id{std::atoi(argv[2]), std::atoi(argv[3]), std::atoi(argv[4])};
   Clarity_Dim3 kd{std::atoi(argv[5]), std::atoi(argv[6]), std::atoi(argv[7])};
   const double param = std::atof(argv[8]);
-  if (op == "nnconv") return nn_conv_case(id, kd, (int)param, argv[11]);
+  if (op == "nnconv" || op == "nnconvinf")
+    return nn_conv_case(id, kd, (int)param, argv[11], op == "nnconvinf");
   const size_t ni = (size_t)id.x * id.y * id.z, nk = (size_t)kd.x * kd.y * kd.z;
   std::vector<float> img = read_raw(argv[9], ni), psf = read_raw(argv[10], nk), out(ni);
   if (Clarity_Register() != CLARITY_SUCCESS) return 3;

@@ -315,3 +315,27 @@ def test_emulated_tiles_just_below_48_kb(emu, tmp_path, oracle_lib, ishape, ksha
     assert rel_l2(run_emu(emu, tmp_path, "convolve", img, psf, 0),
                   oracle_lib.convolve(img, psf)) <= 1e-6
     assert rel_l2(run_emu(emu, tmp_path, "rl", img, psf, 2), oracle_lib.rl(img, psf, 2)) <= 2e-6
+
+
+@pytest.mark.parametrize("dims,cout", [((3, 9, 17), 16), ((2, 8, 13), 32)])
+def test_emulated_weight_gradient_keeps_infinities_to_their_taps(emu, tmp_path, dims, cout):
+    # a tile's voxels beyond the volume have neighbours inside it: their zero
+    # gradients must not meet an infinite input (0 * inf)
+    D, H, W = dims
+    c1 = 16
+    pre = str(tmp_path / "nn")
+    p = subprocess.run([emu, "nnconvinf", str(W), str(H), str(D), str(c1), "0", str(cout), "0",
+                        "-", "-", pre], capture_output=True, text=True,
+                       env=dict(os.environ, ASAN_OPTIONS="detect_leaks=0"))
+    assert p.returncode == 0, p.stderr[-2000:]
+    rd = lambda s, shape: np.fromfile(pre + "." + s, np.float32).reshape(shape)  # noqa: E731
+    x = np.pad(rd("x1", (D, H, W, c1)).astype(np.float64), ((1, 1), (1, 1), (1, 1), (0, 0)))
+    dy = rd("dy", (D, H, W, cout)).astype(np.float64).reshape(-1, cout)
+    dw = rd("dw", (cout, 27, c1))
+    for t in range(27):
+        sh = x[t // 9:t // 9 + D, t // 3 % 3:t // 3 % 3 + H, t % 3:t % 3 + W].reshape(-1, c1)
+        finite = np.isfinite(sh).all(0)
+        assert np.array_equal(np.isfinite(dw[:, t]).all(0), finite), t
+        want = dy.T @ sh[:, finite]
+        assert np.abs(dw[:, t][:, finite] - want).max() <= 1e-5 * np.abs(want).max(), t
+    assert np.isfinite(dw).any() and not np.isfinite(dw).all()

@@ -125,6 +125,42 @@ def test_conv3_weight_gradient_at_tile_edges(clarity_gpu, dims, c1, c2, cout):
     assert ((db.cpu().double() - f.sum(0)).abs() <= bound * f.abs().sum(0) + 1e-30).all()
 
 
+@pytest.mark.parametrize("dims,c1,c2,cout", [((3, 9, 17), 16, 0, 16), ((2, 8, 13), 16, 0, 32),
+                                             ((6, 10, 14), 16, 16, 16)])
+def test_conv3_weight_gradient_keeps_infinities_to_their_taps(clarity_gpu, dims, c1, c2, cout):
+    # a tile's voxels beyond the volume have neighbours inside it: their zero
+    # gradients must not meet an infinite input (0 * inf).  The finite entries'
+    # bound is that of the test above.
+    from clarity_b200 import unet
+    D, H, W = dims
+    g = torch.Generator().manual_seed(sum(dims) + cout)
+    rnd = lambda *s: torch.randn(s, generator=g).to(torch.bfloat16)  # noqa: E731
+    x1, dy = rnd(D, H, W, c1), rnd(D, H, W, cout)
+    x2 = rnd(D // 2, H // 2, W // 2, c2) if c2 else None
+    x1[D - 1, H - 1, W - 1, 3] = float("inf")
+    x1[0, 0, W - 1, 5] = float("-inf")
+    x1[D - 1, 0, 0, 7] = float("nan")
+    cin = c1 + c2
+    dw = torch.zeros(cout * 27 * cin, device="cuda")
+    unet.conv3_wgrad(x1.cuda(), dy.cuda(), dw, None, x2=x2.cuda() if c2 else None)
+    torch.cuda.synchronize()
+    x = x1.double()
+    if c2:
+        up = x2.double()
+        for d in range(3):
+            up = up.repeat_interleave(2, d)
+        x = torch.cat([x, up], 3)
+    p = torch.nn.functional.pad(x, (0, 0, 1, 1, 1, 1, 1, 1))
+    f = dy.double().reshape(-1, cout)
+    got = dw.cpu().double().reshape(cout, 27, cin)
+    for t in range(27):
+        sh = p[t // 9:t // 9 + D, t // 3 % 3:t // 3 % 3 + H, t % 3:t % 3 + W].reshape(-1, cin)
+        ok = sh.isfinite().all(0)
+        assert torch.equal(got[:, t].isfinite().all(0), ok), t
+        assert ((got[:, t][:, ok] - f.T @ sh[:, ok]).abs()
+                <= 256 * 2.0 ** -24 * (f.abs().T @ sh[:, ok].abs()) + 1e-30).all(), t
+
+
 _CROSS = """
 import sys, numpy as np, torch
 from clarity_b200 import unet
