@@ -30,6 +30,7 @@
 
 #include "engine.hpp"
 #include "launch_macro.cuh"
+#include "nn_grid.hpp"
 #include "ops.cuh"
 
 namespace clarity {
@@ -122,7 +123,6 @@ inline void cp_wait() {}
 // supplies its own row address), so an input voxel is read from HBM/L2 once
 // per chunk instead of once per tap.  128 threads; warp w owns tile voxels
 // [32w, 32w + 32) (tile z = w / 2, y rows 4(w % 2) .. +3).
-constexpr int kTZ = 2, kTY = 8, kTX = 8;
 constexpr int kHZ = kTZ + 2, kHY = kTY + 2, kHX = kTX + 2;
 constexpr int kHalo = kHZ * kHY * kHX;  // 400 voxels
 
@@ -744,17 +744,21 @@ struct WgradSmem {
 template <int BM>
 __global__ void __launch_bounds__(128, BM == 16 ? 4 : 3)
     k_conv3_wgrad(const Conv3Args a, const bf16* __restrict__ dy, float* __restrict__ dw,
-                  int tilesx, int tilesy, int ntiles) {
+                  const WgradGrid g) {
   static_assert(BM == 16 || BM == 32, "BM: 16 or 32");
   using SMM = WgradSmem<BM>;
   CLARITY_DYN_SMEM(bf16, sm);
   const int cin = a.c1 + a.c2, N = 27 * cin;
-  const int c0 = blockIdx.x * 16, co0 = blockIdx.y * BM;
-  const int t0 = (int)((long long)ntiles * blockIdx.z / gridDim.z);
-  const int t1 = (int)((long long)ntiles * (blockIdx.z + 1) / gridDim.z);
+  const int cob = blockIdx.x / (cin / 16);
+  const int c0 = (blockIdx.x - cob * (cin / 16)) * 16, co0 = cob * BM;
+  const int run = blockIdx.z * g.gy + blockIdx.y;
+  if (run >= g.runs) return;
+  const int t0 = (int)((long long)g.ntiles * run / g.runs);
+  const int t1 = (int)((long long)g.ntiles * (run + 1) / g.runs);
 
   // origin of the tile to load next
-  int z0 = t0 / tilesx / tilesy * kTZ, y0 = t0 / tilesx % tilesy * kTY, x0 = t0 % tilesx * kTX;
+  int z0 = t0 / g.tilesx / g.tilesy * kTZ, y0 = t0 / g.tilesx % g.tilesy * kTY;
+  int x0 = t0 % g.tilesx * kTX;
   // loads that tile, steps to the next one and returns the loaded one's extents
   // inside the volume, four bits each
   constexpr int kWhole = kTZ << 8 | kTY << 4 | kTX;
@@ -1184,15 +1188,17 @@ static int nn_bad(const char* m) {
   return CLARITY_INVALID_ARGUMENT;
 }
 
-#ifndef CLARITY_HOST_EMULATION
 static int tm_sm_count() {
+#ifndef CLARITY_HOST_EMULATION
   int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-    return 148;
-  return n;
+  if (cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0)
+    return n;
+#endif
+  return 148;
 }
 
+#ifndef CLARITY_HOST_EMULATION
 // Geometry of the tcgen05 convolution for one call, or false when the shape
 // does not suit it (width not a multiple of 32, rows not divisible).
 static bool tm_geometry(const nnk::Conv3Args& a, int* bn_out, nnk::TmGeom* g, int* smem) {
@@ -1385,31 +1391,17 @@ CLARITY_API ClarityResult_t clarityx_nn_conv3_wgrad(const void* x1, int c1, cons
   nnk::Conv3Args a{static_cast<const bf16*>(x1), c1, static_cast<const bf16*>(x2), c2, D, H, W,
                    D / 2, H / 2, W / 2, nullptr, nullptr, cout, 0, nullptr, nullptr};
   const long long V = (long long)D * H * W;
-  const int cin = c1 + c2;
-  // 32 output channels a block where they divide: twice the MMAs per input
-  // fragment; more would not leave registers for three blocks per SM
-  const int bm = cout % 32 == 0 ? 32 : 16;
-  const int tx = (W + nnk::kTX - 1) / nnk::kTX, ty = (H + nnk::kTY - 1) / nnk::kTY;
-  const int ntiles = tx * ty * ((D + nnk::kTZ - 1) / nnk::kTZ);
-  // runs of tiles: enough blocks for the SMs several times over, but at least
-  // four tiles each (once every SM has a block) so that a block's 27 * 16 * bm
-  // atomics stay a small part,
-  // and at most 12 (96 MMAs into one accumulator): the tensor cores' FP32 sums
-  // lose about an ulp a step, and with 31 tiles a run dW's error against 64 bits
-  // was 1.3e-6 where runs of 128 MMAs had 8e-7
-  const int cols = (cin / 16) * (cout / bm);
-  const int runs = std::max((ntiles + 11) / 12,
-                            std::min((148 * (bm == 16 ? 4 : 3) + cols - 1) / cols,
-                                     std::max(ntiles / 4, std::min(ntiles, 148 / cols + 1))));
-  const dim3 grid(cin / 16, cout / bm, runs);
+  nnk::WgradGrid g;
+  if (!nnk::wgrad_grid(D, H, W, c1 + c2, cout, tm_sm_count(), &g))
+    return (ClarityResult_t)nn_bad("wgrad: volumes of 2^31 voxels or more");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bf16* d = static_cast<const bf16*>(dy);
-  auto kern = bm == 32 ? nnk::k_conv3_wgrad<32> : nnk::k_conv3_wgrad<16>;
-  const int smem = bm == 32 ? nnk::WgradSmem<32>::BYTES : nnk::WgradSmem<16>::BYTES;
+  auto kern = g.bm == 32 ? nnk::k_conv3_wgrad<32> : nnk::k_conv3_wgrad<16>;
+  const int smem = g.bm == 32 ? nnk::WgradSmem<32>::BYTES : nnk::WgradSmem<16>::BYTES;
   const cudaError_t se = clarity::smem_opt_in(reinterpret_cast<const void*>(kern), smem);
   if (se != cudaSuccess) return (ClarityResult_t)nn_err(se);
   clarity::note_launch_begin(clarity::KK_OTHER, st);
-  CLARITY_LAUNCH(kern, grid, 128, smem, st)(a, d, dw, tx, ty, ntiles);
+  CLARITY_LAUNCH(kern, dim3(g.cols, g.gy, g.gz), 128, smem, st)(a, d, dw, g);
   if (dbias) {
     const int noct = cout / 8;
     const int bt = noct >= 256 ? 256 : 256 / noct * noct;

@@ -183,3 +183,43 @@ def test_compat_header_compiles_a_reference_style_caller(tmp_path):
                        capture_output=True, text=True)
     assert p.returncode == 0, p.stderr
     assert subprocess.run([str(exe)]).returncode == 0
+
+
+_WGRAD_GRID = r"""
+#include <cstdio>
+#include "nn_grid.hpp"
+int main() {
+  const int dims[][3] = {{1, 8192, 8192}, {384, 512, 512}, {2, 1, 67107840}, {1, 1, 1}, {2, 8, 8},
+                         {26, 40, 40}, {9, 17, 33}, {256, 512, 512}, {2047, 1024, 1024}};
+  const int ch[][2] = {{16, 16}, {48, 16}, {192, 64}, {128, 2064}};
+  for (auto& d : dims)
+    for (auto& c : ch) {
+      clarity::nn::WgradGrid g;
+      if (!clarity::nn::wgrad_grid(d[0], d[1], d[2], c[0], c[1], 148, &g)) return 1;
+      if (g.gy < 1 || g.gy > 65535 || g.gz < 1 || g.gz > 65535) return 2;
+      if ((long long)g.gy * g.gz < g.runs || g.runs < 1 || g.runs > g.ntiles) return 3;
+      if (g.cols != c[0] / 16 * (c[1] / g.bm) || c[1] % g.bm) return 4;
+      if ((long long)g.tilesx * clarity::nn::kTX < d[2] || (long long)g.tilesy * clarity::nn::kTY < d[1])
+        return 5;
+      long long next = 0;  // the runs cover every tile once, at most 12 each
+      for (int r = 0; r < g.runs; ++r) {
+        const long long t0 = (long long)g.ntiles * r / g.runs, t1 = (long long)g.ntiles * (r + 1) / g.runs;
+        if (t0 != next || t1 <= t0 || t1 - t0 > 12) return 6;
+        next = t1;
+      }
+      if (next != g.ntiles) return 7;
+    }
+  clarity::nn::WgradGrid g;
+  return clarity::nn::wgrad_grid(2048, 1024, 1024, 16, 16, 148, &g) ? 8 : 0;
+}
+"""
+
+
+def test_weight_gradient_launch_covers_large_volumes(tmp_path):
+    # a grid's y and z extents end at 65535; 1x8192x8192 voxels have 87382 runs
+    src = tmp_path / "grid.cpp"
+    src.write_text(_WGRAD_GRID)
+    exe = str(tmp_path / "grid")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fsanitize=undefined", "-fno-sanitize-recover",
+                    "-I", os.path.join(ROOT, "clarity_b200", "csrc"), str(src), "-o", exe], check=True)
+    assert subprocess.run([exe]).returncode == 0

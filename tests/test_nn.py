@@ -161,6 +161,35 @@ def test_conv3_weight_gradient_keeps_infinities_to_their_taps(clarity_gpu, dims,
                 <= 256 * 2.0 ** -24 * (f.abs().T @ sh[:, ok].abs()) + 1e-30).all(), t
 
 
+def test_conv3_weight_gradient_of_more_runs_than_a_grid_dimension(clarity_gpu):
+    # 1x8192x8192 voxels: 87382 runs of tiles, against 65535 blocks of a grid's y
+    # or z.  dy is zero but for 303 voxels, the corners and the last tiles among
+    # them: a sum has at most 303 terms and the additions of zeros are exact.
+    from clarity_b200 import unet
+    H = W = 8192
+    g = torch.Generator(device="cuda").manual_seed(8)
+    x = torch.empty((1, H, W, 16), dtype=torch.bfloat16, device="cuda").normal_(generator=g)
+    at = torch.cat([torch.tensor([0, W - 1, (H - 1) * W, H * W - 1, (H - 1) * W - 9]),
+                    H * W - 1 - torch.arange(3, 51),
+                    torch.randint(0, H * W, (250,), generator=torch.Generator().manual_seed(9))])
+    at = at.unique().cuda()
+    v = torch.randn((len(at), 16), generator=g, device="cuda").to(torch.bfloat16)
+    dy = torch.zeros((1, H, W, 16), dtype=torch.bfloat16, device="cuda")
+    dy.view(-1, 16)[at] = v
+    dw = torch.zeros(16 * 27 * 16, device="cuda")
+    db = torch.zeros(16, device="cuda")
+    unet.conv3_wgrad(x, dy, dw, db)
+    torch.cuda.synchronize()
+    f, got = v.double(), dw.double().reshape(16, 27, 16)
+    bound = 2 * 303 * 2.0 ** -24
+    for t in range(27):
+        yy, xx = at // W + t // 3 % 3 - 1, at % W + t % 3 - 1
+        ok = (t // 9 == 1) & (yy >= 0) & (yy < H) & (xx >= 0) & (xx < W)
+        sh = x.view(-1, 16)[(yy * W + xx).clamp(0, H * W - 1)].double() * ok[:, None]
+        assert ((got[:, t] - f.T @ sh).abs() <= bound * (f.abs().T @ sh.abs()) + 1e-30).all(), t
+    assert ((db.double() - f.sum(0)).abs() <= bound * f.abs().sum(0) + 1e-30).all()
+
+
 _CROSS = """
 import sys, numpy as np, torch
 from clarity_b200 import unet
