@@ -190,6 +190,24 @@ def test_conv3_weight_gradient_of_more_runs_than_a_grid_dimension(clarity_gpu):
     assert ((db.double() - f.sum(0)).abs() <= bound * f.abs().sum(0) + 1e-30).all()
 
 
+@pytest.mark.parametrize("cout", [16, 48, 80, 128, 2032, 2048, 2064])
+@pytest.mark.parametrize("voxels", [1, 5, 300])
+def test_conv3_bias_gradient(clarity_gpu, cout, voxels):
+    # one to 128 lanes of threads a channel octet, odd numbers of them, and more
+    # octets than threads; sums of at most 300 terms
+    from clarity_b200 import unet
+    g = torch.Generator().manual_seed(cout + voxels)
+    x = torch.zeros((1, 1, voxels, 16), dtype=torch.bfloat16, device="cuda")
+    dy = torch.randn((1, 1, voxels, cout), generator=g).to(torch.bfloat16)
+    dw = torch.zeros(cout * 27 * 16, device="cuda")
+    db = torch.zeros(cout, device="cuda")
+    unet.conv3_wgrad(x, dy.cuda(), dw, db)
+    torch.cuda.synchronize()
+    f = dy.double().reshape(-1, cout)
+    assert ((db.cpu().double() - f.sum(0)).abs() <= 300 * 2.0 ** -24 * f.abs().sum(0)).all()
+    assert not dw.any()
+
+
 _CROSS = """
 import sys, numpy as np, torch
 from clarity_b200 import unet
