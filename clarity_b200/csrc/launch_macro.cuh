@@ -54,8 +54,6 @@ inline PdlLauncher<P...> pdl_launcher(void (*k)(P...), dim3 grid, dim3 block, si
 // Loop stride of a block-wide strided loop in kernels launched with a
 // compile-time block size.
 #define CLARITY_BLOCK_STRIDE(n) (n)
-// Lanes of the warp that issues bulk copies.
-#define CLARITY_ISSUE_LANES 32
 #else
 #include "emu_cuda.hpp"
 #define CLARITY_LAUNCH(kernel, grid, block, smem, stream) \
@@ -65,7 +63,6 @@ inline PdlLauncher<P...> pdl_launcher(void (*k)(P...), dim3 grid, dim3 block, si
 #define CLARITY_PDL_WAIT() ((void)0)
 #define CLARITY_DYN_SMEM(T, name) T* name = ::clarity_emu::dynamic_smem<T>()
 #define CLARITY_BLOCK_STRIDE(n) ((int)blockDim.x)
-#define CLARITY_ISSUE_LANES ((int)blockDim.x)
 #endif
 
 // The block index and grid size the pass bodies and the operations fused into

@@ -338,9 +338,8 @@ struct EpiWork {
     r.o[x] = v;
     return v;
   }
-    // padding rows / z planes where the result is known to be zero
+  // padding rows where the result is known to be zero
   __device__ __forceinline__ bool zero_row(int, int) const { return false; }
-  __device__ __forceinline__ bool zero_plane(int) const { return false; }
   // rows y0base + BY*j, j < live_rows, can be nonzero (all here)
   __device__ __forceinline__ int live_rows(int, int, int ay) const { return ay; }
   __device__ __forceinline__ void prefetch_row(int, int) const {}
@@ -386,8 +385,6 @@ struct EpiClip {
     return v;
   }
   // rows and planes outside the image are not asked for: not transformed
-  __device__ __forceinline__ bool zero_row(int y, int z) const { return y >= Y || z >= Z; }
-  __device__ __forceinline__ bool zero_plane(int z) const { return z >= Z; }
   int live_planes(int nz) const { return Z < nz ? Z : nz; }
   CLARITY_HD inline int live_rows(int y0base, int by, int ay) const {
     return rows_below(Y, y0base, by, ay);
@@ -455,7 +452,6 @@ struct EpiRLProduct {
     return a;
   }
   __device__ __forceinline__ bool zero_row(int y, int z) const { return y >= Y || z >= Z; }
-  __device__ __forceinline__ bool zero_plane(int z) const { return z >= Z; }
   int live_planes(int nz) const { return Z < nz ? Z : nz; }
   CLARITY_HD inline int live_rows(int y0base, int by, int ay) const {
     return rows_below(Y, y0base, by, ay);
@@ -496,13 +492,6 @@ struct EpiRLProduct {
   __device__ __forceinline__ void finish() {
     block_sum_store(acc, partial);
     if (nblocks && CLARITY_BLOCK_ID() == 0 && threadIdx.x == 0) *nblocks = (int)CLARITY_GRID_DIM();
-  }
-  // a block whose plane lies outside the estimate contributes zero
-  __device__ __forceinline__ void finish_skipped() {
-    if (threadIdx.x == 0) {
-      partial[CLARITY_BLOCK_ID()] = 0.0;
-      if (nblocks && CLARITY_BLOCK_ID() == 0) *nblocks = (int)CLARITY_GRID_DIM();
-    }
   }
 };
 
@@ -560,12 +549,11 @@ struct MidRLRatio {
     if (idiv_partial && x < r.n) idiv_add(a, b);
     return live_ratio(x < r.n, a, b);
   }
-    // g is zero outside the image, so the ratio is exactly zero there
+  // g is zero outside the image, so the ratio is exactly zero there
   // (0/b, or the 1e-5 guard): rows with y >= Y and planes with z >= Z need no
   // transform at all
   __device__ __forceinline__ bool zero_row(int y, int z) const { return y >= g.Y || z >= g.Z; }
-  __device__ __forceinline__ bool zero_plane(int z) const { return z >= g.Z; }
-  // planes a launch needs to cover (the rest are zero_plane)
+  // planes a launch covers (the rest are neither read nor written: Mod::zn)
   int live_planes(int nz) const { return g.Z < nz ? g.Z : nz; }
   // rows y0base + by*j with j < live_rows lie inside the image (y < Y)
   CLARITY_HD inline int live_rows(int y0base, int by, int ay) const {
@@ -596,13 +584,6 @@ struct MidRLRatio {
     if (idiv_partial) {
       block_sum_store(acc, idiv_partial);
       if (nblocks && CLARITY_BLOCK_ID() == 0 && threadIdx.x == 0) *nblocks = (int)CLARITY_GRID_DIM();
-    }
-  }
-  // a block that returned early (plane outside the image) contributes zero
-  __device__ __forceinline__ void finish_skipped() {
-    if (idiv_partial && threadIdx.x == 0) {
-      idiv_partial[CLARITY_BLOCK_ID()] = 0.0;
-      if (nblocks && CLARITY_BLOCK_ID() == 0) *nblocks = (int)CLARITY_GRID_DIM();
     }
   }
 };
@@ -663,9 +644,8 @@ struct EpiJVC {
     r.o[x] = v;
     return v;
   }
-    // padding rows / z planes where the result is known to be zero
+  // padding rows where the result is known to be zero
   __device__ __forceinline__ bool zero_row(int, int) const { return false; }
-  __device__ __forceinline__ bool zero_plane(int) const { return false; }
   // rows y0base + BY*j, j < live_rows, can be nonzero (all here)
   __device__ __forceinline__ int live_rows(int, int, int ay) const { return ay; }
   __device__ __forceinline__ void prefetch_row(int y, int z) const {

@@ -618,12 +618,6 @@ __global__ void __launch_bounds__(SH::THREADS, SH::XY_MINB)
   CLARITY_DYN_SMEM(float2, sm);
   const int z = blockIdx.x / SH::NGROUPS;
   const int y0base = (blockIdx.x - z * SH::NGROUPS) * SH::G;
-  // a plane whose result is known to be zero is neither read nor written;
-  // the next Z pass reads those planes as zeros (Mod::zn)
-  if (mid.zero_plane(z)) {  // neither read nor written (see Mod::zn)
-    if constexpr (requires { mid.finish_skipped(); }) mid.finish_skipped();
-    return;
-  }
   prefetch_tile_rows<SH>(mid, z, y0base);
   const RowSkip<SH, Mid> skip{mid, z, y0base};
   cols_inverse<SH>(sm, S, z, y0base, T.twr, T.twny);
@@ -646,17 +640,15 @@ __global__ void __launch_bounds__(SH::THREADS, SH::XY_MINB)
   mid.finish();
 }
 
-// First z stage of the spectral pass: the FP32 register pass, or (PREC > 0,
-// a 16 x 16 z axis) its tensor-core form on split hi+lo operands.
+// First z stage of the precision form (a 16 x 16 z axis): tensor cores on split
+// hi+lo operands; the emulation has the FP32 register pass.
 template <class SH, int DIR, int PREC>
 __device__ __forceinline__ void z_stage0(float2* sm, const float2* __restrict__ tw) {
 #ifndef CLARITY_HOST_EMULATION
-  if constexpr (PREC != kDftF32) {
-    z_stage16_tc<SH, DIR, PREC>(sm, tw);
-    return;
-  }
-#endif
+  z_stage16_tc<SH, DIR, PREC>(sm, tw);
+#else
   z_tile_pass<SH, typename SH::Z, 0, DIR, true>(sm, tw);
+#endif
 }
 
 // Whether the tensor-core z stage applies to a shape: radix 16 first, whole
@@ -665,10 +657,13 @@ template <class SH>
 constexpr bool kTcZ = SH::Z::radix(0) == 16 && SH::Z::npass >= 2 && SH::BW % 8 == 0 &&
                       !SH::Y_PER_LINE;
 
-template <class SH, class Mod, int PREC = kDftF32>
+// The z pass of the precision form (the FP32 and forward-only passes of its boxes
+// are ks_z3's).
+template <class SH, class Mod, int PREC>
 __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
     ks_z(const Mod mod, const float2* __restrict__ Sin, float2* __restrict__ Sout,
          const Tables T) {
+  static_assert(kTcZ<SH> && PREC != kDftF32 && !Mod::forward_only, "the precision form only");
   CLARITY_DYN_SMEM(float2, sm);
   constexpr int tile = SH::TILE;
   const long long base = (long long)blockIdx.x * tile;
@@ -688,30 +683,22 @@ __global__ void __launch_bounds__(SH::THREADS, SH::Z_MINB)
   }
   __syncthreads();
   tile_forward_from<SH, typename SH::Y, 0, false>(sm, T.twy);
-  if constexpr (Mod::forward_only) {
-    tile_forward_from<SH, typename SH::Z, 0, true>(sm, T.twz);
-  } else {
-    // all z passes but the last, then last + spectral op + first inverse
-    if constexpr (SH::Z::npass >= 2) {
-      z_stage0<SH, -1, PREC>(sm, T.twz);
-      __syncthreads();
-    }
-    if constexpr (SH::Z::npass >= 3) {
-      z_tile_pass<SH, typename SH::Z, 1, -1, true>(sm, T.twz);
-      __syncthreads();
-    }
-    z_mod_pass<SH>(sm, mod, base);
+  // all z passes but the last, then last + spectral op + first inverse
+  z_stage0<SH, -1, PREC>(sm, T.twz);
+  __syncthreads();
+  if constexpr (SH::Z::npass >= 3) {
+    z_tile_pass<SH, typename SH::Z, 1, -1, true>(sm, T.twz);
     __syncthreads();
-    if constexpr (SH::Z::npass >= 3) {
-      z_tile_pass<SH, typename SH::Z, 1, +1, true>(sm, T.twz);
-      __syncthreads();
-    }
-    if constexpr (SH::Z::npass >= 2) {
-      z_stage0<SH, +1, PREC>(sm, T.twz);
-      __syncthreads();
-    }
-    tile_inverse_down_to<SH, typename SH::Y, 0, false>(sm, T.twy);
   }
+  z_mod_pass<SH>(sm, mod, base);
+  __syncthreads();
+  if constexpr (SH::Z::npass >= 3) {
+    z_tile_pass<SH, typename SH::Z, 1, +1, true>(sm, T.twz);
+    __syncthreads();
+  }
+  z_stage0<SH, +1, PREC>(sm, T.twz);
+  __syncthreads();
+  tile_inverse_down_to<SH, typename SH::Y, 0, false>(sm, T.twy);
   {
     // planes z >= zout are not needed downstream (BW even: whole float4s)
     const int zo = mod.zout < SH::NZ ? mod.zout : SH::NZ;

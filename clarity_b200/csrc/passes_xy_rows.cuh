@@ -320,10 +320,6 @@ __global__ void __launch_bounds__(X::THREADS, X::MINB)
     twl[t] = __ldg(&T.twny[(y0base + g) * k1]);
   }
   CLARITY_PDL_WAIT();  // the previous pass's output is complete and visible
-  if (epi.zero_plane(z)) {  // neither read nor written (see Mod::zn)
-    if constexpr (requires { epi.finish_skipped(); }) epi.finish_skipped();
-    return;
-  }
   if constexpr (requires { epi.prepare(); }) epi.prepare();
   // rows j >= L of every line are outside the image (zero for this epilogue)
   constexpr bool CP = Epi::has_zero_rows;

@@ -397,10 +397,6 @@ __global__ void __launch_bounds__(X::THREADS, X::MINB)
     for (int t = threadIdx.x; t < X::M; t += CLARITY_BLOCK_STRIDE(X::THREADS)) s_twx[t] = __ldg(&T.twx[t]);
   const float2* twx = X::TW_SMEM ? s_twx : T.twx;
   CLARITY_PDL_WAIT();  // the previous pass's output is complete and visible
-  if (epi.zero_plane(z)) {  // neither read nor written (see Mod::zn)
-    if constexpr (requires { epi.finish_skipped(); }) epi.finish_skipped();
-    return;
-  }
   // the spectrum box, issued before anything else
   if (threadIdx.x == 0) {
     mbar_arrive_expect_tx(&bar, (uint32_t)(X::BOX_F2 * 8));

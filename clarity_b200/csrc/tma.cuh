@@ -1,10 +1,9 @@
-// tma.cuh -- bulk asynchronous copies (TMA, cp.async.bulk) between global
-// and shared memory, completed on an mbarrier, for sm_100a.
+// tma.cuh -- tiled tensor copies (TMA, cp.async.bulk.tensor) between global and
+// shared memory, completed on an mbarrier, 16-byte asynchronous copies and L2
+// loads and prefetches, for sm_100a.
 //
 // Only plain one-CTA copies are used: every source is this GPU's own memory
-// and no copy is broadcast to other CTAs.  Every address and size is a
-// multiple of 16 bytes (the rule for untiled bulk copies); callers check
-// that at compile time.  Waits are bounded: after kWaitLimit polls a wait
+// and no copy is broadcast to other CTAs.  Waits are bounded: after kWaitLimit polls a wait
 // records an error code in *err and gives up, so a lost completion can
 // never hang the GPU.
 #pragma once
@@ -46,26 +45,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
   return ok != 0;
-}
-// global -> shared, completes `bytes` of the barrier's transaction count
-__device__ __forceinline__ void bulk_load(void* dst_smem, const void* src_gmem,
-                                          uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1], %2, [%3];" ::"r"(smem_u32(dst_smem)),
-      "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-// shared -> global, tracked by the issuing thread's bulk group
-__device__ __forceinline__ void bulk_store(void* dst_gmem, const void* src_smem,
-                                           uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst_gmem),
-               "r"(smem_u32(src_smem)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_store_commit_and_wait() {
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 // make this thread's generic-proxy shared-memory writes visible to bulk copies
 __device__ __forceinline__ void fence_smem_to_async() {
@@ -120,13 +99,6 @@ inline void prefetch_l2(const void*, uint32_t) {}
 inline void mbar_init(uint64_t* bar, uint32_t) { *bar = 0; }
 inline void mbar_arrive_expect_tx(uint64_t*, uint32_t) {}
 inline bool mbar_try_wait(uint64_t*, uint32_t) { return true; }
-inline void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t*) {
-  std::memcpy(dst, src, bytes);
-}
-inline void bulk_store(void* dst, const void* src, uint32_t bytes) {
-  std::memcpy(dst, src, bytes);
-}
-inline void bulk_store_commit_and_wait() {}
 inline void bulk_commit() {}
 inline void bulk_wait_read_all() {}
 inline void fence_smem_to_async() {}
