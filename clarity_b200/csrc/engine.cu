@@ -1020,7 +1020,7 @@ __global__ void k_pad_scaled(PaddedSrc p, const float* __restrict__ scale, float
   }
 }
 
-// out = *scale * in (work box)
+// out = *scale * in
 __global__ void k_scale_copy(const float* __restrict__ in, const float* __restrict__ scale,
                              float* __restrict__ out, long long n) {
   const float s = *scale;

@@ -75,9 +75,10 @@ struct VolPlan {
 #define CLARITY_HD
 #endif
 
-// Division of 0 <= n < 2^20 by a fixed 1 <= d < 2^11 as a multiply-high:
-// m = ceil(2^32 / d) is off by less than d, so n m / 2^32 is off by less than
-// n d / 2^32 < 1/d and its floor is exact.
+// Division of n >= 0 by a fixed d >= 1, n d < 2^32, as a multiply-high:
+// m = ceil(2^32 / d) exceeds 2^32 / d by less than 1, so n m / 2^32 exceeds n / d
+// by less than n / 2^32 < 1 / d: too little to reach the next whole number, and
+// the floor is exact.
 struct FDiv {
   unsigned m, one;  // one: all bits set for d = 1, whose m would be 2^32
 };
@@ -167,7 +168,10 @@ bool make_plan(int nx, int ny, int nz, VolPlan* out, std::string* why);
 int make_plan_candidates(int nx, int ny, int nz, VolPlan* out, int max_out, std::string* why);
 
 // Plans the column-pair passes; false for boxes they do not serve (a z tile
-// beyond shared memory, rows beyond kPairMaxNx, unsupported factors).
+// beyond shared memory, rows beyond kPairMaxNx, unsupported factors).  The longest
+// rows that were measured and tested are 1024 and the x twiddles (8 bytes an
+// element) still leave room for a row quad there; longer boxes keep the
+// runtime-planned passes.
 constexpr int kPairMaxNx = 1280;
 bool make_pair_plan(int nx, int ny, int nz, PairPlan* out);
 // Tables of a pair plan: the padded shared-memory slot of every natural x

@@ -222,6 +222,10 @@ static void search_pair(int n, int depth, int* cur, int* best, int* best_len, in
   }
 }
 
+// FDiv is exact for n d < 2^32.  What the passes divide are indices into a tile in
+// shared memory, by extents of that tile: both below the 16-byte slots it has.
+static_assert((kSmemMax / 16ll) * (kSmemMax / 16) < (1ll << 32), "FDiv");
+
 static bool pair_axis(int n, bool padded, PairAxis* A) {
   std::memset(A, 0, sizeof(*A));
   A->n = n;
