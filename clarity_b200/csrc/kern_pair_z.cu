@@ -1,8 +1,9 @@
-// kern_pair_z.cu -- column-pair pass kernels (pair_dispatch.cuh).
+// kern_pair_z.cu -- column-pair passes (pair_dispatch.cuh): the z passes of every call.
+#ifndef CLARITY_HOST_EMULATION  // one register class there
 #include "pair_dispatch.cuh"
 
 namespace clarity {
-template bool pair_z<ModOTF>(const PlanEntry&, cudaStream_t, const ModOTF&, const float2*, float2*, cudaError_t*);
-template bool pair_z<ModWiener>(const PlanEntry&, cudaStream_t, const ModWiener&, const float2*, float2*, cudaError_t*);
-template bool pair_z<ModForward>(const PlanEntry&, cudaStream_t, const ModForward&, const float2*, float2*, cudaError_t*);
+CLARITY_PAIR_Z(ModForward, false)
+CLARITY_PAIR_Z(ModOTF, false)
 }  // namespace clarity
+#endif

@@ -6,6 +6,7 @@
 #include "engine.hpp"
 #include "ops.cuh"
 #include "passes.cuh"
+#include <type_traits>
 
 namespace clarity {
 
@@ -20,13 +21,29 @@ bool static_xy_inv_fwd(const PlanEntry&, cudaStream_t, const F&, float2*, cudaEr
 template <class F>
 bool static_xy_inverse(const PlanEntry&, cudaStream_t, const F&, const float2*, cudaError_t*);
 
-// Column-pair launches (pair_dispatch.cuh, instantiated in kern_pair_*.cu).
-template <class F>
-bool pair_xy_forward(const PlanEntry&, cudaStream_t, const F&, float2*, cudaError_t*);
-template <class F, bool FUSE>
-bool pair_xy_inverse(const PlanEntry&, cudaStream_t, const F&, float2*, cudaError_t*);
-template <class F>
-bool pair_z(const PlanEntry&, cudaStream_t, const F&, const float2*, float2*, cudaError_t*);
+// Column-pair launches (pair_dispatch.cuh).  BIG is the kernels' register class:
+// radices above 16.  The classes are instantiated in files of their own
+// (kern_pair_*.cu), the functors by who uses them together: the runtime unpacks
+// and loads a file's whole code at the first launch of a kernel in it.  With both
+// classes and unrelated functors in a file the first convolution of a process took
+// 65 to 73 ms at the 32x32x16 box and the first RL after it 60 to 67, against 15 to
+// 19 and 9 to 13 (one B200; the runtime-planned passes 25 to 29 and 40 to 45).
+template <class F, bool BIG>
+cudaError_t pair_xy_forward(const PlanEntry&, cudaStream_t, const F&, float2*);
+template <class F, bool FUSE, bool BIG>
+cudaError_t pair_xy_inverse(const PlanEntry&, cudaStream_t, const F&, float2*);
+template <class F, bool BIG>
+cudaError_t pair_z(const PlanEntry&, cudaStream_t, const F&, const float2*, float2*);
+
+// launch(BIG) for a plan's class.  The emulation runs one thread per block, so the
+// classes do not differ there: one instantiation halves its build.
+template <class L>
+inline cudaError_t pair_class(bool big, const L& launch) {
+#ifndef CLARITY_HOST_EMULATION
+  if (!big) return launch(std::false_type{});
+#endif
+  return launch(std::true_type{});
+}
 
 #ifndef CL_CHECK
 #define CL_CHECK(call)                                         \
@@ -55,8 +72,13 @@ Status xy_forward(Context& ctx, const PlanEntry& pe, const Pro& pro,
                          float2* S) {
   const VolPlan& P = pe.P;
   cudaError_t se = cudaSuccess;
-  if (pair_xy_forward(pe, ctx.exec_stream(), pro, S, &se) ||
-      static_xy_forward(pe, ctx.exec_stream(), pro, S, &se))
+  if (pe.pair.ok) {
+    se = pair_class(pe.pair.big_xy, [&](auto big) {
+      return pair_xy_forward<Pro, decltype(big)::value>(pe, ctx.exec_stream(), pro, S);
+    });
+    return status_from_cuda(se, "xy forward");
+  }
+  if (static_xy_forward(pe, ctx.exec_stream(), pro, S, &se))
     return status_from_cuda(se, "xy forward");
   auto k = k_xy_forward<Pro>;
   CL_CHECK(prep_kernel(k, P.xy_smem));
@@ -73,8 +95,14 @@ Status xy_inverse(Context& ctx, const PlanEntry& pe, const Epi& epi,
                          const float2* S) {
   const VolPlan& P = pe.P;
   cudaError_t se = cudaSuccess;
-  if (pair_xy_inverse<Epi, false>(pe, ctx.exec_stream(), epi, const_cast<float2*>(S), &se) ||
-      static_xy_inverse(pe, ctx.exec_stream(), epi, S, &se))
+  if (pe.pair.ok) {
+    se = pair_class(pe.pair.big_xy, [&](auto big) {
+      return pair_xy_inverse<Epi, false, decltype(big)::value>(pe, ctx.exec_stream(), epi,
+                                                               const_cast<float2*>(S));
+    });
+    return status_from_cuda(se, "xy inverse");
+  }
+  if (static_xy_inverse(pe, ctx.exec_stream(), epi, S, &se))
     return status_from_cuda(se, "xy inverse");
   auto k = k_xy_inverse<Epi>;
   CL_CHECK(prep_kernel(k, P.xy_smem));
@@ -91,8 +119,13 @@ Status xy_inv_fwd(Context& ctx, const PlanEntry& pe, const Mid& mid,
                          float2* S) {
   const VolPlan& P = pe.P;
   cudaError_t se = cudaSuccess;
-  if (pair_xy_inverse<Mid, true>(pe, ctx.exec_stream(), mid, S, &se) ||
-      static_xy_inv_fwd(pe, ctx.exec_stream(), mid, S, &se))
+  if (pe.pair.ok) {
+    se = pair_class(pe.pair.big_xy, [&](auto big) {
+      return pair_xy_inverse<Mid, true, decltype(big)::value>(pe, ctx.exec_stream(), mid, S);
+    });
+    return status_from_cuda(se, "xy inverse+forward");
+  }
+  if (static_xy_inv_fwd(pe, ctx.exec_stream(), mid, S, &se))
     return status_from_cuda(se, "xy inverse+forward");
   auto k = k_xy_inv_fwd<Mid>;
   CL_CHECK(prep_kernel(k, P.xy_smem));
@@ -109,8 +142,13 @@ Status z_pass(Context& ctx, const PlanEntry& pe, const Mod& mod,
                      const float2* Sin, float2* Sout) {
   const VolPlan& P = pe.P;
   cudaError_t se = cudaSuccess;
-  if (pair_z(pe, ctx.exec_stream(), mod, Sin, Sout, &se) ||
-      static_z(pe, ctx.exec_stream(), mod, Sin, Sout, &se))
+  if (pe.pair.ok) {
+    se = pair_class(pe.pair.big_z, [&](auto big) {
+      return pair_z<Mod, decltype(big)::value>(pe, ctx.exec_stream(), mod, Sin, Sout);
+    });
+    return status_from_cuda(se, "z pass");
+  }
+  if (static_z(pe, ctx.exec_stream(), mod, Sin, Sout, &se))
     return status_from_cuda(se, "z pass");
   auto k = k_z<Mod>;
   CL_CHECK(prep_kernel(k, P.z_smem));
