@@ -3,10 +3,11 @@
 // the heavy kernels compile in parallel, and engine.cu sees them through the
 // extern declarations at the bottom.
 #pragma once
+#include <type_traits>
+
 #include "engine.hpp"
 #include "ops.cuh"
 #include "passes.cuh"
-#include <type_traits>
 
 namespace clarity {
 

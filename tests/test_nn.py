@@ -190,6 +190,25 @@ def test_conv3_weight_gradient_of_more_runs_than_a_grid_dimension(clarity_gpu):
     assert ((db.double() - f.sum(0)).abs() <= bound * f.abs().sum(0) + 1e-30).all()
 
 
+def test_conv3_weight_gradient_of_the_longest_runs(clarity_gpu):
+    # 756 tiles in 63 runs of 12: 96 MMAs into an accumulator, each within two
+    # roundings of its partial sum, then 63 atomic additions
+    from clarity_b200 import unet
+    D, H, W, c = 17, 55, 96, 64
+    g = torch.Generator(device="cuda").manual_seed(12)
+    x = torch.randn((D, H, W, c), generator=g, device="cuda").to(torch.bfloat16)
+    dy = torch.randn((D, H, W, c), generator=g, device="cuda").to(torch.bfloat16)
+    dw = torch.zeros(c * 27 * c, device="cuda")
+    unet.conv3_wgrad(x, dy, dw, None)
+    torch.cuda.synchronize()
+    p = torch.nn.functional.pad(x.double(), (0, 0, 1, 1, 1, 1, 1, 1))
+    f, got = dy.double().reshape(-1, c), dw.double().reshape(c, 27, c)
+    bound = (2 * 96 + 63) * 2.0 ** -24
+    for t in range(27):
+        sh = p[t // 9:t // 9 + D, t // 3 % 3:t // 3 % 3 + H, t % 3:t % 3 + W].reshape(-1, c)
+        assert ((got[:, t] - f.T @ sh).abs() <= bound * (f.abs().T @ sh.abs())).all(), t
+
+
 @pytest.mark.parametrize("cout", [16, 48, 80, 128, 2032, 2048, 2064])
 @pytest.mark.parametrize("voxels", [1, 5, 300])
 def test_conv3_bias_gradient(clarity_gpu, cout, voxels):
