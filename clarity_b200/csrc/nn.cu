@@ -302,9 +302,9 @@ __global__ void __launch_bounds__(128) k_conv3(const Conv3Args a) {
 //     add bias, apply ReLU and pack to BF16, release the accumulators to the
 //     next item's MMAs (with one buffer they would wait for the stores
 //     otherwise), then apply the mask and store.
-// Measured on one B200, 32 -> 32 channels at 128x128x32: 65.4 -> 55.4 us by the
-// direct slab reads, the early release and the resident weights; 16 -> 16 at
-// 256x256x64: 249 -> 169 us.  What bounds it now is the MMAs' A operand: one
+// Measured on one B200, 32 -> 32 channels at 128x128x32: 67 -> 60 us by the direct
+// slab reads and the early release, 57 with the resident weights; 16 -> 16 at
+// 256x256x64: 256 -> 252 -> 170 us.  What bounds it now is the MMAs' A operand: one
 // takes about 50 cycles at N = 16 and 32 alike, at most a third of them math.
 // Shared memory holds kTmStages stages; TMEM holds two window buffers and one
 // or two accumulator buffers.  Every wait is bounded: a wait that runs out
@@ -728,8 +728,9 @@ __global__ void __launch_bounds__(kTmThreads, 1)
 // times an infinity there would be a NaN).  What bounds
 // it is the fragment loads (one per two MMAs at BM = 16); the form it replaces
 // gathered every tap's shifted input from L2 anew, 16 voxels at a time.
-// Measured on one B200 at 128x128x48: the largest layer, 16+32 -> 16 channels,
-// 952 -> 177 us; the 13 layers of a training step together 2860 -> 770 us.
+// Measured on one B200 with the bias gradient at 128x128x48: the largest layer,
+// 16+32 -> 16 channels, 953 -> 152 us; the 13 layers of a training step together
+// 2870 -> 640 us.
 constexpr int kWgTaps = 7;        // taps per warp (the last warp has 6)
 constexpr int kVoxTile = kTZ * kTY * kTX;  // 128
 
@@ -1257,8 +1258,8 @@ static bool tm_geometry(const nnk::Conv3Args& a, int* bn_out, nnk::TmGeom* g, in
   // The weights of a stage are 16-byte rows, as slow for a tensor copy as the
   // slab's 32-byte ones: where every item has the same weights and they fit
   // beside the stages, they are loaded once (16 -> 16 channels at 256x256x64,
-  // 55 items a block: 249 -> 169 us; 32 -> 32 at 128x128x32, 6.9 items: 58.5 ->
-  // 55.4).  Nothing overlaps that load, so blocks of a few items stream them
+  // 55 items a block: 252 -> 170 us; 32 -> 32 at 128x128x32, 6.9 items: 60.3 ->
+  // 56.7).  Nothing overlaps that load, so blocks of a few items stream them
   // (96 -> 32 at 64x64x24, 2.6 items: 47.4 us against 53.4).
   const long long all = 3ll * ((a.c1 + a.c2) / 16) * wb;
   const bool res = G.nnb == 1 && items >= 4ll * tm_sm_count() &&
